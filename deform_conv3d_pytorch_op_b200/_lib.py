@@ -95,6 +95,24 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The C++ host side of the autograd Functions (``_dcn_torch.so``, built beside this file)."""
+    global _native
+    if _native is None:
+        lib()                                     # the same error where nothing has been built
+        try:
+            from . import _dcn_torch
+        except ImportError as e:
+            raise DcnError("_dcn_torch.so is missing or does not load (%s): build it with `python -m "
+                           "deform_conv3d_pytorch_op_b200.build`; there is no fallback implementation" % e) from e
+        _dcn_torch.set_error(DcnError)
+        _native = _dcn_torch
+    return _native
+
+
 def check(status: int, what: str = "") -> None:
     if status != 0:
         raise DcnError("%s failed: %s (status %d)" % (what or "libdcn call", lib().dcn_status_string(status).decode(),

@@ -40,11 +40,6 @@ def check_status(device=None) -> None:
         _lib.check(_lib.lib().dcn_check_status(_lib.current_stream(dev)), "device status")
 
 
-def status_check_enabled() -> bool:
-    """``DCN_CHECK_STATUS=1``: poll the status word after every backward pass (never inside a stream capture)."""
-    return os.environ.get("DCN_CHECK_STATUS", "0") not in ("", "0")
-
-
 def _nvtx_enabled() -> bool:
     """``DCN_NVTX=1``: wrap every library call of :class:`Op` in an NVTX range named after the entry point, so that
     the passes show up by name on a profiler's timeline (the reference has only wall-clock prints,
