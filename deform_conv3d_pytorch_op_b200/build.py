@@ -15,7 +15,7 @@ CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
 LIB = os.path.join(CSRC, "libdcn.so")
 BINDING = os.path.join(os.path.dirname(CSRC), "_dcn_torch.so")
 BINDING_SOURCE = os.path.join(CSRC, "dcn_torch.cpp")
-SOURCES = ["dcn_api.cu", "dcn_simt.cu", "dcn_tc.cu"]
+SOURCES = ["dcn_api.cu", "dcn_simt.cu", "dcn_exact.cu", "dcn_tc.cu"]
 HEADERS = ["dcn_common.cuh", "dcn_internal.h", os.path.join("..", "..", "include", "dcn.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"] + os.environ.get("DCN_NVCC_EXTRA", "").split()

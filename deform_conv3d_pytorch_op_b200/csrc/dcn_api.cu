@@ -72,6 +72,19 @@ bool workspace_ok(const void* ws, size_t have, size_t need) {
     return ws != nullptr && have >= need && aligned(ws, 256);
 }
 
+// Which EXACT kernels a problem takes when the caller brings the workspace they want: those of dcn_exact.cu, except
+// for very small problems (one launch each way, dcn_simt_small.cuh) and for contractions so short that most of a 64-row
+// tile would be padding (measured: 8 x 2 -> 4 channels, 64x64, K = 18: 92 us a step against 64 us; from K = 36 up,
+// 12x12 and larger, 5-70 % faster in fp32 and fp64).
+bool exact_worth(const dcn_problem* p, const Geom& g) {
+    return g.Kg >= 32 && !dcn::simt_small_supported(g, p->dtype, p->ndim, p->deformable) &&
+           dcn::exact_supported(g, p->dtype, p->deformable);
+}
+bool exact_ready(const dcn_problem* p, const Geom& g, int pass, const void* ws, size_t ws_bytes) {
+    return ws != nullptr && exact_worth(p, g) &&
+           workspace_ok(ws, ws_bytes, dcn::exact_workspace_bytes(g, p->dtype, p->deformable, pass));
+}
+
 int check_ptrs(const dcn_problem* p, std::initializer_list<const void*> ptrs) {
     const size_t es = p->dtype == DCN_F64 ? 8 : 4;
     for (const void* q : ptrs)
@@ -120,9 +133,11 @@ int dcn_precision_supported(const dcn_problem* p) {
 }
 
 size_t dcn_workspace_bytes(const dcn_problem* p, int pass) {
-    if (validate(p) != DCN_OK || p->precision == DCN_PREC_EXACT) return 0;
+    if (validate(p) != DCN_OK) return 0;
     Geom g;
     make_geom(p, g);
+    if (p->precision == DCN_PREC_EXACT)
+        return exact_worth(p, g) ? dcn::exact_workspace_bytes(g, p->dtype, p->deformable, pass) : 0;
     if (!dcn::tc_supported(g, p->ndim, p->deformable)) return 0;
     if (pass == DCN_PASS_BACKWARD) return dcn::tc_backward_workspace_bytes(g);
     return dcn::tc_workspace_bytes(g, p->ndim, pass);
@@ -133,6 +148,7 @@ int dcn_launch_count(const dcn_problem* p, int pass) {
     Geom g;
     make_geom(p, g);
     if (p->precision == DCN_PREC_EXACT) {
+        if (exact_worth(p, g)) return dcn::exact_launch_count(pass);
         if (pass != DCN_PASS_BACKWARD) return 1;
         if (dcn::simt_small_supported(g, p->dtype, p->ndim, p->deformable)) return 2;      // zero fill + one kernel
         return dcn::simt_backward_both_supported(g, p->dtype) ? 1 : 2;
@@ -157,6 +173,8 @@ int dcn_forward(const dcn_problem* p, const void* x, const void* offset, const v
         return dcn::tc_forward(g, p->ndim, p->deformable, (const float*)x, (const float*)offset,
                                (const float*)weight, (const float*)bias, (float*)y, ws, ws_bytes, st);
     }
+    if (exact_ready(p, g, DCN_PASS_FORWARD, ws, ws_bytes))
+        return dcn::exact_forward(g, p->dtype, p->ndim, p->deformable, x, offset, weight, bias, y, ws, st);
     if (dcn::simt_small_supported(g, p->dtype, p->ndim, p->deformable))
         return dcn::simt_small_forward(g, p->ndim, x, offset, weight, bias, y, st);
     return dcn::simt_forward(g, p->dtype, p->ndim, p->deformable, x, offset, weight, bias, y, st);
@@ -201,6 +219,9 @@ int dcn_backward_data(const dcn_problem* p, const void* x, const void* offset, c
                                      (const float*)weight, (const float*)dy, (float*)dx, (float*)doffset, ws,
                                      ws_bytes, st);
     }
+    if (exact_ready(p, g, DCN_PASS_BACKWARD_DATA, ws, ws_bytes))
+        return dcn::exact_backward(g, p->dtype, p->ndim, p->deformable, DCN_PASS_BACKWARD_DATA, 1, x, offset, weight, dy, dx,
+                                   doffset, nullptr, ws, st);
     return dcn::simt_backward_data(g, p->dtype, p->ndim, p->deformable, x, offset, weight, dy, dx,
                                    p->deformable ? doffset : nullptr, st);
 }
@@ -224,6 +245,9 @@ int dcn_backward_weight(const dcn_problem* p, const void* x, const void* offset,
                 return DCN_ERR_WORKSPACE;
             r = dcn::tc_backward_weight(g, p->ndim, p->deformable, (const float*)x, (const float*)offset,
                                         (const float*)dy, (float*)dweight, ws, ws_bytes, st);
+        } else if (exact_ready(p, g, DCN_PASS_BACKWARD_WEIGHT, ws, ws_bytes)) {
+            r = dcn::exact_backward(g, p->dtype, p->ndim, p->deformable, DCN_PASS_BACKWARD_WEIGHT, 1, x, offset, nullptr, dy,
+                                    nullptr, nullptr, dweight, ws, st);
         } else {
             r = dcn::simt_backward_weight(g, p->dtype, p->ndim, p->deformable, x, offset, dy, dweight, st);
         }
@@ -253,6 +277,9 @@ int dcn_backward(const dcn_problem* p, const void* x, const void* offset, const 
             r = dcn::tc_backward(g, p->ndim, p->deformable, (const float*)x, (const float*)offset, (const float*)weight,
                                  (const float*)dy, x_channels_last, (float*)dx, (float*)doffset, (float*)dweight, ws,
                                  ws_bytes, st);
+        } else if (exact_ready(p, g, DCN_PASS_BACKWARD, ws, ws_bytes)) {
+            r = dcn::exact_backward(g, p->dtype, p->ndim, p->deformable, DCN_PASS_BACKWARD, 0, x, offset, weight, dy, dx,
+                                    doffset, dweight, ws, st);
         } else {
             const size_t es = p->dtype == DCN_F64 ? 8 : 4;
             const bool small = dcn::simt_small_supported(g, p->dtype, p->ndim, p->deformable);
@@ -349,7 +376,20 @@ size_t dcn_layer_workspace_bytes(const dcn_problem* p, int pass) {
     Geom g, gq;
     make_geom(p, g);
     make_geom(&q, gq);
-    if (p->precision == DCN_PREC_EXACT) return pass == DCN_PASS_FORWARD ? 0 : layer_doff_bytes(p, g);
+    if (p->precision == DCN_PREC_EXACT) {
+        // both convolutions' passes run one after the other in the same scratch
+        size_t scratch = 0;
+        if (exact_worth(p, g)) {
+            const dcn_problem* both[2] = {p, &q};
+            for (const dcn_problem* r : both)
+                for (int k = 0; k < 4; ++k)
+                    if ((k == 0) == (pass == DCN_PASS_FORWARD)) {
+                        const size_t b = dcn_workspace_bytes(r, k);
+                        scratch = b > scratch ? b : scratch;
+                    }
+        }
+        return pass == DCN_PASS_FORWARD ? scratch : layer_doff_bytes(p, g) + scratch;
+    }
     if (!dcn::tc_supported(g, p->ndim, 1) || !dcn::tc_supported(gq, p->ndim, 0)) return 0;
     return dcn::tc_layer_workspace_bytes(g, gq, p->ndim, pass == DCN_PASS_FORWARD ? 0 : 3);
 }
@@ -392,9 +432,9 @@ int dcn_layer_forward(const dcn_problem* p, const void* x, const void* offset_we
         if (dcn::simt_small_layer_supported(g, gq, p->dtype, p->ndim))      // one kernel, offsets formed on the SM
             return dcn::simt_small_layer_forward(g, gq, p->ndim, x, offset_weight, offset_bias, weight, bias, offset, y,
                                                  static_cast<cudaStream_t>(stream));
-        const int r = dcn_forward(&q, x, nullptr, offset_weight, offset_bias, offset, nullptr, 0, stream);
+        const int r = dcn_forward(&q, x, nullptr, offset_weight, offset_bias, offset, ws, ws_bytes, stream);
         if (r != DCN_OK) return r;
-        return dcn_forward(p, x, offset, weight, bias, y, nullptr, 0, stream);
+        return dcn_forward(p, x, offset, weight, bias, y, ws, ws_bytes, stream);
     }
     if (p->dtype != DCN_F32) return DCN_ERR_UNSUPPORTED;
     Geom g, gq;
@@ -436,10 +476,14 @@ int dcn_layer_backward(const dcn_problem* p, const void* x, const void* offset, 
     if (p->precision == DCN_PREC_EXACT) {
         if (chain && !workspace_ok(ws, ws_bytes, layer_doff_bytes(p, g))) return DCN_ERR_WORKSPACE;
         void* doff = chain ? ws : nullptr;
-        int r = dcn_backward(p, x, offset, weight, dy, nullptr, dx, doff, dweight, dbias, nullptr, 0, stream);
+        // behind dOffset: the scratch of the passes, which they take one after the other
+        const size_t at = layer_doff_bytes(p, g);
+        void* sub = ws != nullptr && ws_bytes > at ? static_cast<uint8_t*>(ws) + at : nullptr;
+        const size_t sub_bytes = sub != nullptr ? ws_bytes - at : 0;
+        int r = dcn_backward(p, x, offset, weight, dy, nullptr, dx, doff, dweight, dbias, sub, sub_bytes, stream);
         if (r != DCN_OK || !chain) return r;
         if (dx != nullptr) {                                            // accumulates into the dx just written
-            r = dcn_backward_data(&q, nullptr, nullptr, offset_weight, doff, dx, nullptr, nullptr, 0, stream);
+            r = dcn_backward_data(&q, nullptr, nullptr, offset_weight, doff, dx, nullptr, sub, sub_bytes, stream);
             if (r != DCN_OK) return r;
         }
         if (doffset_weight != nullptr) {
@@ -447,7 +491,7 @@ int dcn_layer_backward(const dcn_problem* p, const void* x, const void* offset, 
             if (cudaMemsetAsync(doffset_weight, 0, (size_t)gq.O * gq.Cg * gq.kv * es, st) != cudaSuccess) return DCN_ERR_CUDA;
         }
         if (doffset_weight != nullptr || doffset_bias != nullptr)
-            r = dcn_backward_weight(&q, x, nullptr, doff, doffset_weight, doffset_bias, nullptr, 0, stream);
+            r = dcn_backward_weight(&q, x, nullptr, doff, doffset_weight, doffset_bias, sub, sub_bytes, stream);
         return r;
     }
     if (p->dtype != DCN_F32) return DCN_ERR_UNSUPPORTED;

@@ -36,6 +36,16 @@ int bias_grad(const Geom& g, int dtype, const void* dy, void* dbias, cudaStream_
 int debug_points(const Geom& g, int dtype, int ndim, const void* off, int n, void* coords, int32_t* valid,
                  int32_t* lo, int32_t* hi, cudaStream_t st);
 
+// EXACT precision over a channels-last copy of the input, dcn_exact.cu (needs a workspace).  pass: 0 forward, 1 backward
+// data, 2 backward weight, 3 both; add: dX and dW accumulate instead of being overwritten.
+bool exact_supported(const Geom& g, int dtype, int deform);
+size_t exact_workspace_bytes(const Geom& g, int dtype, int deform, int pass);
+int exact_launch_count(int pass);
+int exact_forward(const Geom& g, int dtype, int ndim, int deform, const void* x, const void* off, const void* w,
+                  const void* bias, void* y, void* ws, cudaStream_t st);
+int exact_backward(const Geom& g, int dtype, int ndim, int deform, int pass, int add, const void* x, const void* off,
+                   const void* w, const void* dy, void* dx, void* doff, void* dw, void* ws, cudaStream_t st);
+
 // BF16 tensor-core (tcgen05) path, dcn_tc.cu.  fp32 tensors only.
 bool tc_supported(const Geom& g, int ndim, int deform);
 size_t tc_workspace_bytes(const Geom& g, int ndim, int pass);

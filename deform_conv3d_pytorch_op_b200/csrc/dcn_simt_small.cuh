@@ -502,17 +502,21 @@ small_backward_kernel(const Geom g, const float* __restrict__ x, const float* __
     }
 }
 
-// fp32 deformable problems of at most 2^25 multiply-adds per pass whose group weights fit the shared memory.
+// fp32 deformable problems whose group weights fit the shared memory and whose busiest SM does at most 110k
+// multiply-adds per pass, a wave of CTAs counting as 25k beside its own: the line where the kernels of dcn_exact.cu
+// become faster (B200, GPU time of one step: 2 x 16 -> 32 channels, 32x32, 98k: 30 against 42 us; 4 x 16 -> 16, 32x32,
+// two waves, 124k: 44 against 36 us; 3-D 2 x 16 -> 16, 4x10x10, 135k: 55 against 40 us; 8 x 3 -> 8, 40x40, six waves,
+// 170k: 50 against 42 us).  DCN_SMALL_LOG2 puts a limit of that power of two on all multiply-adds of a pass in its place.
 inline bool small_supported(const Geom& g, int dtype, int ndim, int deform) {
     if (dtype != 0 || !deform) return false;
-    // multiply-adds per pass up to which these kernels are taken (DCN_SMALL_LOG2 overrides the exponent)
-    static const double limit = [] {
-        const char* e = getenv("DCN_SMALL_LOG2");
-        const int lg = e != nullptr ? atoi(e) : 25;     // measured crossover with the tiled kernels: 2^25 .. 2^25.2
-        return (double)(1ull << (lg < 0 ? 0 : (lg > 40 ? 40 : lg)));
-    }();
-    if ((double)g.P * g.Kg * g.Og * g.G > limit) return false;
+    static const int lg = [] { const char* e = getenv("DCN_SMALL_LOG2"); return e != nullptr ? atoi(e) : -1; }();
+    const double macs = (double)g.P * g.Kg * g.Og * g.G;
+    if (macs > (lg < 0 ? 33554432.0 : (double)(1ull << (lg > 40 ? 40 : lg)))) return false;
     const SmallDims d = small_dims(g, ndim);
+    if (lg < 0) {
+        const long long ctas = (g.P + d.TP - 1) / d.TP * g.G, waves = (ctas + 147) / 148;
+        if ((double)waves * (25e3 + macs / (double)ctas) > 110e3) return false;
+    }
     return d.smem_bwd <= 96 * 1024 && d.smem_fwd <= 96 * 1024;
 }
 

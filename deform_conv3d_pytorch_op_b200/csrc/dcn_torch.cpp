@@ -203,7 +203,8 @@ struct CallTensors {
     Tensor x, off, w, b, ow, ob;         // off: kDeform; ow, ob: kLayer
 };
 
-// Forward pass; `keep` receives the workspace, whose start holds the input copy the backward pass takes over.
+// Forward pass; on the bf16 path `keep` receives the workspace, whose start holds the input copy (half the input's
+// size) that the backward pass takes over.
 // For a layer t.off receives the offsets.
 Tensor run_forward(const Problem& q, Kind kind, CallTensors& t, Tensor* keep) {
     const Tensor x = prep(t.x, "input", t.x, q.act);
@@ -239,7 +240,7 @@ Tensor run_forward(const Problem& q, Kind kind, CallTensors& t, Tensor* keep) {
         Range range("dcn_forward");
         check(dcn_forward(&q.p, ptr(x), ptr(off), ptr(w), ptr(b), wptr(y), wptr(ws), bytes, st), "dcn_forward");
     }
-    if (keep != nullptr) *keep = ws;
+    if (keep != nullptr && q.p.precision == DCN_PREC_BF16) *keep = ws;
     return y;
 }
 

@@ -97,7 +97,8 @@ int dcn_validate(const dcn_problem* p);
  * counts per convolution group and per deformable group that are multiples of 8), else 0. */
 int dcn_precision_supported(const dcn_problem* p);
 
-/* Scratch bytes `pass` needs (0 for the EXACT precision).  The workspace must be 256-byte aligned. */
+/* Scratch bytes `pass` wants.  The workspace must be 256-byte aligned.  BF16 needs it; EXACT runs without one on slower
+ * kernels, and wants none (0) where the problem is too small to gain from it. */
 size_t dcn_workspace_bytes(const dcn_problem* p, int pass);
 
 /* Number of kernel launches `pass` enqueues for this problem (memsets not counted); used by callers
