@@ -221,7 +221,7 @@ int dcn_backward_data(const dcn_problem* p, const void* x, const void* offset, c
     }
     if (exact_ready(p, g, DCN_PASS_BACKWARD_DATA, ws, ws_bytes))
         return dcn::exact_backward(g, p->dtype, p->ndim, p->deformable, DCN_PASS_BACKWARD_DATA, 1, x, offset, weight, dy, dx,
-                                   doffset, nullptr, ws, st);
+                                   doffset, nullptr, nullptr, ws, st);
     return dcn::simt_backward_data(g, p->dtype, p->ndim, p->deformable, x, offset, weight, dy, dx,
                                    p->deformable ? doffset : nullptr, st);
 }
@@ -238,6 +238,7 @@ int dcn_backward_weight(const dcn_problem* p, const void* x, const void* offset,
     make_geom(p, g);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int r = DCN_OK;
+    bool bias_done = false;
     if (dweight != nullptr) {
         if (p->precision == DCN_PREC_BF16) {
             if (!dcn::tc_supported(g, p->ndim, p->deformable)) return DCN_ERR_UNSUPPORTED;
@@ -247,13 +248,14 @@ int dcn_backward_weight(const dcn_problem* p, const void* x, const void* offset,
                                         (const float*)dy, (float*)dweight, ws, ws_bytes, st);
         } else if (exact_ready(p, g, DCN_PASS_BACKWARD_WEIGHT, ws, ws_bytes)) {
             r = dcn::exact_backward(g, p->dtype, p->ndim, p->deformable, DCN_PASS_BACKWARD_WEIGHT, 1, x, offset, nullptr, dy,
-                                    nullptr, nullptr, dweight, ws, st);
+                                    nullptr, nullptr, dweight, dbias, ws, st);
+            bias_done = true;
         } else {
             r = dcn::simt_backward_weight(g, p->dtype, p->ndim, p->deformable, x, offset, dy, dweight, st);
         }
         if (r != DCN_OK) return r;
     }
-    if (dbias != nullptr) r = dcn::bias_grad(g, p->dtype, dy, dbias, st);
+    if (dbias != nullptr && !bias_done) r = dcn::bias_grad(g, p->dtype, dy, dbias, st);
     return r;
 }
 
@@ -269,17 +271,19 @@ int dcn_backward(const dcn_problem* p, const void* x, const void* offset, const 
     make_geom(p, g);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int r = DCN_OK;
+    bool bias_done = false;
     if (dx != nullptr || doffset != nullptr || dweight != nullptr) {
         if (p->precision == DCN_PREC_BF16) {
             if (!dcn::tc_supported(g, p->ndim, p->deformable)) return DCN_ERR_UNSUPPORTED;
             if (!workspace_ok(ws, ws_bytes, dcn::tc_backward_workspace_bytes(g))) return DCN_ERR_WORKSPACE;
             if (x_channels_last != nullptr && !aligned(x_channels_last, 16)) return DCN_ERR_ALIGN;
             r = dcn::tc_backward(g, p->ndim, p->deformable, (const float*)x, (const float*)offset, (const float*)weight,
-                                 (const float*)dy, x_channels_last, (float*)dx, (float*)doffset, (float*)dweight, ws,
-                                 ws_bytes, st);
+                                 (const float*)dy, x_channels_last, (float*)dx, (float*)doffset, (float*)dweight,
+                                 (float*)dbias, &bias_done, ws, ws_bytes, st);
         } else if (exact_ready(p, g, DCN_PASS_BACKWARD, ws, ws_bytes)) {
             r = dcn::exact_backward(g, p->dtype, p->ndim, p->deformable, DCN_PASS_BACKWARD, 0, x, offset, weight, dy, dx,
-                                    doffset, dweight, ws, st);
+                                    doffset, dweight, dbias, ws, st);
+            bias_done = true;
         } else {
             const size_t es = p->dtype == DCN_F64 ? 8 : 4;
             const bool small = dcn::simt_small_supported(g, p->dtype, p->ndim, p->deformable);
@@ -290,7 +294,8 @@ int dcn_backward(const dcn_problem* p, const void* x, const void* offset, const 
                 return DCN_ERR_CUDA;
             const bool all = dx != nullptr && dweight != nullptr && (!p->deformable || doffset != nullptr);
             if (small) {
-                r = dcn::simt_small_backward(g, p->ndim, x, offset, weight, dy, dx, doffset, dweight, st);
+                r = dcn::simt_small_backward(g, p->ndim, x, offset, weight, dy, dx, doffset, dweight, dbias, st);
+                bias_done = true;
             } else if (all && dcn::simt_backward_both_supported(g, p->dtype)) {
                 r = dcn::simt_backward_both(g, p->ndim, p->deformable, x, offset, weight, dy, dx,
                                             p->deformable ? doffset : nullptr, dweight, st);     // one launch
@@ -304,7 +309,7 @@ int dcn_backward(const dcn_problem* p, const void* x, const void* offset, const 
         }
         if (r != DCN_OK) return r;
     }
-    if (dbias != nullptr) r = dcn::bias_grad(g, p->dtype, dy, dbias, st);
+    if (dbias != nullptr && !bias_done) r = dcn::bias_grad(g, p->dtype, dy, dbias, st);
     return r;
 }
 
@@ -402,7 +407,7 @@ int dcn_layer_launch_count(const dcn_problem* p, int pass) {
     make_geom(&q, gq);
     if (pass == DCN_PASS_FORWARD) {
         if (p->precision == DCN_PREC_EXACT && dcn::simt_small_layer_supported(g, gq, p->dtype, p->ndim)) return 1;
-        // (bf16: the input copy is built once for both convolutions)
+        // (bf16: one prologue for both convolutions)
         const int both = dcn_launch_count(&q, DCN_PASS_FORWARD) + dcn_launch_count(p, DCN_PASS_FORWARD);
         return p->precision == DCN_PREC_BF16 && both > 0 ? both - 1 : both;
     }
@@ -411,8 +416,8 @@ int dcn_layer_launch_count(const dcn_problem* p, int pass) {
     const int main = dcn_launch_count(p, DCN_PASS_BACKWARD);
     const int rest = dcn_launch_count(&q, DCN_PASS_BACKWARD_DATA) + dcn_launch_count(&q, DCN_PASS_BACKWARD_WEIGHT);
     if (main == 0 || rest == 0) return 0;
-    // bf16: the plain convolution's two gradient kernels share the packed dOffset and take the input copy over
-    return p->precision == DCN_PREC_BF16 ? main + rest - 2 : main + rest;
+    // bf16: prologue, two kernels, the pass that packs dOffset, two kernels, epilogue
+    return p->precision == DCN_PREC_BF16 ? 7 : main + rest;
 }
 
 int dcn_layer_forward(const dcn_problem* p, const void* x, const void* offset_weight, const void* offset_bias,
@@ -469,8 +474,9 @@ int dcn_layer_backward(const dcn_problem* p, const void* x, const void* offset, 
         int r = DCN_OK;
         if (dx != nullptr || doffset_weight != nullptr || doffset_bias != nullptr || dweight != nullptr)
             r = dcn::simt_small_layer_backward(g, gq, p->ndim, x, offset, offset_weight, weight, dy, dx, doffset_weight,
-                                               doffset_bias, dweight, st);
-        if (r == DCN_OK && dbias != nullptr) r = dcn::bias_grad(g, p->dtype, dy, dbias, st);
+                                               doffset_bias, dweight, dbias, st);
+        else if (dbias != nullptr)
+            r = dcn::bias_grad(g, p->dtype, dy, dbias, st);
         return r;
     }
     if (p->precision == DCN_PREC_EXACT) {
@@ -499,16 +505,17 @@ int dcn_layer_backward(const dcn_problem* p, const void* x, const void* offset, 
     if (!workspace_ok(ws, ws_bytes, dcn::tc_layer_workspace_bytes(g, gq, p->ndim, 3))) return DCN_ERR_WORKSPACE;
     if (x_channels_last != nullptr && !aligned(x_channels_last, 16)) return DCN_ERR_ALIGN;
     float* doff = nullptr;
+    bool bias_done = false, bias_off_done = false;
     int r = dcn::tc_layer_backward(g, gq, p->ndim, (const float*)x, (const float*)offset, (const float*)offset_weight,
                                    (const float*)weight, (const float*)dy, x_channels_last, (float*)dx,
-                                   (float*)doffset_weight, (float*)dweight, doffset_bias != nullptr ? &doff : nullptr, ws,
-                                   ws_bytes, st);
+                                   (float*)doffset_weight, (float*)doffset_bias, (float*)dweight, (float*)dbias, &doff,
+                                   &bias_done, &bias_off_done, ws, ws_bytes, st);
     if (r != DCN_OK) return r;
-    if (dbias != nullptr) {
+    if (dbias != nullptr && !bias_done) {
         r = dcn::bias_grad(g, p->dtype, dy, dbias, st);
         if (r != DCN_OK) return r;
     }
-    if (doffset_bias != nullptr) r = dcn::bias_grad(gq, p->dtype, doff, doffset_bias, st);
+    if (doffset_bias != nullptr && !bias_off_done) r = dcn::bias_grad(gq, p->dtype, doff, doffset_bias, st);
     return r;
 }
 

@@ -376,15 +376,15 @@ struct Acc<float, R, C> {
 };
 
 // ------------------------------------------------------------------------------------------------------------------
-// Prologue of a pass, one launch: block ranges for the input copy, the points, the weight and a zero fill.
+// Prologue of a pass, one launch: block ranges for the bias gradient, the input copy, the points, the weight and a zero fill.
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
 struct PrepArgs {
-    const T *x, *off, *w;
-    T *xcl, *wk, *zero;              // wk: w2 (forward) or wt (backward)
+    const T *x, *off, *w, *dy;
+    T *xcl, *wk, *zero, *dbias;      // wk: w2 (forward) or wt (backward)
     Entry<T>* pts;
     size_t zero_n;                   // elements
-    unsigned nx, np, nw, nz;         // blocks of each part
+    unsigned nb, nx, np, nw, nz;     // blocks of each part
     unsigned tx, ty;                 // input copy: tiles along the positions / channels
     unsigned bpk;                    // points: blocks of one (deformable group, tap)
     int backward;
@@ -395,6 +395,24 @@ __global__ void __launch_bounds__(kXThreads)
 exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
     __shared__ T tile[32][33];
     unsigned b = blockIdx.x;
+    if (b < a.nb) {                                                    // bias gradient: one output channel
+        T s = (T)0;
+        for (long long i = threadIdx.x; i < g.P; i += kXThreads) {
+            uint32_t n, opos;
+            g.d_ov.divmod((uint32_t)i, n, opos);
+            s += __ldg(a.dy + ((size_t)n * g.O + b) * g.ov + opos);
+        }
+        T* red = &tile[0][0];
+        red[threadIdx.x] = s;
+        __syncthreads();
+        for (int st = kXThreads / 2; st > 0; st >>= 1) {
+            if ((int)threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) a.dbias[b] = red[0];
+        return;
+    }
+    b -= a.nb;
     if (b < a.nx) {                                                    // x -> xcl, 32 channels x 32 positions
         const unsigned px = b % a.tx, r = b / a.tx, cy = r % a.ty, n = r / a.ty;
         const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
@@ -1244,6 +1262,7 @@ ExactLayout exact_layout(const Geom& g, const ExactGeom& x, int dtype, int defor
 
 template <typename T, int D>
 int launch_prep(const Geom& g, const ExactGeom& x, PrepArgs<T> a, cudaStream_t st) {
+    a.nb = a.dbias != nullptr ? (unsigned)g.O : 0u;
     a.nx = a.np = a.nw = a.nz = 0;
     a.bpk = 1;
     a.tx = (unsigned)((g.iv + 31) / 32);
@@ -1258,7 +1277,7 @@ int launch_prep(const Geom& g, const ExactGeom& x, PrepArgs<T> a, cudaStream_t s
         a.nw = (unsigned)((n + 4 * kXThreads - 1) / (4 * kXThreads));
     }
     if (a.zero != nullptr) a.nz = (unsigned)((a.zero_n * sizeof(T) + 64 * kXThreads - 1) / (64 * kXThreads));
-    const unsigned blocks = a.nx + a.np + a.nw + a.nz;
+    const unsigned blocks = a.nb + a.nx + a.np + a.nw + a.nz;
     if (blocks == 0) return 0;
     exact_prep_kernel<T, D><<<blocks, kXThreads, 0, st>>>(g, x, a);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
@@ -1340,13 +1359,14 @@ int run_forward(const Geom& g, const ExactGeom& x, const void* x_in, const void*
 // pass 1: backward data, 2: backward weight, 3: both.  add: dX and dW accumulate (else they are overwritten).
 template <typename T, int D, bool DEFORM, int V>
 int run_backward(const Geom& g, const ExactGeom& x, int pass, int add, const void* x_in, const void* off, const void* w,
-                 const void* dy, void* dx, void* doff, void* dw, uint8_t* ws, cudaStream_t st) {
+                 const void* dy, void* dx, void* doff, void* dw, void* db, uint8_t* ws, cudaStream_t st) {
     const int dtype = sizeof(T) == 8;
     const ExactLayout l = exact_layout(g, x, dtype, DEFORM, pass);
     const bool data = dx != nullptr || (DEFORM && doff != nullptr);
     PrepArgs<T> a = {};
     a.backward = 1;
-    a.x = (const T*)x_in; a.off = (const T*)off; a.w = (const T*)w;
+    a.x = (const T*)x_in; a.off = (const T*)off; a.w = (const T*)w; a.dy = (const T*)dy;
+    a.dbias = (T*)db;
     a.xcl = (DEFORM || dw != nullptr) ? (T*)(ws + l.xcl) : nullptr;
     a.pts = DEFORM ? (Entry<T>*)(ws + l.pts) : nullptr;
     a.wk = data ? (T*)(ws + l.wk) : nullptr;
@@ -1445,11 +1465,11 @@ int exact_forward(const Geom& g, int dtype, int ndim, int deform, const void* x_
 }
 
 int exact_backward(const Geom& g, int dtype, int ndim, int deform, int pass, int add, const void* x_in, const void* off,
-                   const void* w, const void* dy, void* dx, void* doff, void* dw, void* ws, cudaStream_t st) {
+                   const void* w, const void* dy, void* dx, void* doff, void* dw, void* db, void* ws, cudaStream_t st) {
     const ExactGeom x = exact_geom(g, dtype);
     uint8_t* b = (uint8_t*)ws;
-    if (dtype == 0) DCN_EXACT_D(run_backward, float, g, x, pass, add, x_in, off, w, dy, dx, doff, dw, b, st);
-    DCN_EXACT_D(run_backward, double, g, x, pass, add, x_in, off, w, dy, dx, doff, dw, b, st);
+    if (dtype == 0) DCN_EXACT_D(run_backward, float, g, x, pass, add, x_in, off, w, dy, dx, doff, dw, db, b, st);
+    DCN_EXACT_D(run_backward, double, g, x, pass, add, x_in, off, w, dy, dx, doff, dw, db, b, st);
 }
 
 }  // namespace dcn

@@ -21,14 +21,14 @@ bool simt_small_supported(const Geom& g, int dtype, int ndim, int deform);
 int simt_small_forward(const Geom& g, int ndim, const void* x, const void* off, const void* w, const void* bias,
                        void* y, cudaStream_t st);
 int simt_small_backward(const Geom& g, int ndim, const void* x, const void* off, const void* w, const void* dy,
-                        void* dx, void* doff, void* dw, cudaStream_t st);
+                        void* dx, void* doff, void* dw, void* db, cudaStream_t st);
 // fused layer forward for small problems: offsets computed in the kernel (gq: the offset-producing convolution)
 bool simt_small_layer_supported(const Geom& g, const Geom& gq, int dtype, int ndim);
 int simt_small_layer_forward(const Geom& g, const Geom& gq, int ndim, const void* x, const void* w_off, const void* b_off,
                              const void* w, const void* bias, void* offsets, void* y, cudaStream_t st);
 int simt_small_layer_backward(const Geom& g, const Geom& gq, int ndim, const void* x, const void* offsets,
                               const void* w_off, const void* w, const void* dy, void* dx, void* dw_off, void* db_off,
-                              void* dw, cudaStream_t st);
+                              void* dw, void* db, cudaStream_t st);
 bool simt_backward_both_supported(const Geom& g, int dtype);
 int simt_backward_both(const Geom& g, int ndim, int deform, const void* x, const void* off, const void* w,
                        const void* dy, void* dx, void* doff, void* dw, cudaStream_t st);
@@ -44,7 +44,7 @@ int exact_launch_count(int pass);
 int exact_forward(const Geom& g, int dtype, int ndim, int deform, const void* x, const void* off, const void* w,
                   const void* bias, void* y, void* ws, cudaStream_t st);
 int exact_backward(const Geom& g, int dtype, int ndim, int deform, int pass, int add, const void* x, const void* off,
-                   const void* w, const void* dy, void* dx, void* doff, void* dw, void* ws, cudaStream_t st);
+                   const void* w, const void* dy, void* dx, void* doff, void* dw, void* db, void* ws, cudaStream_t st);
 
 // BF16 tensor-core (tcgen05) path, dcn_tc.cu.  fp32 tensors only.
 bool tc_supported(const Geom& g, int ndim, int deform);
@@ -56,17 +56,19 @@ int tc_backward_data(const Geom& g, int ndim, int deform, const float* x, const 
 int tc_backward_weight(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* dy,
                        float* dw, void* ws, size_t ws_bytes, cudaStream_t st);
 size_t tc_backward_workspace_bytes(const Geom& g);
+// bias_done: whether dbias came out with the other gradients (it rides on the pass that packs dy)
 int tc_backward(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
-                const float* dy, const void* xcl_in, float* dx, float* doff, float* dw, void* ws, size_t ws_bytes,
-                cudaStream_t st);
+                const float* dy, const void* xcl_in, float* dx, float* doff, float* dw, float* dbias, bool* bias_done,
+                void* ws, size_t ws_bytes, cudaStream_t st);
 // deformable layer = offset-producing plain convolution (gq) + deformable convolution (g) of the same input
 size_t tc_layer_workspace_bytes(const Geom& g, const Geom& gq, int ndim, int pass);
 int tc_layer_forward(const Geom& g, const Geom& gq, int ndim, const float* x, const float* w_off, const float* b_off,
                      const float* w, const float* bias, float* offsets, float* y, void* ws, size_t ws_bytes,
                      cudaStream_t st);
 int tc_layer_backward(const Geom& g, const Geom& gq, int ndim, const float* x, const float* offsets, const float* w_off,
-                      const float* w, const float* dy, const void* xcl_in, float* dx, float* dw_off, float* dw,
-                      float** doff_out, void* ws, size_t ws_bytes, cudaStream_t st);
+                      const float* w, const float* dy, const void* xcl_in, float* dx, float* dw_off, float* db_off, float* dw,
+                      float* dbias, float** doff_out, bool* bias_done, bool* bias_off_done, void* ws, size_t ws_bytes,
+                      cudaStream_t st);
 int tc_forward_static(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
                       const float* bias, float* y, cudaStream_t st);
 size_t tc_static_scratch_bytes();

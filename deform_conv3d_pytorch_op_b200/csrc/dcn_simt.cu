@@ -464,10 +464,8 @@ simt_backward_both_kernel(const Geom g, const float* __restrict__ x, const float
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
-bias_grad_kernel(const Geom g, const T* __restrict__ dy, T* __restrict__ dbias) {
+__device__ __forceinline__ void bias_grad_block(const Geom& g, const T* __restrict__ dy, T* __restrict__ dbias, int o) {
     __shared__ T red[kThreads];
-    const int o = blockIdx.x;
     T s = (T)0;
     for (int n = 0; n < g.N; ++n) {
         const T* p = dy + ((size_t)n * g.O + o) * g.ov;
@@ -480,6 +478,12 @@ bias_grad_kernel(const Geom g, const T* __restrict__ dy, T* __restrict__ dbias) 
         __syncthreads();
     }
     if (threadIdx.x == 0) dbias[o] = red[0];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+bias_grad_kernel(const Geom g, const T* __restrict__ dy, T* __restrict__ dbias) {
+    bias_grad_block(g, dy, dbias, blockIdx.x);
 }
 
 // Same for a channels-last dy [N * ov positions][O]: a block sums one channel over all positions.
@@ -629,16 +633,16 @@ int simt_small_layer_forward(const Geom& g, const Geom& gq, int ndim, const void
 
 int simt_small_layer_backward(const Geom& g, const Geom& gq, int ndim, const void* x, const void* offsets,
                               const void* w_off, const void* w, const void* dy, void* dx, void* dw_off, void* db_off,
-                              void* dw, cudaStream_t st) {
+                              void* dw, void* db, cudaStream_t st) {
     const SmallLayer lay{(const float*)w_off, (float*)dw_off, (float*)db_off};
-    if (ndim == 2) return launch_small_backward<2>(g, (const float*)x, (const float*)offsets, (const float*)w, (const float*)dy, (float*)dx, nullptr, (float*)dw, st, &gq, &lay);
-    return launch_small_backward<3>(g, (const float*)x, (const float*)offsets, (const float*)w, (const float*)dy, (float*)dx, nullptr, (float*)dw, st, &gq, &lay);
+    if (ndim == 2) return launch_small_backward<2>(g, (const float*)x, (const float*)offsets, (const float*)w, (const float*)dy, (float*)dx, nullptr, (float*)dw, (float*)db, st, &gq, &lay);
+    return launch_small_backward<3>(g, (const float*)x, (const float*)offsets, (const float*)w, (const float*)dy, (float*)dx, nullptr, (float*)dw, (float*)db, st, &gq, &lay);
 }
 
 int simt_small_backward(const Geom& g, int ndim, const void* x, const void* off, const void* w, const void* dy,
-                        void* dx, void* doff, void* dw, cudaStream_t st) {
-    if (ndim == 2) return launch_small_backward<2>(g, (const float*)x, (const float*)off, (const float*)w, (const float*)dy, (float*)dx, (float*)doff, (float*)dw, st);
-    return launch_small_backward<3>(g, (const float*)x, (const float*)off, (const float*)w, (const float*)dy, (float*)dx, (float*)doff, (float*)dw, st);
+                        void* dx, void* doff, void* dw, void* db, cudaStream_t st) {
+    if (ndim == 2) return launch_small_backward<2>(g, (const float*)x, (const float*)off, (const float*)w, (const float*)dy, (float*)dx, (float*)doff, (float*)dw, (float*)db, st);
+    return launch_small_backward<3>(g, (const float*)x, (const float*)off, (const float*)w, (const float*)dy, (float*)dx, (float*)doff, (float*)dw, (float*)db, st);
 }
 
 // fp32 problems whose two backward grids together stay small take one launch for both passes (all outputs must be

@@ -532,19 +532,32 @@ int launch_small_forward(const Geom& g, const float* x, const float* off, const 
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
-// Zero fill of up to five output buffers in one launch; lets the dependent launch start at once.
+// Zero fill of up to five output buffers (16-byte stores but for the ends) and, in blocks behind it, the bias gradient,
+// in one launch; lets the dependent launch start at once.
 struct ZeroList {
-    float4* p[5];
-    size_t n4[5];
+    float* p[5];
+    size_t n[5];
+    unsigned blocks;                     // of the zero fill; one more per output channel follows where dbias is wanted
+    float* dbias;
 };
 __global__ void __launch_bounds__(256)
-small_zero_kernel(const ZeroList z) {
+small_zero_kernel(const Geom g, const float* __restrict__ dy, const ZeroList z) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    if (blockIdx.x >= z.blocks) {
+        bias_grad_block(g, dy, z.dbias, (int)(blockIdx.x - z.blocks));
+        return;
+    }
+    const size_t stride = (size_t)z.blocks * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int b = 0; b < 5; ++b)
-        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < z.n4[b]; i += stride) z.p[b][i] = zero;
+    for (int b = 0; b < 5; ++b) {
+        if (z.n[b] == 0) continue;
+        const size_t head = ((16 - (reinterpret_cast<uintptr_t>(z.p[b]) & 15)) & 15) / 4;
+        const size_t h = head < z.n[b] ? head : z.n[b], n4 = (z.n[b] - h) / 4, tail = z.n[b] - h - 4 * n4;
+        if (first < h) z.p[b][first] = 0.f;
+        if (first < tail) z.p[b][h + 4 * n4 + first] = 0.f;
+        for (size_t i = first; i < n4; i += stride) reinterpret_cast<float4*>(z.p[b] + h)[i] = zero;
+    }
 }
 
 inline bool small_pdl_enabled() {
@@ -553,13 +566,13 @@ inline bool small_pdl_enabled() {
 }
 
 // dX, dW (dOffset with several convolution groups; the offset-producing convolution's gradients in layer mode) are
-// zero-filled here: by one kernel when the buffers allow 16-byte stores, and then the main kernel is launched as its
-// programmatic dependent, so that its input-only prologue (weights, dy tile, sampling points) runs while the zero
-// fill is still in flight.
+// zero-filled here by one kernel, which also sums the bias gradient; the main kernel is launched as its programmatic
+// dependent, so that its input-only prologue (weights, dy tile, sampling points) runs while the zero fill is still in
+// flight.
 // lay / gq: null for the operator alone; else the layer's backward pass (doff is then not an output).
 template <int D>
 int launch_small_backward(const Geom& g, const float* x, const float* off, const float* w, const float* dy, float* dx,
-                          float* doff, float* dw, cudaStream_t st, const Geom* gq = nullptr,
+                          float* doff, float* dw, float* dbias, cudaStream_t st, const Geom* gq = nullptr,
                           const SmallLayer* lay = nullptr) {
     const SmallDims d = small_dims(g, D);
     const bool layer = lay != nullptr;
@@ -568,26 +581,19 @@ int launch_small_backward(const Geom& g, const float* x, const float* off, const
                       layer ? lay->db_off : nullptr};
     const size_t lens[5] = {(size_t)g.N * g.C * g.iv, (size_t)g.O * g.Cg * g.kv, (size_t)g.N * g.dg * g.kv * D * g.ov,
                             layer ? (size_t)gq->O * gq->Kg : 0, layer ? (size_t)gq->O : 0};
-    bool pdl = small_pdl_enabled();
+    const bool pdl = small_pdl_enabled();
     ZeroList z;
-    size_t most = 0;
+    size_t most = 4;
     for (int b = 0; b < 5; ++b) {
-        const size_t n = bufs[b] != nullptr ? lens[b] : 0;
-        if (n % 4 != 0 || (reinterpret_cast<uintptr_t>(bufs[b]) & 15) != 0) pdl = false;
-        z.p[b] = reinterpret_cast<float4*>(bufs[b]);
-        z.n4[b] = n / 4;
-        if (n / 4 > most) most = n / 4;
+        z.p[b] = bufs[b];
+        z.n[b] = bufs[b] != nullptr ? lens[b] : 0;
+        if (z.n[b] > most) most = z.n[b];
     }
-    if (pdl) {
-        size_t blocks = (most + 255) / 256;
-        if (blocks < 1) blocks = 1;
-        if (blocks > 296) blocks = 296;
-        small_zero_kernel<<<(unsigned)blocks, 256, 0, st>>>(z);
-        if (cudaGetLastError() != cudaSuccess) return -5;
-    } else {
-        for (int b = 0; b < 5; ++b)
-            if (bufs[b] != nullptr && cudaMemsetAsync(bufs[b], 0, lens[b] * sizeof(float), st) != cudaSuccess) return -5;
-    }
+    const size_t blocks = (most + 1023) / 1024;
+    z.blocks = (unsigned)(blocks > 296 ? 296 : blocks);
+    z.dbias = dbias;
+    small_zero_kernel<<<z.blocks + (dbias != nullptr ? (unsigned)g.O : 0u), 256, 0, st>>>(g, dy, z);
+    if (cudaGetLastError() != cudaSuccess) return -5;
     size_t smem = (size_t)d.smem_bwd;
     if (layer) smem += 4 * ((size_t)d.TP * (gq->Kg + 1) + (size_t)d.ndg * g.kv * D * gq->Kg);
     cudaLaunchConfig_t cfg = {};

@@ -16,6 +16,8 @@
 // Requirements (dcn_precision_supported): fp32 tensors, C/G and C/dg multiples of 8.
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "dcn_internal.h"
 #include "dcn_tc_common.cuh"
 
@@ -47,102 +49,6 @@ TcDims tc_dims(const Geom& g) {
     d.MB = (d.MT + 1) / 2;
     d.PT = (g.P + kTileN - 1) / kTileN;
     return d;
-}
-
-// ---------------------------------------------------------------------------------------------------
-// Pre-pass 1: NC(L)HW fp32 -> N(L)HWC bf16
-// ---------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-to_channels_last_bf16(const float* __restrict__ x, __nv_bfloat16* __restrict__ xcl, int C, int iv) {
-    // tile of 64 channels x 32 positions: 128-byte reads along the positions, 128-byte writes of bf16 pairs along
-    // the channels (C is a multiple of 8, so a pair never straddles the end)
-    __shared__ float tile[64][33];
-    const int n = blockIdx.z;
-    const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 64;
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-    const float* xn = x + (size_t)n * C * iv;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int c = c0 + ty + i * 8, p = p0 + tx;
-        tile[ty + i * 8][tx] = (c < C && p < iv) ? __ldg(xn + (size_t)c * iv + p) : 0.f;
-    }
-    __syncthreads();
-    uint32_t* on = reinterpret_cast<uint32_t*>(xcl + (size_t)n * iv * C);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int p = p0 + ty + i * 8, c = c0 + 2 * tx;
-        if (p < iv && c < C) on[((size_t)p * C + c) >> 1] = pack_bf16x2(tile[2 * tx][ty + i * 8], tile[2 * tx + 1][ty + i * 8]);
-    }
-}
-
-// ---------------------------------------------------------------------------------------------------
-// Pre-pass 2: weights.  Step one reorders and rounds the weight once, with coalesced reads and writes:
-//   W [O][Cg][kv] fp32  ->  Wt [O][kv * Cg] bf16,  GEMM-K order k' = tap * Cg + c
-// (a block takes one output channel and walks its row in pieces of 64 input channels through shared memory;
-// reading W directly in k' order would be a stride-kv gather, 8 to 27 times the traffic).  It also raises
-// *wmax_bits to the bit pattern of max|W| when asked to.  The operand tiles of the three passes are then cut out
-// of Wt, every tile row being a contiguous run of it.
-// ---------------------------------------------------------------------------------------------------
-constexpr int kWtChunk = 64;       // input channels per shared-memory piece
-
-__global__ void __launch_bounds__(256)
-weight_to_kmajor_bf16(const Geom g, const float* __restrict__ w, __nv_bfloat16* __restrict__ wt,
-                      unsigned int* __restrict__ wmax_bits) {
-    extern __shared__ float wrow[];                                  // [<= 64 channels][kv]
-    const int o = blockIdx.x;
-    const float* src = w + (size_t)o * g.Cg * g.kv;
-    __nv_bfloat16* dst = wt + (size_t)o * g.Kg;
-    float mx = 0.f;
-    {
-        const int c0 = blockIdx.y * kWtChunk;                        // one piece of 64 channels per block
-        const int nc = g.Cg - c0 < kWtChunk ? g.Cg - c0 : kWtChunk;
-        for (int i = threadIdx.x; i < nc * g.kv; i += blockDim.x) {
-            const float v = __ldg(src + (size_t)c0 * g.kv + i);
-            wrow[i] = v;
-            mx = fmaxf(mx, fabsf(v));
-        }
-        __syncthreads();
-        // pairs of channels of one tap: consecutive threads write consecutive 4-byte words of a tap's row segment
-        const int np = nc / 2;                                       // channel counts are multiples of 8
-        for (int i = threadIdx.x; i < np * g.kv; i += blockDim.x) {
-            const int tap = i / np, cp = i - tap * np;
-            const uint32_t v = pack_bf16x2(wrow[(2 * cp) * g.kv + tap], wrow[(2 * cp + 1) * g.kv + tap]);
-            *reinterpret_cast<uint32_t*>(dst + (size_t)tap * g.Cg + c0 + 2 * cp) = v;
-        }
-    }
-    if (wmax_bits != nullptr) {
-        const unsigned int m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-        if ((threadIdx.x & 31) == 0 && m != 0) atomicMax(wmax_bits, m);
-    }
-}
-
-size_t wt_bytes(const Geom& g) { return align_up((size_t)g.O * g.Kg * 2, 256); }
-
-int launch_weight_to_kmajor(const Geom& g, const float* w, __nv_bfloat16* wt, unsigned int* wmax_bits, cudaStream_t st) {
-    const int smem = kWtChunk * g.kv * (int)sizeof(float);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(weight_to_kmajor_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return -5;
-    weight_to_kmajor_bf16<<<dim3((unsigned)g.O, (unsigned)((g.Cg + kWtChunk - 1) / kWtChunk)), 256, smem, st>>>(g, w, wt, wmax_bits);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
-}
-
-// Wt -> swizzled K-major bf16 tiles [G][MT][KC][128 rows x 64 k'] of the forward pass.  Rows >= Og and
-// k' >= kv*Cg are zero.  One thread per 16-byte chunk (8 consecutive k').
-__global__ void __launch_bounds__(256)
-pack_weight_fwd(const Geom g, const __nv_bfloat16* __restrict__ wt, uint8_t* __restrict__ wpk, int MT, int KC) {
-    const int tile = blockIdx.x;                  // (j * MT + mt) * KC + kc
-    const int kc = tile % KC, mt = (tile / KC) % MT, j = tile / KC / MT;
-    uint8_t* dst = wpk + (size_t)tile * kTileBytes;
-    for (int e = threadIdx.x; e < 128 * 8; e += blockDim.x) {
-        const int row = e / 8, chunk = e % 8;
-        const int o = mt * 128 + row;
-        const int kp = kc * kTileK + chunk * 8;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (o < g.Og && kp < g.Kg)                // Kg is a multiple of 8: a chunk is inside or outside as a whole
-            v = __ldg(reinterpret_cast<const uint4*>(wt + (size_t)(j * g.Og + o) * g.Kg + kp));
-        *reinterpret_cast<uint4*>(dst + swz_offset(row, chunk)) = v;
-    }
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -187,53 +93,33 @@ __device__ __forceinline__ uint4 sample_chunk(const Geom& g, const __nv_bfloat16
 }
 
 int sm_count() {
-    int dev = 0, n = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 148;
+    constexpr int kMaxDevices = 64;
+    static volatile int count_of_device[kMaxDevices] = {};
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
+    int n = count_of_device[dev];
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+        count_of_device[dev] = n;              // racing first calls find the same number
+    }
+    return n;
 }
 
+#include "dcn_tc_passes.cuh"
 #include "dcn_tc_fwd_direct.cuh"
 #include "dcn_tc_sampler.cuh"
 #include "dcn_tc_fwd.cuh"
 
 struct FwdWorkspace {
-    size_t xcl_off, xcl_bytes, wpk_off, wpk_bytes, wt_off, total;
+    size_t xcl_off, wpk_off, total;
 };
 FwdWorkspace fwd_workspace(const Geom& g) {
     const TcDims d = tc_dims(g);
     FwdWorkspace w;
     w.xcl_off = 0;
-    w.xcl_bytes = align_up((size_t)g.N * g.iv * g.C * 2, 256);
-    w.wpk_off = w.xcl_bytes;
-    w.wpk_bytes = align_up((size_t)g.G * d.MT * d.KC * kTileBytes, 256);
-    w.wt_off = w.wpk_off + w.wpk_bytes;
-    w.total = w.wt_off + wt_bytes(g);
+    w.wpk_off = align_up((size_t)g.N * g.iv * g.C * 2, 256);
+    w.total = w.wpk_off + align_up((size_t)g.G * d.MT * d.KC * kTileBytes, 256);
     return w;
-}
-
-// fp32 -> bf16 of an input that already is channels-last (8 elements per thread; C is a multiple of 8)
-__global__ void __launch_bounds__(256)
-cast_bf16(const float* __restrict__ x, __nv_bfloat16* __restrict__ xcl, size_t n8) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(x) + 2 * i);
-        const float4 b = __ldg(reinterpret_cast<const float4*>(x) + 2 * i + 1);
-        reinterpret_cast<uint4*>(xcl)[i] = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w),
-                                                      pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
-    }
-}
-
-int launch_channels_last(const Geom& g, const float* x, __nv_bfloat16* xcl, cudaStream_t st) {
-    if (g.cl) {
-        if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return -7;      // vector loads
-        const size_t n8 = (size_t)g.N * g.iv * g.C / 8;
-        const size_t want = (n8 + 255) / 256;
-        const int blocks = (int)(want < (size_t)(8 * sm_count()) ? want : (size_t)(8 * sm_count()));
-        cast_bf16<<<blocks, 256, 0, st>>>(x, xcl, n8);
-        return cudaGetLastError() == cudaSuccess ? 0 : -5;
-    }
-    dim3 grid((unsigned)((g.iv + 31) / 32), (unsigned)((g.C + 63) / 64), (unsigned)g.N);
-    to_channels_last_bf16<<<grid, 256, 0, st>>>(x, xcl, g.C, g.iv);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 #include "dcn_tc_wgrad.cuh"
@@ -256,7 +142,9 @@ BwdWeightWorkspace bwd_weight_workspace(const Geom& g) {
 }
 
 struct BwdDataWorkspace {
-    size_t xcl_off, dpk_off, wpk_off, scale_off, wt_off, dxcl_off, dxcl_bytes, dwpk_off, gath_off, total;   // dwpk: fused backward only; gath: forward workspace of the transposed convolution
+    // dwpk, sums (row sums of the dy tiles, for the bias gradient): fused backward only; gath: forward workspace of the
+    // transposed convolution
+    size_t xcl_off, dpk_off, wpk_off, scale_off, dxcl_off, dxcl_bytes, dwpk_off, sums_off, gath_off, total;
 };
 size_t gather_dgrad_bytes(const Geom& g);      // 0 unless the problem can take the gather form (any ndim)
 BwdDataWorkspace bwd_data_workspace(const Geom& g) {
@@ -268,13 +156,13 @@ BwdDataWorkspace bwd_data_workspace(const Geom& g) {
     size_t wpk_bytes = (size_t)g.G * d.NB * d.OC * 2 * kTileBytes;
     if (g.Cg % 8 == 0 && b2_wpk_bytes(g) > wpk_bytes) wpk_bytes = b2_wpk_bytes(g);   // slab-wise tiles of dcn_tc_bwd2d.cuh
     w.scale_off = w.wpk_off + align_up(wpk_bytes, 256);
-    w.wt_off = w.scale_off + 256;                      // two words: bit patterns of max|dy| and max|W|
-    w.dxcl_off = w.wt_off + wt_bytes(g);
+    w.dxcl_off = w.scale_off + 256;                    // two words: bit patterns of max|dy| and max|W|
     w.dxcl_bytes = align_up((size_t)g.N * g.iv * g.C * 4, 256);
     // the shared-memory-accumulating kernel has no channels-last dX scratch; its sampling-point entries live there
     if (g.Cg % 8 == 0 && b2_points_bytes(g) > w.dxcl_bytes) w.dxcl_bytes = align_up(b2_points_bytes(g), 256);
     w.dwpk_off = w.dxcl_off + w.dxcl_bytes;
-    w.gath_off = w.dwpk_off + align_up(dwpk_bytes(g), 256);
+    w.sums_off = w.dwpk_off + align_up(dwpk_bytes(g), 256);
+    w.gath_off = w.sums_off + align_up((size_t)g.G * d.MT * 128 * d.PC2 * 4, 256);
     w.total = w.gath_off + gather_dgrad_bytes(g);
     return w;
 }
@@ -310,54 +198,11 @@ bool use_gather_dgrad(const Geom& g, int ndim, int deform, Geom& gt) {
     return !off && !deform && transposed_geom(g, ndim, gt);
 }
 
-// Wt'[c][tap' * Og + ol] = W[j*Og + ol][cl][kv - 1 - tap'] (c = j*Cg + cl) as bf16: the k-major weights of the
-// transposed convolution, in the layout pack_weight_fwd reads.
-__global__ void __launch_bounds__(256)
-weight_flip_to_kmajor_bf16(const Geom g, const float* __restrict__ w, __nv_bfloat16* __restrict__ wt) {
-    const long long total = (long long)g.C * g.kv * g.Og;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int ol = (int)(i % g.Og);
-        const long long r = i / g.Og;
-        const int tap = (int)(r % g.kv);
-        const int c = (int)(r / g.kv);
-        const int j = c / g.Cg, cl = c - j * g.Cg;
-        wt[i] = __float2bfloat16_rn(__ldg(w + ((size_t)(j * g.Og + ol) * g.Cg + cl) * g.kv + (g.kv - 1 - tap)));
-    }
-}
-
 size_t gather_dgrad_bytes(const Geom& g) {
     Geom gt;
     if (g.dg != 1 || g.cpg != g.C) return 0;                     // deformable problems never take it
     if (!transposed_geom(g, 3, gt)) return 0;
     return align_up(fwd_workspace(gt).total, 256);
-}
-
-// dX of a plain stride-1 convolution through the forward kernel.  add: dX already holds a partial result (the
-// layer's deformable part, or the accumulating entry point): the tiles are added to it with reductions.
-// dx_cl: dX is stored channels-last (it may differ from the layout of dy: the layer's dOffset is always channel-first).
-int run_gather_dgrad(const Geom& g, const Geom& gt, int ndim, const float* w, const float* dy, float* dx, bool add,
-                     bool dx_cl, void* ws, cudaStream_t st) {
-    const FwdWorkspace l = fwd_workspace(gt);
-    uint8_t* base = static_cast<uint8_t*>(ws);
-    __nv_bfloat16* dycl = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
-    uint8_t* wpk = base + l.wpk_off;
-    __nv_bfloat16* wt = reinterpret_cast<__nv_bfloat16*>(base + l.wt_off);
-    const TcDims d = tc_dims(gt);
-    int r = launch_channels_last(gt, dy, dycl, st);              // gt.cl == g.cl: dy has the layout of y
-    if (r != 0) return r;
-    {
-        const long long total = (long long)g.C * g.kv * g.Og;
-        const int blocks = (int)((total + 255) / 256 < 8ll * sm_count() ? (total + 255) / 256 : 8ll * sm_count());
-        weight_flip_to_kmajor_bf16<<<blocks, 256, 0, st>>>(g, w, wt);
-        if (cudaGetLastError() != cudaSuccess) return -5;
-    }
-    pack_weight_fwd<<<gt.G * d.MT * d.KC, 256, 0, st>>>(gt, wt, wpk, d.MT, d.KC);
-    if (cudaGetLastError() != cudaSuccess) return -5;
-    Geom gk = gt;
-    gk.cl = dx_cl ? 1 : 0;
-    // add: the tiles leave through reductions into the dX that is already there
-    return ndim == 2 ? launch_tc_forward<2, false>(gk, dycl, nullptr, wpk, nullptr, dx, st, add)
-                     : launch_tc_forward<3, false>(gk, dycl, nullptr, wpk, nullptr, dx, st, add);
 }
 
 // The shared-memory-accumulating backward-data kernel is taken whenever it fits (DCN_BWD2D=0 forces the
@@ -367,30 +212,107 @@ bool use_bwd2d(const Geom& g, int ndim, int deform) {
     return !off && b2_supported(g, ndim, deform);
 }
 
-// dy packed (max|dy| taken on the way), slab-wise weight tiles (max|W|), cleared dOffset, then the kernel.
-int run_bwd2d(const Geom& g, const __nv_bfloat16* xcl, const float* off, const float* w, const float* dy, uint8_t* dpk,
-              uint8_t* wpk, __nv_bfloat16* wt, unsigned int* scale, uint4* pts, float* dx, float* doff, bool accumulate,
-              cudaStream_t st) {
-    const B2Dims d = b2_dims(g);
-    {
-        const long long total = (long long)g.N * g.dg * g.kv * g.ov;
-        const long long want = (total + 255) / 256;
-        const int blocks = (int)(want < 16ll * sm_count() ? want : 16ll * sm_count());
-        b2_points_kernel<<<blocks, 256, 0, st>>>(g, off, pts, d.Wp, d.W2);
-        if (cudaGetLastError() != cudaSuccess) return -5;
+// The gradient kernels of one convolution and the passes around them: `prologue` adds what has to be done before them
+// (it may enqueue a memset), `run` launches them, `epilogue` adds what turns their scratch into the caller's tensors.
+// The caller launches the passes, together with those of another convolution where it has one.
+struct Backward {
+    const Geom& g;
+    int ndim, deform;
+    bool add;                            // dX and dW accumulate (else they are overwritten)
+    const float *off, *w, *dy;
+    float *dx, *doff, *dw, *dbias;
+    bool dx_cl;                          // dX is stored channels-last (g.cl says so of dy)
+    bool dx_partial;                     // dX holds a partial result already (add, for dX alone)
+    const __nv_bfloat16* xcl;
+    uint8_t* base;
+    BwdDataWorkspace l;
+    DgDims d;
+    bool b2, gather, scatter, tiles, bias_here;
+    Geom gt, gk;                         // transposed convolution; with the layout of dX
+    FwdPlan plan;                        // of the gather
+
+    Backward(const Geom& g_, int ndim_, int deform_, bool add_, const float* off_, const float* w_, const float* dy_, float* dx_,
+             float* doff_, float* dw_, float* dbias_, void* ws)
+        : g(g_), ndim(ndim_), deform(deform_), add(add_), off(off_), w(w_), dy(dy_), dx(dx_), doff(deform_ ? doff_ : nullptr),
+          dw(dw_), dbias(dbias_), dx_cl(g_.cl != 0), dx_partial(add_), xcl(nullptr), base(static_cast<uint8_t*>(ws)),
+          l(bwd_data_workspace(g_)), d(dg_dims(g_)) {
+        const bool data = dx != nullptr || doff != nullptr;
+        b2 = data && use_bwd2d(g, ndim, deform);
+        gather = !b2 && dx != nullptr && use_gather_dgrad(g, ndim, deform, gt);
+        scatter = data && !b2 && !gather;
+        tiles = b2 || scatter || dw != nullptr;
+        bias_here = dbias != nullptr && tiles;
     }
-    if (cudaMemsetAsync(scale, 0, 8, st) != cudaSuccess) return -5;
-    int r = launch_pack_dy(g, dy, dpk, d.MT, d.PC, st, scale);
-    if (r != 0) return r;
-    r = launch_weight_to_kmajor(g, w, wt, scale + 1, st);
-    if (r != 0) return r;
-    pack_weight_slab<<<g.G * d.SL * d.OC, 256, 0, st>>>(g, wt, wpk, d.SL, d.OC);
-    if (cudaGetLastError() != cudaSuccess) return -5;
-    if (doff != nullptr &&
-        cudaMemsetAsync(doff, 0, (size_t)g.N * g.dg * g.kv * 2 * g.ov * sizeof(float), st) != cudaSuccess)
-        return -5;
-    return launch_tc_bwd2d(g, xcl, pts, dpk, wpk, scale, dx, doff, accumulate, st);
-}
+    __nv_bfloat16* own_xcl() const { return reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off); }
+    bool needs_x() const { return dw != nullptr || (deform && (b2 || scatter)); }
+    unsigned int* scale() const { return reinterpret_cast<unsigned int*>(base + l.scale_off); }
+    float* dxcl() const {                // scatter target: a channels-last dX itself, else the scratch
+        return dx == nullptr ? nullptr : (dx_cl ? dx : reinterpret_cast<float*>(base + l.dxcl_off));
+    }
+    float* sums() const { return bias_here ? reinterpret_cast<float*>(base + l.sums_off) : nullptr; }
+
+    // what depends on the weight and the offsets only (`before`), and what needs dy (`with_dy`)
+    int before(Passes& p, cudaStream_t st) {
+        if (b2) {
+            const B2Dims e = b2_dims(g);
+            if (cudaMemsetAsync(scale(), 0, 8, st) != cudaSuccess) return -5;
+            p.points(g, off, reinterpret_cast<uint4*>(base + l.dxcl_off), e.Wp, e.W2);
+            p.weight(g, kTilesSlab, w, base + l.wpk_off, scale() + 1);
+        }
+        if (scatter) {
+            if (dx_cl && dx != nullptr && (reinterpret_cast<uintptr_t>(dx) & 15) != 0) return -7;   // 16-byte reductions
+            p.weight(g, kTilesBwd, w, base + l.wpk_off);
+            if (dx != nullptr && !(dx_cl && dx_partial)) p.zero(dxcl(), (size_t)g.N * g.iv * g.C);
+        }
+        if (doff != nullptr) p.zero(doff, (size_t)g.N * g.dg * g.kv * ndim * g.ov);
+        if (gather) {
+            const FwdWorkspace f = fwd_workspace(gt);
+            gk = gt;
+            gk.cl = dx_cl ? 1 : 0;
+            plan = fwd_plan(gk, ndim, 0, dx, dx_partial);
+            if (plan.direct && dx_partial) return -5;
+            p.weight(g, kTilesFlip, w, base + l.gath_off + f.wpk_off);
+            add_zeros(p, plan);
+        }
+        return 0;
+    }
+    void with_dy(Passes& p) {
+        if (tiles) p.pack_dy(g, dy, base + l.dpk_off, d.MT, d.PC2, b2 ? scale() : nullptr, sums());
+        if (gather) p.copy_x(gt, dy, reinterpret_cast<__nv_bfloat16*>(base + l.gath_off + fwd_workspace(gt).xcl_off));
+    }
+    int run(cudaStream_t st) {
+        int r = 0;
+        const uint8_t* dpk = base + l.dpk_off;
+        if (b2)
+            r = launch_tc_bwd2d(g, xcl, reinterpret_cast<uint4*>(base + l.dxcl_off), dpk, base + l.wpk_off, scale(), dx, doff,
+                                dx_partial, st);
+        if (scatter) {
+            if (ndim == 2) r = deform ? launch_tc_dgrad<2, true>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, st)
+                                      : launch_tc_dgrad<2, false>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, st);
+            else r = deform ? launch_tc_dgrad<3, true>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, st)
+                            : launch_tc_dgrad<3, false>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, st);
+        }
+        if (r == 0 && gather) {
+            const FwdWorkspace f = fwd_workspace(gt);
+            r = launch_tc_forward(gk, plan, ndim, 0, reinterpret_cast<const __nv_bfloat16*>(base + l.gath_off + f.xcl_off), nullptr,
+                                  base + l.gath_off + f.wpk_off, nullptr, dx, st);
+        }
+        if (r == 0 && dw != nullptr) {   // the weight kernel reads dy tiles with the same layout and stride (PC2 == wg_dims().PC)
+            float* dwpk = reinterpret_cast<float*>(base + l.dwpk_off);
+            if (ndim == 2) r = deform ? launch_tc_wgrad<2, true>(g, xcl, off, dpk, dwpk, st)
+                                      : launch_tc_wgrad<2, false>(g, xcl, off, dpk, dwpk, st);
+            else r = deform ? launch_tc_wgrad<3, true>(g, xcl, off, dpk, dwpk, st)
+                            : launch_tc_wgrad<3, false>(g, xcl, off, dpk, dwpk, st);
+        }
+        return r;
+    }
+    bool folds_dx() const { return scatter && dx != nullptr && !dx_cl; }
+    void fold_dx(Passes& p) const { if (folds_dx()) p.fold_dx(g, dxcl(), dx, dx_partial); }
+    void epilogue(Passes& p) const {
+        if (dw != nullptr) add_dw_fold(p, g, reinterpret_cast<const float*>(base + l.dwpk_off), dw, add);
+        if (bias_here) p.fold_bias(g, sums(), dbias, d.MT, d.PC2);
+    }
+};
 
 }  // namespace
 
@@ -414,17 +336,13 @@ int tc_launch_count(const Geom& g, int ndim, int deform, int pass) {
     const bool b2 = use_bwd2d(g, ndim, deform);
     Geom gt;
     const bool gather = use_gather_dgrad(g, ndim, deform, gt);
-    if (pass == 0) return 4;      // channels-last copy, weight reorder, weight tiles, implicit GEMM
-    if (gather && pass == 1) return 4;      // dy copy, mirrored weights, weight tiles, forward kernel on dy (adds into dX)
-    if (gather && pass == 3) return 8;      // the first four of those + input copy, dy pack, wgrad, dW unpack
-    if (pass == 1) {
-        if (b2) return 6;         // input copy, sampling points, dy pack, weight reorder, slab tiles, GEMM + scatter
-        return g.cl ? 5 : 6;      // input copy, dy pack, weight reorder, weight tiles, GEMM + scatter, (dx transpose-add)
-    }
-    if (pass == 2) return 4;      // channels-last copy, dy pack, implicit GEMM, dW unpack
-    // fused backward (input copy taken over from the forward pass when the caller hands it in: counted here)
-    if (b2) return 8;             // input copy, points, dy pack, weight reorder, slab tiles, dgrad, wgrad, dW unpack
-    return g.cl ? 7 : 8;          // input copy, dy pack, weight reorder, weight tiles, dgrad, (dx transpose,) wgrad, dW unpack
+    if (pass == 0) return 2;                               // prologue, implicit GEMM
+    if (pass == 1) return b2 || gather || g.cl ? 2 : 3;    // prologue, GEMM + scatter (or gather), (dX transpose)
+    if (pass == 2) return 3;                               // prologue, implicit GEMM, dW fold
+    // fused backward without the forward pass's workspace: the jobs of the prologue one by one, two GEMMs, epilogue
+    if (b2) return 8;                                      // points, slab tiles, zero fill, dy pack, input copy
+    if (gather) return 7 + fwd_plan(gt, ndim, 0, nullptr, false).zeros;   // mirrored tiles, (zero fill,) dy pack, dy copy, input copy
+    return 7;                                              // weight tiles, zero fill, dy pack, input copy
 }
 
 int tc_debug_points(const Geom& g, int ndim, int deform, const float* off, int n, float* coords, int32_t* valid,
@@ -434,96 +352,50 @@ int tc_debug_points(const Geom& g, int ndim, int deform, const float* off, int n
     if (ws_bytes < l.total) return -4;
     uint4* pts = reinterpret_cast<uint4*>(static_cast<uint8_t*>(ws) + l.dxcl_off);
     const B2Dims d = b2_dims(g);
-    const long long total = (long long)g.N * g.dg * g.kv * g.ov;
-    const long long want = (total + 255) / 256;
+    Passes p;
+    p.points(g, off, pts, d.Wp, d.W2);
+    const int r = p.launch(st);
+    if (r != 0) return r;
+    const long long want = ((long long)g.dg * g.kv * g.ov + 255) / 256;
     const int blocks = (int)(want < 16ll * sm_count() ? want : 16ll * sm_count());
-    b2_points_kernel<<<blocks, 256, 0, st>>>(g, off, pts, d.Wp, d.W2);
-    if (cudaGetLastError() != cudaSuccess) return -5;
     b2_points_decode_kernel<<<blocks, 256, 0, st>>>(g, pts, n, d.Wp, d.W2, coords, valid, lo, hi);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
-// `xcl_in`: a channels-last bf16 copy of x that already exists (the workspace's own copy is then not built).
-static int tc_forward_x(const Geom& g, int ndim, int deform, const float* x, const __nv_bfloat16* xcl_in, const float* off,
-                        const float* w, const float* bias, float* y, void* ws, size_t ws_bytes, cudaStream_t st) {
+int tc_forward(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
+               const float* bias, float* y, void* ws, size_t ws_bytes, cudaStream_t st) {
     const FwdWorkspace l = fwd_workspace(g);
     if (ws_bytes < l.total) return -4;
     uint8_t* base = static_cast<uint8_t*>(ws);
-    const __nv_bfloat16* xcl = xcl_in;
+    __nv_bfloat16* xcl = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
     uint8_t* wpk = base + l.wpk_off;
-    const TcDims d = tc_dims(g);
-    int r = 0;
-    if (xcl == nullptr) {
-        __nv_bfloat16* mine = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
-        r = launch_channels_last(g, x, mine, st);
-        if (r != 0) return r;
-        xcl = mine;
-    }
-    __nv_bfloat16* wt = reinterpret_cast<__nv_bfloat16*>(base + l.wt_off);
-    r = launch_weight_to_kmajor(g, w, wt, nullptr, st);
+    const FwdPlan plan = fwd_plan(g, ndim, deform, y, false);
+    Passes p;
+    p.copy_x(g, x, xcl);
+    p.weight(g, kTilesFwd, w, wpk);
+    add_zeros(p, plan);
+    const int r = p.launch(st);
     if (r != 0) return r;
-    pack_weight_fwd<<<g.G * d.MT * d.KC, 256, 0, st>>>(g, wt, wpk, d.MT, d.KC);
-    if (cudaGetLastError() != cudaSuccess) return -5;
-    if (ndim == 2) return deform ? launch_tc_forward<2, true>(g, xcl, off, wpk, bias, y, st)
-                                 : launch_tc_forward<2, false>(g, xcl, off, wpk, bias, y, st);
-    return deform ? launch_tc_forward<3, true>(g, xcl, off, wpk, bias, y, st)
-                  : launch_tc_forward<3, false>(g, xcl, off, wpk, bias, y, st);
-}
-
-int tc_forward(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
-               const float* bias, float* y, void* ws, size_t ws_bytes, cudaStream_t st) {
-    return tc_forward_x(g, ndim, deform, x, nullptr, off, w, bias, y, ws, ws_bytes, st);
+    return launch_tc_forward(g, plan, ndim, deform, xcl, off, wpk, bias, y, st);
 }
 
 int tc_backward_data(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
                      const float* dy, float* dx, float* doff, void* ws, size_t ws_bytes, cudaStream_t st) {
-    const BwdDataWorkspace l = bwd_data_workspace(g);
-    if (ws_bytes < l.total) return -4;
-    uint8_t* base = static_cast<uint8_t*>(ws);
-    __nv_bfloat16* xcl = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
-    uint8_t* dpk = base + l.dpk_off;
-    uint8_t* wpk = base + l.wpk_off;
-    if (g.cl && dx != nullptr && (reinterpret_cast<uintptr_t>(dx) & 15) != 0) return -7;   // 16-byte reductions
-    // a channels-last dx is the scatter target itself (this entry point accumulates into dx)
-    float* dxcl = dx == nullptr ? nullptr : (g.cl ? dx : reinterpret_cast<float*>(base + l.dxcl_off));
-    if (!deform) doff = nullptr;
-    const DgDims d = dg_dims(g);
-    int r = 0;
-    if (deform) {
-        r = launch_channels_last(g, x, xcl, st);
-        if (r != 0) return r;
-    }
-    if (use_bwd2d(g, ndim, deform))
-        return run_bwd2d(g, xcl, off, w, dy, dpk, wpk, reinterpret_cast<__nv_bfloat16*>(base + l.wt_off),
-                         reinterpret_cast<unsigned int*>(base + l.scale_off),
-                         reinterpret_cast<uint4*>(base + l.dxcl_off), dx, doff, true, st);
-    {
-        Geom gt;
-        if (dx != nullptr && use_gather_dgrad(g, ndim, deform, gt))          // plain, stride 1: a gather, added to dx
-            return run_gather_dgrad(g, gt, ndim, w, dy, dx, true, g.cl != 0, base + l.gath_off, st);
-    }
-    r = launch_pack_dy(g, dy, dpk, d.MT, d.PC2, st);
+    if (ws_bytes < bwd_data_workspace(g).total) return -4;
+    Backward b(g, ndim, deform, true, off, w, dy, dx, doff, nullptr, nullptr, ws);     // accumulates into dX
+    Passes p;
+    int r = b.before(p, st);
     if (r != 0) return r;
-    r = launch_weight_to_kmajor(g, w, reinterpret_cast<__nv_bfloat16*>(base + l.wt_off), nullptr, st);
-    if (r != 0) return r;
-    pack_weight_bwd<<<g.G * d.NB * d.OC, 256, 0, st>>>(g, reinterpret_cast<const __nv_bfloat16*>(base + l.wt_off), wpk,
-                                                       d.NB, d.OC);
-    if (cudaGetLastError() != cudaSuccess) return -5;
-    if (dxcl != nullptr && !g.cl && cudaMemsetAsync(dxcl, 0, (size_t)g.N * g.iv * g.C * 4, st) != cudaSuccess) return -5;
-    if (doff != nullptr &&
-        cudaMemsetAsync(doff, 0, (size_t)g.N * g.dg * g.kv * ndim * g.ov * sizeof(float), st) != cudaSuccess)
-        return -5;
-    if (ndim == 2) r = deform ? launch_tc_dgrad<2, true>(g, xcl, off, dpk, wpk, dxcl, doff, st)
-                              : launch_tc_dgrad<2, false>(g, xcl, off, dpk, wpk, dxcl, doff, st);
-    else r = deform ? launch_tc_dgrad<3, true>(g, xcl, off, dpk, wpk, dxcl, doff, st)
-                    : launch_tc_dgrad<3, false>(g, xcl, off, dpk, wpk, dxcl, doff, st);
-    if (r != 0) return r;
-    if (dx != nullptr && !g.cl) {
-        dim3 grid((unsigned)((g.iv + 31) / 32), (unsigned)((g.C + 31) / 32), (unsigned)g.N);
-        from_channels_last<true><<<grid, 256, 0, st>>>(dxcl, dx, g.C, g.iv);
-        if (cudaGetLastError() != cudaSuccess) return -5;
+    b.with_dy(p);
+    if (b.needs_x()) {
+        p.copy_x(g, x, b.own_xcl());
+        b.xcl = b.own_xcl();
     }
-    return 0;
+    r = p.launch(st);
+    if (r == 0) r = b.run(st);
+    Passes q;
+    b.fold_dx(q);
+    return r != 0 ? r : q.launch(st);
 }
 
 int tc_backward_weight(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* dy,
@@ -534,9 +406,10 @@ int tc_backward_weight(const Geom& g, int ndim, int deform, const float* x, cons
     __nv_bfloat16* xcl = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
     uint8_t* dpk = base + l.dpk_off;
     const WgDims d = wg_dims(g);
-    int r = launch_channels_last(g, x, xcl, st);
-    if (r != 0) return r;
-    r = launch_pack_dy(g, dy, dpk, d.MT, d.PC, st);
+    Passes p;
+    p.copy_x(g, x, xcl);
+    p.pack_dy(g, dy, dpk, d.MT, d.PC, nullptr, nullptr);
+    int r = p.launch(st);
     if (r != 0) return r;
     float* dwpk = reinterpret_cast<float*>(base + l.dwpk_off);
     if (ndim == 2) r = deform ? launch_tc_wgrad<2, true>(g, xcl, off, dpk, dwpk, st)
@@ -544,7 +417,9 @@ int tc_backward_weight(const Geom& g, int ndim, int deform, const float* x, cons
     else r = deform ? launch_tc_wgrad<3, true>(g, xcl, off, dpk, dwpk, st)
                     : launch_tc_wgrad<3, false>(g, xcl, off, dpk, dwpk, st);
     if (r != 0) return r;
-    return dwpk_fold<true>(g, dwpk, dw, st);         // this entry point accumulates into dW
+    Passes q;
+    add_dw_fold(q, g, dwpk, dw, true);               // this entry point accumulates into dW
+    return q.launch(st);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -555,76 +430,28 @@ int tc_backward_weight(const Geom& g, int ndim, int deform, const float* x, cons
 size_t tc_backward_workspace_bytes(const Geom& g) { return bwd_data_workspace(g).total; }
 
 int tc_backward(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
-                const float* dy, const void* xcl_in, float* dx, float* doff, float* dw, void* ws, size_t ws_bytes,
-                cudaStream_t st) {
-    const BwdDataWorkspace l = bwd_data_workspace(g);
-    if (ws_bytes < l.total) return -4;
-    uint8_t* base = static_cast<uint8_t*>(ws);
-    const __nv_bfloat16* xcl = static_cast<const __nv_bfloat16*>(xcl_in);
-    uint8_t* dpk = base + l.dpk_off;
-    uint8_t* wpk = base + l.wpk_off;
-    if (g.cl && dx != nullptr && (reinterpret_cast<uintptr_t>(dx) & 15) != 0) return -7;   // 16-byte reductions
-    // a channels-last dx is the scatter target itself (zero-filled here: this entry point overwrites)
-    float* dxcl = dx == nullptr ? nullptr : (g.cl ? dx : reinterpret_cast<float*>(base + l.dxcl_off));
-    if (!deform) doff = nullptr;
-    const DgDims d = dg_dims(g);
-    int r = 0;
-    const bool need_x = dw != nullptr || (deform && (dx != nullptr || doff != nullptr));
-    if (xcl == nullptr && need_x) {
-        __nv_bfloat16* mine = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
-        r = launch_channels_last(g, x, mine, st);
-        if (r != 0) return r;
-        xcl = mine;
+                const float* dy, const void* xcl_in, float* dx, float* doff, float* dw, float* dbias, bool* bias_done,
+                void* ws, size_t ws_bytes, cudaStream_t st) {
+    if (ws_bytes < bwd_data_workspace(g).total) return -4;
+    Backward b(g, ndim, deform, false, off, w, dy, dx, doff, dw, dbias, ws);
+    *bias_done = b.bias_here;
+    Passes p;
+    int r = b.before(p, st);
+    if (r != 0) return r;
+    b.with_dy(p);
+    b.xcl = static_cast<const __nv_bfloat16*>(xcl_in);
+    if (b.xcl == nullptr && b.needs_x()) {
+        p.copy_x(g, x, b.own_xcl());
+        b.xcl = b.own_xcl();
     }
-    const bool b2 = (dx != nullptr || doff != nullptr) && use_bwd2d(g, ndim, deform);
-    if (b2) {
-        r = run_bwd2d(g, xcl, off, w, dy, dpk, wpk, reinterpret_cast<__nv_bfloat16*>(base + l.wt_off),
-                      reinterpret_cast<unsigned int*>(base + l.scale_off),
-                      reinterpret_cast<uint4*>(base + l.dxcl_off), dx, doff, false, st);
-        if (r != 0) return r;
-    } else {
-        r = launch_pack_dy(g, dy, dpk, d.MT, d.PC2, st);
-        if (r != 0) return r;
-    }
-    Geom gt;
-    const bool gather = !b2 && dx != nullptr && use_gather_dgrad(g, ndim, deform, gt);
-    if (gather) {                                                          // plain, stride 1: dX as a gather
-        r = run_gather_dgrad(g, gt, ndim, w, dy, dx, false, g.cl != 0, base + l.gath_off, st);
-        if (r != 0) return r;
-    }
-    if (!b2 && !gather && (dx != nullptr || doff != nullptr)) {
-        r = launch_weight_to_kmajor(g, w, reinterpret_cast<__nv_bfloat16*>(base + l.wt_off), nullptr, st);
-        if (r != 0) return r;
-        pack_weight_bwd<<<g.G * d.NB * d.OC, 256, 0, st>>>(g, reinterpret_cast<const __nv_bfloat16*>(base + l.wt_off), wpk,
-                                                           d.NB, d.OC);
-        if (cudaGetLastError() != cudaSuccess) return -5;
-        if (dxcl != nullptr && cudaMemsetAsync(dxcl, 0, (size_t)g.N * g.iv * g.C * 4, st) != cudaSuccess) return -5;
-        if (doff != nullptr &&
-            cudaMemsetAsync(doff, 0, (size_t)g.N * g.dg * g.kv * ndim * g.ov * sizeof(float), st) != cudaSuccess)
-            return -5;
-        if (ndim == 2) r = deform ? launch_tc_dgrad<2, true>(g, xcl, off, dpk, wpk, dxcl, doff, st)
-                                  : launch_tc_dgrad<2, false>(g, xcl, off, dpk, wpk, dxcl, doff, st);
-        else r = deform ? launch_tc_dgrad<3, true>(g, xcl, off, dpk, wpk, dxcl, doff, st)
-                        : launch_tc_dgrad<3, false>(g, xcl, off, dpk, wpk, dxcl, doff, st);
-        if (r != 0) return r;
-        if (dx != nullptr && !g.cl) {
-            dim3 grid((unsigned)((g.iv + 31) / 32), (unsigned)((g.C + 31) / 32), (unsigned)g.N);
-            from_channels_last<false><<<grid, 256, 0, st>>>(dxcl, dx, g.C, g.iv);
-            if (cudaGetLastError() != cudaSuccess) return -5;
-        }
-    }
-    if (dw != nullptr) {
-        float* dwpk = reinterpret_cast<float*>(base + l.dwpk_off);
-        // the weight kernel reads dy tiles with the same layout and stride (PC2 == wg_dims().PC)
-        if (ndim == 2) r = deform ? launch_tc_wgrad<2, true>(g, xcl, off, dpk, dwpk, st)
-                                  : launch_tc_wgrad<2, false>(g, xcl, off, dpk, dwpk, st);
-        else r = deform ? launch_tc_wgrad<3, true>(g, xcl, off, dpk, dwpk, st)
-                        : launch_tc_wgrad<3, false>(g, xcl, off, dpk, dwpk, st);
-        if (r != 0) return r;
-        r = dwpk_fold<false>(g, dwpk, dw, st);       // the fused entry point overwrites dW
-        if (r != 0) return r;
-    }
-    return 0;
+    // (a call on its own keeps its passes apart, one name each on a profiler's timeline)
+    r = p.launch(st, xcl_in == nullptr);
+    if (r == 0) r = b.run(st);
+    if (r != 0) return r;
+    Passes q;
+    b.fold_dx(q);
+    b.epilogue(q);
+    return q.launch(st);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -649,84 +476,72 @@ int tc_layer_forward(const Geom& g, const Geom& gq, int ndim, const float* x, co
                      const float* w, const float* bias, float* offsets, float* y, void* ws, size_t ws_bytes,
                      cudaStream_t st) {
     if (ws_bytes < tc_layer_workspace_bytes(g, gq, ndim, 0)) return -4;
+    const FwdWorkspace l = fwd_workspace(g), lq = fwd_workspace(gq);
     uint8_t* base = static_cast<uint8_t*>(ws);
-    const size_t main_bytes = align_up(fwd_workspace(g).total, 256);
-    __nv_bfloat16* xcl = reinterpret_cast<__nv_bfloat16*>(base + fwd_workspace(g).xcl_off);
-    int r = launch_channels_last(g, x, xcl, st);
+    uint8_t* baseq = base + align_up(l.total, 256);
+    __nv_bfloat16* xcl = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
+    const FwdPlan pq = fwd_plan(gq, ndim, 0, offsets, false), pl = fwd_plan(g, ndim, 1, y, false);
+    Passes p;
+    p.copy_x(g, x, xcl);
+    p.weight(gq, kTilesFwd, w_off, baseq + lq.wpk_off);
+    p.weight(g, kTilesFwd, w, base + l.wpk_off);
+    add_zeros(p, pq);
+    add_zeros(p, pl);
+    int r = p.launch(st);
     if (r != 0) return r;
-    r = tc_forward_x(gq, ndim, 0, x, xcl, nullptr, w_off, b_off, offsets, base + main_bytes, ws_bytes - main_bytes, st);
+    r = launch_tc_forward(gq, pq, ndim, 0, xcl, nullptr, baseq + lq.wpk_off, b_off, offsets, st);
     if (r != 0) return r;
-    return tc_forward_x(g, ndim, 1, x, xcl, offsets, w, bias, y, base, main_bytes, st);
-}
-
-// Gradients of the offset-producing convolution given dOffset: its input gradient is ADDED to dx (which the
-// deformable part has already written, in the layout of g), its weight gradient overwrites dw_off.
-static int plain_backward_into(const Geom& gq, int ndim, bool dx_channels_last, const __nv_bfloat16* xcl,
-                               const float* w_off, const float* dyq, float* dx, float* dw_off, void* ws,
-                               cudaStream_t st) {
-    const BwdDataWorkspace l = bwd_data_workspace(gq);
-    uint8_t* base = static_cast<uint8_t*>(ws);
-    uint8_t* dpk = base + l.dpk_off;
-    uint8_t* wpk = base + l.wpk_off;
-    const DgDims d = dg_dims(gq);
-    int r = launch_pack_dy(gq, dyq, dpk, d.MT, d.PC2, st);
-    if (r != 0) return r;
-    Geom gt;
-    if (dx != nullptr && use_gather_dgrad(gq, ndim, 0, gt)) {      // stride 1: a gather, added to the dX already there
-        r = run_gather_dgrad(gq, gt, ndim, w_off, dyq, dx, true, dx_channels_last, base + l.gath_off, st);
-        if (r != 0) return r;
-        dx = nullptr;                                              // done
-    }
-    if (dx != nullptr) {
-        __nv_bfloat16* wt = reinterpret_cast<__nv_bfloat16*>(base + l.wt_off);
-        r = launch_weight_to_kmajor(gq, w_off, wt, nullptr, st);
-        if (r != 0) return r;
-        pack_weight_bwd<<<gq.G * d.NB * d.OC, 256, 0, st>>>(gq, wt, wpk, d.NB, d.OC);
-        if (cudaGetLastError() != cudaSuccess) return -5;
-        float* dxcl = dx_channels_last ? dx : reinterpret_cast<float*>(base + l.dxcl_off);
-        if (!dx_channels_last && cudaMemsetAsync(dxcl, 0, (size_t)gq.N * gq.iv * gq.C * 4, st) != cudaSuccess) return -5;
-        r = ndim == 2 ? launch_tc_dgrad<2, false>(gq, xcl, nullptr, dpk, wpk, dxcl, nullptr, st)
-                      : launch_tc_dgrad<3, false>(gq, xcl, nullptr, dpk, wpk, dxcl, nullptr, st);
-        if (r != 0) return r;
-        if (!dx_channels_last) {
-            dim3 grid((unsigned)((gq.iv + 31) / 32), (unsigned)((gq.C + 31) / 32), (unsigned)gq.N);
-            from_channels_last<true><<<grid, 256, 0, st>>>(dxcl, dx, gq.C, gq.iv);
-            if (cudaGetLastError() != cudaSuccess) return -5;
-        }
-    }
-    if (dw_off != nullptr) {
-        float* dwpk = reinterpret_cast<float*>(base + l.dwpk_off);
-        r = ndim == 2 ? launch_tc_wgrad<2, false>(gq, xcl, nullptr, dpk, dwpk, st)
-                      : launch_tc_wgrad<3, false>(gq, xcl, nullptr, dpk, dwpk, st);
-        if (r != 0) return r;
-        r = dwpk_fold<false>(gq, dwpk, dw_off, st);
-        if (r != 0) return r;
-    }
-    return 0;
+    return launch_tc_forward(g, pl, ndim, 1, xcl, offsets, base + l.wpk_off, bias, y, st);
 }
 
 int tc_layer_backward(const Geom& g, const Geom& gq, int ndim, const float* x, const float* offsets, const float* w_off,
-                      const float* w, const float* dy, const void* xcl_in, float* dx, float* dw_off, float* dw,
-                      float** doff_out, void* ws, size_t ws_bytes, cudaStream_t st) {
+                      const float* w, const float* dy, const void* xcl_in, float* dx, float* dw_off, float* db_off, float* dw,
+                      float* dbias, float** doff_out, bool* bias_done, bool* bias_off_done, void* ws, size_t ws_bytes,
+                      cudaStream_t st) {
     if (ws_bytes < tc_layer_workspace_bytes(g, gq, ndim, 3)) return -4;
     uint8_t* base = static_cast<uint8_t*>(ws);
     float* doff = reinterpret_cast<float*>(base);
     uint8_t* ws_main = base + layer_doff_bytes(g, ndim);
-    const size_t main_bytes = align_up(bwd_data_workspace(g).total, 256);
-    uint8_t* ws_q = ws_main + main_bytes;
-    const __nv_bfloat16* xcl = static_cast<const __nv_bfloat16*>(xcl_in);
-    if (xcl == nullptr) {
-        __nv_bfloat16* mine = reinterpret_cast<__nv_bfloat16*>(ws_main + bwd_data_workspace(g).xcl_off);
-        const int r0 = launch_channels_last(g, x, mine, st);
-        if (r0 != 0) return r0;
-        xcl = mine;
+    uint8_t* ws_q = ws_main + align_up(bwd_data_workspace(g).total, 256);
+    const bool chain = dx != nullptr || dw_off != nullptr || db_off != nullptr;      // dOffset is needed downstream
+    Backward b(g, ndim, 1, false, offsets, w, dy, dx, chain ? doff : nullptr, dw, dbias, ws_main);
+    // gradients of the offset-producing convolution given dOffset: its dX is added to the one of the deformable part
+    Backward q(gq, ndim, 0, false, nullptr, w_off, doff, dx, nullptr, dw_off, db_off, ws_q);
+    q.dx_cl = g.cl != 0;
+    q.dx_partial = true;
+    *bias_done = b.bias_here;
+    *bias_off_done = q.bias_here;
+    *doff_out = doff;
+    const bool second = dx != nullptr || dw_off != nullptr;
+    Passes p;
+    b.xcl = static_cast<const __nv_bfloat16*>(xcl_in);
+    if (b.xcl == nullptr) {
+        p.copy_x(g, x, b.own_xcl());
+        b.xcl = b.own_xcl();
     }
-    const bool chain = dx != nullptr || dw_off != nullptr || doff_out != nullptr;     // dOffset is needed downstream
-    int r = tc_backward(g, ndim, 1, x, offsets, w, dy, xcl, dx, chain ? doff : nullptr, dw, ws_main, main_bytes, st);
+    q.xcl = b.xcl;
+    int r = b.before(p, st);
     if (r != 0) return r;
-    if (doff_out != nullptr) *doff_out = doff;
-    if (dx == nullptr && dw_off == nullptr) return 0;
-    return plain_backward_into(gq, ndim, g.cl != 0, xcl, w_off, doff, dx, dw_off, ws_q, st);
+    b.with_dy(p);
+    if (second) r = q.before(p, st);
+    if (r == 0) r = p.launch(st);
+    if (r == 0) r = b.run(st);
+    if (r != 0) return r;
+    Passes mid, end;
+    b.fold_dx(mid);                      // before anything is added to dX
+    if (second) {
+        q.with_dy(mid);
+        r = mid.launch(st);
+        if (r == 0) r = q.run(st);
+        if (r != 0) return r;
+        q.fold_dx(end);
+        q.epilogue(end);
+    } else {
+        r = mid.launch(st);
+        if (r != 0) return r;
+    }
+    b.epilogue(end);
+    return end.launch(st);
 }
 
 // ---------------------------------------------------------------------------------------------------

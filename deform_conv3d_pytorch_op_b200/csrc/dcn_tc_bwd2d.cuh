@@ -26,7 +26,7 @@
 //
 // GEMM (per position tile of 128, 32 output channels per pipeline stage):
 //   col[P, (tap, c)] = sum over o of dy[o, P] * W[o, c, tap]        N = kv * 8 columns (padded to 16)
-//   A operand: dy, pack_dy tiles read MN-major (two 64-position halves)      B operand: the slab's W^T, K-major,
+//   A operand: dy, packed tiles read MN-major (two 64-position halves)      B operand: the slab's W^T, K-major,
 //   resident in shared memory for the whole (sample, slab)
 // Offset gradient (the reference's deformable_col2im_offset, deform2d/lib/deform_conv2d_cuda_kernel.cu:250-347):
 // the same thread reads the 4 corner rows of the slab's input plane (bf16, also in shared memory), forms the
@@ -90,75 +90,6 @@ inline bool b2_supported(const Geom& g, int ndim, int deform) {
 size_t b2_wpk_bytes(const Geom& g) {
     const B2Dims d = b2_dims(g);
     return (size_t)g.G * d.SL * d.w_bytes + 2048;     // + the rows an MMA reads past the last tile
-}
-
-// Wt [O][kv * Cg] bf16 (k' order) -> per (group, slab, 64-channel chunk of o) one K-major bf16 tile
-// [kv * 8 rows][64 o], row = tap * 8 + (channel within the slab), swizzled; o >= Og is zero.  The 8 channels of a
-// (slab, tap) are 16 contiguous bytes of Wt.
-__global__ void __launch_bounds__(256)
-pack_weight_slab(const Geom g, const __nv_bfloat16* __restrict__ wt, uint8_t* __restrict__ wpk, int SL, int OC) {
-    __shared__ __align__(16) uint16_t piece[64][16 * 8 + 8];        // [o][tap * 8 + c], up to 16 taps
-    const int tile = blockIdx.x;                          // (j * SL + slab) * OC + oc
-    const int oc = tile % OC, slab = (tile / OC) % SL, j = tile / OC / SL;
-    uint8_t* dst = wpk + (size_t)tile * g.kv * 1024;
-    const uint16_t* src = reinterpret_cast<const uint16_t*>(wt);
-    for (int e = threadIdx.x; e < 64 * g.kv; e += blockDim.x) {
-        const int ol = e / g.kv, tap = e - ol * g.kv;
-        const int o = oc * 64 + ol;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (o < g.Og) v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(j * g.Og + o) * g.Kg + (size_t)tap * g.Cg + slab * 8));
-        *reinterpret_cast<uint4*>(&piece[ol][tap * 8]) = v;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < g.kv * 64; e += blockDim.x) {
-        const int row = e % (g.kv * 8), chunk = e / (g.kv * 8);
-        uint32_t pk[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            pk[q] = (uint32_t)piece[chunk * 8 + 2 * q][row] | ((uint32_t)piece[chunk * 8 + 2 * q + 1][row] << 16);
-        *reinterpret_cast<uint4*>(dst + swz_offset(row, chunk)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-    }
-}
-
-// Sampling points, located once for all channel slabs of a deformable group.  One 16-byte entry per (sample,
-// deformable group, tap, output position), positions contiguous:
-//   x  bits 0-19 byte offset of the (lo_h, lo_w) pixel in the blocked dX plane | bits 27-28 its class
-//      | bit 29 hi_w != lo_w | bit 30 hi_h != lo_h | bit 31 valid
-//   y  lo_h * Wp + lo_w (pixel index in the linear x plane)      z, w  the fractions lw_h, lw_w (fp32 bits)
-// An invalid point has bits 29-31 and the fractions zero and names some pixel inside the plane (the tap's
-// undeformed position, clamped): the kernel adds zeros there, and spreading those zeros over the plane keeps
-// them from colliding on one address.
-// The point is located exactly as everywhere else in the library (locate: int32 base + offset in one fp32
-// rounding, validity, truncation, edge rule); dcn_debug_tc_points decodes these entries for the bit-exactness test.
-__global__ void __launch_bounds__(256)
-b2_points_kernel(const Geom g, const float* __restrict__ off, uint4* __restrict__ pts, int Wp, int W2) {
-    const long long total = (long long)g.N * g.dg * g.kv * g.ov;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-        uint32_t q1, pos, q2, tap, n, grp;
-        g.d_ov.divmod((uint32_t)e, q1, pos);
-        g.d_kv.divmod(q1, q2, tap);
-        n = q2 / (uint32_t)g.dg;
-        grp = q2 - n * (uint32_t)g.dg;
-        const OutPos op = decompose_pos(g, (long long)n * g.ov + pos);
-        Pt<float, 2> s;
-        locate<float, 2>(g, offset_block<float, 2>(g, off, (int)n), (int)grp, (int)tap, op, s);
-        uint4 r = make_uint4(0u, 0u, 0u, 0u);
-        int h0, w0;
-        if (s.valid) {
-            h0 = s.lo[0];
-            w0 = s.lo[1];
-            r.x = ((s.hi[1] != w0 ? 1u : 0u) << 29) | ((s.hi[0] != h0 ? 1u : 0u) << 30) | (1u << 31);
-            r.z = __float_as_uint(s.lw[0]);
-            r.w = __float_as_uint(s.lw[1]);
-        } else {
-            h0 = op.base[1] < 0 ? 0 : (op.base[1] >= g.in[1] ? g.in[1] - 1 : op.base[1]);
-            w0 = op.base[2] < 0 ? 0 : (op.base[2] >= g.in[2] ? g.in[2] - 1 : op.base[2]);
-        }
-        const uint32_t cls = (uint32_t)((h0 & 1) * 2 + (w0 & 1));
-        r.x |= (uint32_t)(((h0 >> 1) * W2 + (w0 >> 1)) * 128) + cls * 32u + (cls << 27);
-        r.y = (uint32_t)(h0 * Wp + w0);
-        pts[e] = r;
-    }
 }
 
 size_t b2_points_bytes(const Geom& g) { return (size_t)g.N * g.dg * g.kv * g.ov * 16; }

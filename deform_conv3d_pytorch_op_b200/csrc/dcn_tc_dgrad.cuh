@@ -1,6 +1,6 @@
 // Input and offset gradients on tcgen05, row-wise epilogue variant (included by dcn_tc.cu inside its anonymous
 // namespace): every epilogue thread keeps its output position for the scatter as well.  Fallback of
-// dcn_tc_dgrad2.cuh for channel-group sizes that variant does not take; also defines the packers, the
+// dcn_tc_dgrad2.cuh for channel-group sizes that variant does not take; also defines the
 // work decomposition and the GEMM description shared by both.
 //
 //   col[P, k'] = sum over o of dy[o, P] * W[o, k']                    k' = tap * Cg + c
@@ -12,7 +12,7 @@
 //                    registers (the channel axis lies along the thread's own columns), combined with the
 //                    interpolation-weight derivatives and added to dOffset once per (group, tap, position).
 // The reference's column buffer (col) never reaches memory.
-//   A operand: dy, bf16, pack_dy tiles read as MN-major [64 o rows][64 P per 128-byte row], two P halves
+//   A operand: dy, bf16, packed tiles read as MN-major [64 o rows][64 P per 128-byte row], two P halves
 //   B operand: W^T, bf16, pre-packed [k' rows][64 o per 128-byte row]              -> K-major
 #pragma once
 
@@ -26,59 +26,6 @@ struct DgSmem {
     static constexpr int kBarOffset = kDgStages * kStageBytes;
     static constexpr int kTotal = kBarOffset + (2 * kDgStages + 4) * 8 + 16;
 };
-
-// Wt [O][kv * Cg] bf16 (k' order) -> bf16 tiles [G][NB][OC][256 k' rows x 64 o], swizzled K-major: the transpose of a
-// 64 x 256 piece of Wt through shared memory, 512-byte row reads and 128-byte tile-row writes.
-__global__ void __launch_bounds__(256)
-pack_weight_bwd(const Geom g, const __nv_bfloat16* __restrict__ wt, uint8_t* __restrict__ wpk, int NB, int OC) {
-    __shared__ __align__(16) uint16_t piece[64][256 + 8];   // [o][k'], rows padded against bank conflicts
-    const int tile = blockIdx.x;                          // (j * NB + nb) * OC + oc
-    const int oc = tile % OC, nb = (tile / OC) % NB, j = tile / OC / NB;
-    uint8_t* dst = wpk + (size_t)tile * (2 * kTileBytes);
-    const uint16_t* src = reinterpret_cast<const uint16_t*>(wt);
-    for (int e = threadIdx.x; e < 64 * 32; e += blockDim.x) {
-        const int ol = e / 32, part = e % 32;
-        const int o = oc * 64 + ol, kq = nb * 256 + part * 8;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (o < g.Og && kq < g.Kg) v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(j * g.Og + o) * g.Kg + kq));
-        *reinterpret_cast<uint4*>(&piece[ol][part * 8]) = v;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < 256 * 8; e += blockDim.x) {
-        const int row = e % 256, chunk = e / 256;         // consecutive threads read consecutive k' of one o
-        uint32_t pk[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            pk[q] = (uint32_t)piece[chunk * 8 + 2 * q][row] | ((uint32_t)piece[chunk * 8 + 2 * q + 1][row] << 16);
-        *reinterpret_cast<uint4*>(dst + swz_offset(row, chunk)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-    }
-}
-
-// dx[n, c, p] (+)= dx_cl[n, p, c]
-template <bool ACCUMULATE>
-__global__ void __launch_bounds__(256)
-from_channels_last(const float* __restrict__ dxcl, float* __restrict__ dx, int C, int iv) {
-    __shared__ float tile[32][33];
-    const int n = blockIdx.z;
-    const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-    const float* in = dxcl + (size_t)n * iv * C;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int p = p0 + ty + i * 8, c = c0 + tx;
-        tile[ty + i * 8][tx] = (p < iv && c < C) ? in[(size_t)p * C + c] : 0.f;
-    }
-    __syncthreads();
-    float* out = dx + (size_t)n * C * iv;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int c = c0 + ty + i * 8, p = p0 + tx;
-        if (c < C && p < iv) {
-            if (ACCUMULATE) out[(size_t)c * iv + p] += tile[tx][ty + i * 8];
-            else out[(size_t)c * iv + p] = tile[tx][ty + i * 8];
-        }
-    }
-}
 
 template <int D, bool DEFORM>
 __global__ void __launch_bounds__(kDgThreads, 1)

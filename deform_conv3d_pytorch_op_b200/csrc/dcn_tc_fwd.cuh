@@ -490,8 +490,17 @@ tc_forward_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const flo
 
 // Largest number of distinct (deformable group, tap) keys any 64-wide K chunk touches.
 inline int max_slots_per_chunk(const Geom& g, int cols_per_chunk) {
-    const int kq = g.kv * g.Cg;
+    const int kq = g.kv * g.Cg, width = cols_per_chunk * 8;
     int best = 1;
+    if (g.Cg % g.cpg == 0 || g.cpg % g.Cg == 0) {          // keys change at every multiple of the segment length
+        const int seg = g.cpg < g.Cg ? g.cpg : g.Cg;
+        for (int k0 = 0; k0 < kq; k0 += width) {
+            const int k1 = k0 + width < kq ? k0 + width : kq;
+            const int slots = (k1 - 1) / seg - k0 / seg + 1 + (k0 + width > kq ? 1 : 0);
+            if (slots > best) best = slots;
+        }
+        return best;
+    }
     for (int j = 0; j < g.G; ++j) {
         for (int k0 = 0; k0 < kq; k0 += cols_per_chunk * 8) {
             int slots = 0, prev = -2;
@@ -511,14 +520,24 @@ inline int max_slots_per_chunk(const Geom& g, int cols_per_chunk) {
     return best;
 }
 
-// accumulate: add to what y holds (no zero fill; every tile leaves through reductions)
+// How a forward pass runs: stages, work split and what of y has to be zero before the kernel starts (parts of a split
+// tile are added to it).
+struct FwdPlan {
+    FwdSplit sp;
+    int stages, n_tabs, smem, max_slots, grid;
+    bool direct;                         // the corner table does not fit beside the stages
+    struct { float* p; size_t len; int rows, pitch; } zero[2];
+    int zeros;
+};
+
+// accumulate: add to what y holds (every tile leaves through reductions; the direct variant cannot)
 template <int D, bool DEFORM>
-int launch_tc_forward(const Geom& g, const __nv_bfloat16* xcl, const float* off, const uint8_t* wpk,
-                      const float* bias, float* y, cudaStream_t st, bool accumulate = false) {
+FwdPlan fwd_plan(const Geom& g, float* y, bool accumulate) {
     const TcDims d = tc_dims(g);
-    const int max_slots = max_slots_per_chunk(g, 8);
-    const size_t tab_one = (size_t)max_slots * 128 * sizeof(TabEntry<D, DEFORM>);
-    const size_t ost_bytes = (size_t)kFwdOffRing * max_slots * D * 128 * sizeof(float);
+    FwdPlan pl = {};
+    pl.max_slots = max_slots_per_chunk(g, 8);
+    const size_t tab_one = (size_t)pl.max_slots * 128 * sizeof(TabEntry<D, DEFORM>);
+    const size_t ost_bytes = (size_t)kFwdOffRing * pl.max_slots * D * 128 * sizeof(float);
     auto need = [&](int stages, int tabs) {
         return (long long)stages * kFwdStageBytes + (long long)tabs * tab_one + ost_bytes + sizeof(FwdCtl) + 1024;
     };
@@ -526,23 +545,19 @@ int launch_tc_forward(const Geom& g, const __nv_bfloat16* xcl, const float* off,
     // parity, which is only sound while no warp runs two laps of the ring ahead of another: with the tables
     // consumed in order that holds for rings of four and more.  A ring of five or six comes before the fourth
     // operand stage (the stage count hardly matters: the producers, not the MMA, bound a stage).
-    int stages = 0, n_tabs = 0;
     const int pref[][2] = {{4, 6}, {4, 5}, {3, 6}, {3, 5}, {4, 4}, {3, 4}, {2, 6}, {2, 5}, {2, 4}};
     for (const auto& c : pref) {
-        if (need(c[0], c[1]) <= kSmemLimit) { stages = c[0]; n_tabs = c[1]; break; }
+        if (need(c[0], c[1]) <= kSmemLimit) { pl.stages = c[0]; pl.n_tabs = c[1]; break; }
     }
-    if (stages == 0) {
-        if (accumulate) return -5;                  // (the direct variant overwrites)
-        return launch_tc_forward_direct<D, DEFORM>(g, xcl, off, wpk, bias, y, st);   // table too large
+    if (pl.stages == 0) {
+        pl.direct = true;
+        return pl;
     }
-    const int smem = (int)need(stages, n_tabs);
-    constexpr int GW = 16;
-    auto kern = tc_forward_kernel<D, DEFORM, GW>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -5;
+    pl.smem = (int)need(pl.stages, pl.n_tabs);
     // split the K range when there are fewer tiles than SMs (small batches / late layers of a network)
     const long long base_tiles = (long long)g.G * d.MB * d.PT;
     const int S = sm_count();
-    FwdSplit sp;
+    FwdSplit& sp = pl.sp;
     sp.acc = accumulate ? 1 : 0;
     sp.KS0 = 1;
     if (base_tiles * 2 <= S) {
@@ -557,8 +572,12 @@ int launch_tc_forward(const Geom& g, const __nv_bfloat16* xcl, const float* off,
     sp.KS1 = 1;
     sp.cpk1 = d.KC;
     sp.n_items = sp.T0;
+    auto zero = [&](float* p, size_t len, int rows, int pitch) {
+        auto& z = pl.zero[pl.zeros++];
+        z.p = p; z.len = len; z.rows = rows; z.pitch = pitch;
+    };
     if (sp.KS0 > 1) {
-        if (!accumulate && cudaMemsetAsync(y, 0, (size_t)g.N * g.O * g.ov * sizeof(float), st) != cudaSuccess) return -5;
+        if (!accumulate) zero(y, (size_t)g.N * g.O * g.ov, 1, 0);
     } else if (!accumulate && g.G * d.MB == 1 && base_tiles > S && base_tiles % S != 0) {
         // Tail of an uneven grid: the R tiles left after the last full wave are split along K into as many pieces
         // as there are SMs to take them.  With one (group, channel block) the tile index is the position tile, so
@@ -574,25 +593,46 @@ int launch_tc_forward(const Geom& g, const __nv_bfloat16* xcl, const float* off,
             sp.n_items = sp.T0 + R * sp.KS1;
             const long long P0 = sp.T0 * kTileN;
             if (g.cl) {
-                if (cudaMemsetAsync(y + (size_t)P0 * g.O, 0, (size_t)(g.P - P0) * g.O * sizeof(float), st) != cudaSuccess)
-                    return -5;
+                zero(y + (size_t)P0 * g.O, (size_t)(g.P - P0) * g.O, 1, 0);
             } else {
                 long long n0 = P0 / g.ov;
                 const long long o0 = P0 % g.ov;
                 if (o0 != 0) {      // the sample the tail starts in: the positions [o0, ov) of every channel
-                    if (cudaMemset2DAsync(y + (size_t)n0 * g.O * g.ov + o0, (size_t)g.ov * sizeof(float), 0,
-                                          (size_t)(g.ov - o0) * sizeof(float), (size_t)g.O, st) != cudaSuccess)
-                        return -5;
+                    zero(y + (size_t)n0 * g.O * g.ov + o0, (size_t)(g.ov - o0), g.O, g.ov);
                     ++n0;
                 }
-                if (n0 < g.N &&
-                    cudaMemsetAsync(y + (size_t)n0 * g.O * g.ov, 0, (size_t)(g.N - n0) * g.O * g.ov * sizeof(float), st) !=
-                        cudaSuccess)
-                    return -5;
+                if (n0 < g.N) zero(y + (size_t)n0 * g.O * g.ov, (size_t)(g.N - n0) * g.O * g.ov, 1, 0);
             }
         }
     }
-    const int grid = (int)(sp.n_items < S ? sp.n_items : S);
-    kern<<<grid, fwd_threads(GW), smem, st>>>(g, xcl, off, wpk, bias, y, d.KC, d.MT, d.MB, d.PT, stages, max_slots, n_tabs, sp);
+    pl.grid = (int)(sp.n_items < S ? sp.n_items : S);
+    return pl;
+}
+
+template <int D, bool DEFORM>
+int launch_tc_forward(const Geom& g, const FwdPlan& pl, const __nv_bfloat16* xcl, const float* off, const uint8_t* wpk,
+                      const float* bias, float* y, cudaStream_t st) {
+    if (pl.direct) return launch_tc_forward_direct<D, DEFORM>(g, xcl, off, wpk, bias, y, st);
+    const TcDims d = tc_dims(g);
+    constexpr int GW = 16;
+    auto kern = tc_forward_kernel<D, DEFORM, GW>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem) != cudaSuccess) return -5;
+    kern<<<pl.grid, fwd_threads(GW), pl.smem, st>>>(g, xcl, off, wpk, bias, y, d.KC, d.MT, d.MB, d.PT, pl.stages, pl.max_slots,
+                                                    pl.n_tabs, pl.sp);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+inline FwdPlan fwd_plan(const Geom& g, int ndim, int deform, float* y, bool accumulate) {
+    if (ndim == 2) return deform ? fwd_plan<2, true>(g, y, accumulate) : fwd_plan<2, false>(g, y, accumulate);
+    return deform ? fwd_plan<3, true>(g, y, accumulate) : fwd_plan<3, false>(g, y, accumulate);
+}
+inline void add_zeros(Passes& p, const FwdPlan& pl) {
+    for (int i = 0; i < pl.zeros; ++i) p.zero(pl.zero[i].p, pl.zero[i].len, pl.zero[i].rows, pl.zero[i].pitch);
+}
+inline int launch_tc_forward(const Geom& g, const FwdPlan& pl, int ndim, int deform, const __nv_bfloat16* xcl,
+                             const float* off, const uint8_t* wpk, const float* bias, float* y, cudaStream_t st) {
+    if (ndim == 2) return deform ? launch_tc_forward<2, true>(g, pl, xcl, off, wpk, bias, y, st)
+                                 : launch_tc_forward<2, false>(g, pl, xcl, off, wpk, bias, y, st);
+    return deform ? launch_tc_forward<3, true>(g, pl, xcl, off, wpk, bias, y, st)
+                  : launch_tc_forward<3, false>(g, pl, xcl, off, wpk, bias, y, st);
 }

@@ -1,14 +1,14 @@
 // Weight gradient on tcgen05, direct-sampling variant (included by dcn_tc.cu inside its anonymous namespace):
 // each producer thread locates its own sampling points.  Fallback of dcn_tc_wgrad2.cuh for problems whose
-// coordinate table does not fit in shared memory; also defines pack_dy and the work decomposition.
+// coordinate table does not fit in shared memory; also defines the work decomposition.
 //
 //   dW[o, k'] += sum over positions P of dy[o, P] * sample(k', P)          k' = tap * Cg + c
 //
 // GEMM view: M = output channels (128-row tiles, up to two per CTA), N = a block of up to 256 k' columns,
 // K = output positions, 64 per pipeline stage.  One CTA owns one (group, o-block, k'-block) and a slice of
 // the position range; partial sums are added with 16-byte fp32 reductions to the packed scratch dwpk[o][k']
-// (tiny and L2-resident), which unpack_dw folds into dW afterwards.
-//   A operand: dy, bf16, pre-packed by pack_dy into swizzled [128 o][64 P] tiles  -> K-major, bulk-copied
+// (tiny and L2-resident), which a fold job adds into dW afterwards.
+//   A operand: dy, bf16, pre-packed into swizzled [128 o][64 P] tiles  -> K-major, bulk-copied
 //   B operand: sampled patch, [64 P rows][64 k' per 128-byte row] sub-tiles        -> MN-major, produced here
 #pragma once
 
@@ -24,82 +24,6 @@ struct WgSmem {
     static constexpr int kBarOffset = kWgStages * kStageBytes;
     static constexpr int kTotal = kBarOffset + (2 * kWgStages + 1) * 8 + 16;
 };
-
-// dy [N, O, ov] fp32 -> bf16 tiles [G][MT][PC][128 o rows x 64 positions], swizzled; rows >= Og and
-// positions >= P are zero.  Used by both backward kernels.
-// If absmax_bits is not null it is raised to the bit pattern of max|dy| (non-negative floats order like their bits).
-__global__ void __launch_bounds__(256)
-pack_dy(const Geom g, const float* __restrict__ dy, uint8_t* __restrict__ dpk, int MT, long long PC,
-        unsigned int* __restrict__ absmax_bits) {
-    const long long pc = blockIdx.x;
-    const int mt = blockIdx.y % MT, j = blockIdx.y / MT;
-    uint8_t* dst = dpk + (((size_t)j * MT + mt) * PC + pc) * kTileBytes;
-    const int lane = threadIdx.x % 32, wrp = threadIdx.x / 32;
-    // lane handles positions 2*lane, 2*lane+1 of the 64; each warp walks rows wrp, wrp+8, ...
-    const long long P0 = pc * 64 + 2 * lane;
-    uint32_t n0 = 0, op0 = 0, n1 = 0, op1 = 0;
-    const bool ok0 = P0 < g.P, ok1 = P0 + 1 < g.P;
-    if (ok0) g.d_ov.divmod((uint32_t)P0, n0, op0);
-    if (ok1) g.d_ov.divmod((uint32_t)(P0 + 1), n1, op1);
-    float mx = 0.f;
-    // both positions in one sample and 8-byte aligned (even ov, aligned dy): one 8-byte load per row
-    const bool pair = ok1 && n0 == n1 && (g.ov & 1) == 0 && (reinterpret_cast<uintptr_t>(dy) & 7) == 0;
-    for (int row = wrp; row < 128; row += 8) {      // (forcing this loop to unroll 8-fold measured 20 % slower)
-        const int ol = mt * 128 + row;
-        float a = 0.f, b = 0.f;
-        if (ol < g.Og) {
-            const int o = j * g.Og + ol;
-            if (pair) {
-                const float2 t = __ldg(reinterpret_cast<const float2*>(dy + ((size_t)n0 * g.O + o) * g.ov + op0));
-                a = t.x; b = t.y;
-            } else {
-                if (ok0) a = __ldg(dy + ((size_t)n0 * g.O + o) * g.ov + op0);
-                if (ok1) b = __ldg(dy + ((size_t)n1 * g.O + o) * g.ov + op1);
-            }
-        }
-        mx = fmaxf(mx, fmaxf(fabsf(a), fabsf(b)));
-        const uint32_t chunk = lane / 4;            // 8 positions per 16-byte chunk
-        *reinterpret_cast<uint32_t*>(dst + swz_offset(row, chunk) + (lane % 4) * 4) = pack_bf16x2(a, b);
-    }
-    if (absmax_bits != nullptr) {
-        __shared__ unsigned int blk_max;
-        if (threadIdx.x == 0) blk_max = 0u;
-        __syncthreads();
-        const unsigned int m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-        if (lane == 0 && m != 0) atomicMax(&blk_max, m);
-        __syncthreads();
-        if (threadIdx.x == 0 && blk_max != 0) atomicMax(absmax_bits, blk_max);
-    }
-}
-
-// Same tiles from a channels-last dy [N * ov positions][O]: a thread packs 8 consecutive positions of one
-// output channel (one 16-byte chunk); consecutive threads take consecutive channels, so the reads coalesce.
-__global__ void __launch_bounds__(256)
-pack_dy_cl(const Geom g, const float* __restrict__ dy, uint8_t* __restrict__ dpk, int MT, long long PC) {
-    const long long pc = blockIdx.x;
-    const int mt = blockIdx.y % MT, j = blockIdx.y / MT;
-    uint8_t* dst = dpk + (((size_t)j * MT + mt) * PC + pc) * kTileBytes;
-    for (int item = threadIdx.x; item < 128 * 8; item += 256) {
-        const int row = item % 128, chunk = item / 128;
-        const int ol = mt * 128 + row;
-        float v[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const long long P = pc * 64 + chunk * 8 + e;
-            v[e] = (ol < g.Og && P < g.P) ? __ldg(dy + (size_t)P * g.O + j * g.Og + ol) : 0.f;
-        }
-        *reinterpret_cast<uint4*>(dst + swz_offset(row, chunk)) =
-            make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
-    }
-}
-
-inline int launch_pack_dy(const Geom& g, const float* dy, uint8_t* dpk, int MT, long long PC, cudaStream_t st,
-                          unsigned int* absmax_bits = nullptr) {
-    const dim3 grid((unsigned)PC, (unsigned)(g.G * MT));
-    if (g.cl) pack_dy_cl<<<grid, 256, 0, st>>>(g, dy, dpk, MT, PC);
-    else pack_dy<<<grid, 256, 0, st>>>(g, dy, dpk, MT, PC, absmax_bits);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
-}
 
 template <int D, bool DEFORM>
 __global__ void __launch_bounds__(kWgThreads, 1)
@@ -223,7 +147,7 @@ tc_wgrad_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, cons
                 const int ol = (mb * 2 + mt) * 128 + q * 32 + lane;
                 const bool o_ok = ol < g.Og;
                 // partial sums of this position split: plain stores into its slice of the packed scratch
-                // dwpk[split][G][MB*256 rows][NB*256 columns] (added up in split order by unpack_dw)
+                // dwpk[split][G][MB*256 rows][NB*256 columns] (added up in split order by the dW fold)
                 float* dwo = dw + (size_t)blockIdx.y * wg_slice_elems(gridDim.x) +
                              ((size_t)j * MB * 256 + (o_ok ? ol : 0)) * ((size_t)NB * kWgNMax) + (size_t)nb * kWgNMax;
                 for (int cc = 0; cc < NW / 32; ++cc) {
@@ -276,49 +200,15 @@ inline WgDims wg_dims(const Geom& g) {
     return d;
 }
 
-// dwpk[split][G][rows][cols] (k' = tap * Cg + c along the columns) -> dW [O][Cg][kv] of the reference layout, the
-// position splits added in split order (deterministic); ACC adds to dW (the separate weight-gradient entry point
-// accumulates), else dW is overwritten.
-template <bool ACC>
-__global__ void __launch_bounds__(256)
-unpack_dw(const Geom g, const float* __restrict__ dwpk, float* __restrict__ dw, int rows, int cols, int splits,
-          size_t slice) {
-    const long long total = (long long)g.O * g.Cg * g.kv;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int tap = (int)(i % g.kv);
-        const long long oc = i / g.kv;
-        const int c = (int)(oc % g.Cg);
-        const int o = (int)(oc / g.Cg);
-        const int j = o / g.Og, ol = o - j * g.Og;
-        const float* src = dwpk + ((size_t)j * rows + ol) * cols + (size_t)tap * g.Cg + c;
-        // loads in batches of eight (independent, all in flight), additions in split order
-        float v = 0.f;
-        for (int s0 = 0; s0 < splits; s0 += 8) {
-            float t[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) t[u] = (s0 + u < splits) ? __ldg(src + (size_t)(s0 + u) * slice) : 0.f;
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (s0 + u < splits) v = (s0 + u == 0) ? t[u] : v + t[u];
-        }
-        if (ACC) dw[i] += v;
-        else dw[i] = v;
-    }
-}
-
 inline size_t dwpk_bytes(const Geom& g) {
     const WgDims d = wg_dims(g);
     return (size_t)d.splits * wg_slice_elems(g.G * d.MB * d.NB) * sizeof(float);
 }
 
-template <bool ACC>
-int dwpk_fold(const Geom& g, const float* dwpk, float* dw, cudaStream_t st) {
+// the fold of the position splits' sums into dW (add: accumulate)
+inline void add_dw_fold(Passes& p, const Geom& g, const float* dwpk, float* dw, bool add) {
     const WgDims d = wg_dims(g);
-    const long long total = (long long)g.O * g.Cg * g.kv;
-    const int blocks = (int)((total + 255) / 256 < 16 * sm_count() ? (total + 255) / 256 : 16 * sm_count());
-    unpack_dw<ACC><<<blocks, 256, 0, st>>>(g, dwpk, dw, d.MB * 256, d.NB * kWgNMax, d.splits,
-                                           wg_slice_elems(g.G * d.MB * d.NB));
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    p.fold_dw(g, dwpk, dw, d.MB * 256, d.NB * kWgNMax, d.splits, wg_slice_elems(g.G * d.MB * d.NB), add);
 }
 
 template <int D, bool DEFORM>

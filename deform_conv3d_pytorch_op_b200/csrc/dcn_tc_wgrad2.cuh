@@ -5,8 +5,8 @@
 // GEMM view: M = output channels (128-row tiles, up to two per CTA), N = a block of up to 256 k' columns,
 // K = output positions, 64 per pipeline stage.  One CTA owns one (group, o-block, k'-block) and a slice of
 // the position range; partial sums are added with 16-byte fp32 reductions to a packed, zero-filled scratch
-// dwpk[o][k'] (tiny and L2-resident) that unpack_dw folds into dW's [O][Cg][kv] layout afterwards.
-//   A operand: dy, bf16, pre-packed by pack_dy into swizzled [128 o][64 P] tiles  -> K-major, bulk-copied
+// dwpk[o][k'] (tiny and L2-resident) that the dW fold brings into dW's [O][Cg][kv] layout afterwards.
+//   A operand: dy, bf16, pre-packed into swizzled [128 o][64 P] tiles  -> K-major, bulk-copied
 //   B operand: sampled patch, [64 P rows][64 k' per 128-byte row] sub-tiles        -> MN-major, produced here
 // Warps: 0 MMA issue, 1 dy-tile loader, 2-5 coordinate warps (warp k fills the table of every 4th stage, as in
 // dcn_tc_fwd.cuh; after the last table the same warps are the epilogue), 6-21 gather warps (dcn_tc_sampler.cuh).
@@ -197,7 +197,7 @@ tc_wgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
                 const bool o_ok = ol < g.Og;
                 // The partial sums of this position split go to ITS slice of the packed scratch
                 // dwpk[split][G][MB*256 rows][NB*256 columns] with plain 16-byte stores: every element a slice's
-                // reader touches is written exactly once, and unpack_dw adds the slices in split order, so dW does
+                // reader touches is written exactly once, and the dW fold adds the slices in split order, so dW does
                 // not depend on the order in which the CTAs finish.
                 float* dwo = dw + (size_t)blockIdx.y * wg_slice_elems(gridDim.x) +
                              ((size_t)j * MB * 256 + (o_ok ? ol : 0)) * ((size_t)NB * kWgNMax) + (size_t)nb * kWgNMax;
