@@ -394,6 +394,8 @@ template <typename T, int D>
 __global__ void __launch_bounds__(kXThreads)
 exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
     __shared__ T tile[32][33];
+    pdl_trigger();
+    pdl_wait();
     unsigned b = blockIdx.x;
     if (b < a.nb) {                                                    // bias gradient: one output channel
         T s = (T)0;
@@ -655,6 +657,7 @@ exact_forward_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl
         }
         if (cf < ch1) fetch(kf, nf);
     };
+    pdl_wait();
     fetch(kf, 0);
     load_a(ch0);                                                      // (completes with the first item)
 #pragma unroll
@@ -812,6 +815,8 @@ exact_weight_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl,
 
     Acc<T, TM, TN> acc;
     acc.clear();
+    pdl_trigger();
+    pdl_wait();
     if (ch0 < ch1) {
         long long ci = ch0, cf = ch0;                                 // chunks of the next item to issue / entry to fetch
         auto step = [&](int it) {
@@ -944,6 +949,8 @@ exact_data_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl, c
     Acc<T, TM, TN> acc;
     acc.clear();
     const int nch = (g.Og + kBK - 1) / kBK;
+    pdl_trigger();
+    pdl_wait();
     load(0);
     store(0);
     for (int ch = 0; ch < nch; ++ch) {
@@ -1099,6 +1106,7 @@ template <typename T>
 __global__ void __launch_bounds__(kXThreads)
 exact_fold_kernel(const Geom g, const ExactGeom xg, const FoldArgs<T> a) {
     __shared__ T tile[32][33];
+    pdl_wait();
     unsigned b = blockIdx.x;
     if (b < a.nx) {
         const unsigned px = b % a.tx, r = b / a.tx, cy = r % a.ty, n = r / a.ty;
@@ -1279,8 +1287,7 @@ int launch_prep(const Geom& g, const ExactGeom& x, PrepArgs<T> a, cudaStream_t s
     if (a.zero != nullptr) a.nz = (unsigned)((a.zero_n * sizeof(T) + 64 * kXThreads - 1) / (64 * kXThreads));
     const unsigned blocks = a.nb + a.nx + a.np + a.nw + a.nz;
     if (blocks == 0) return 0;
-    exact_prep_kernel<T, D><<<blocks, kXThreads, 0, st>>>(g, x, a);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launch_dependent(exact_prep_kernel<T, D>, dim3(blocks), dim3(kXThreads), 0, st, g, x, a) == cudaSuccess ? 0 : -5;
 }
 
 template <typename K>
@@ -1294,8 +1301,7 @@ int launch_forward(const Geom& g, const ExactGeom& x, dim3 grid, const T* xcl, c
     auto kernel = exact_forward_kernel<T, D, DEFORM, V, TM, TN, TY>;
     const int smem = 2 * kBK * (TM * TY + 16 * TN) * (int)sizeof(T) + Sampler<T, D, DEFORM, V, 16 * TY>::kBytes;
     if (!allow_smem(kernel, smem)) return -5;
-    kernel<<<grid, 16 * TY, smem, st>>>(g, x, xcl, pts, w2, bias, y, per);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launch_dependent(kernel, grid, dim3(16 * TY), smem, st, g, x, xcl, pts, w2, bias, y, per) == cudaSuccess ? 0 : -5;
 }
 
 template <typename T, int D, bool DEFORM, int V, int TM, int TN, int TY>
@@ -1304,8 +1310,7 @@ int launch_weight(const Geom& g, const ExactGeom& x, dim3 grid, const T* xcl, co
     auto kernel = exact_weight_kernel<T, D, DEFORM, V, TM, TN, TY>;
     const int smem = 2 * kBK * (TM * TY + 16 / (int)sizeof(T) + 16 * TN) * (int)sizeof(T) + Sampler<T, D, DEFORM, V, 16 * TY>::kBytes;
     if (!allow_smem(kernel, smem)) return -5;
-    kernel<<<grid, 16 * TY, smem, st>>>(g, x, xcl, pts, dy, dwp, per);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launch_dependent(kernel, grid, dim3(16 * TY), smem, st, g, x, xcl, pts, dy, dwp, per) == cudaSuccess ? 0 : -5;
 }
 
 // FN<T, D, DEFORM, V, TM, TN, TY> with the tile that exact_tiles() chose
@@ -1381,9 +1386,9 @@ int run_backward(const Geom& g, const ExactGeom& x, int pass, int add, const voi
             return -5;
         constexpr int BN = 16 * kDataTn<T, V>;
         const dim3 grid((unsigned)((g.P + BN - 1) / BN), (unsigned)(g.G * (x.Kp64 / 64)));
-        exact_data_kernel<T, D, DEFORM, V><<<grid, kXThreads, 0, st>>>(g, x, a.xcl, a.pts, a.wk, (const T*)dy, a.zero,
-                                                                       DEFORM ? (T*)doff : nullptr, plain);
-        if (cudaGetLastError() != cudaSuccess) return -5;
+        if (launch_dependent(exact_data_kernel<T, D, DEFORM, V>, grid, dim3(kXThreads), 0, st, g, x, a.xcl, a.pts, a.wk,
+                             (const T*)dy, a.zero, DEFORM ? (T*)doff : nullptr, plain) != cudaSuccess)
+            return -5;
     }
     FoldArgs<T> f = {};
     f.add = add;
@@ -1406,8 +1411,7 @@ int run_backward(const Geom& g, const ExactGeom& x, int pass, int add, const voi
     }
     const unsigned blocks = f.nx + (dw != nullptr ? (unsigned)(((size_t)g.O * x.Kp64 + kXThreads - 1) / kXThreads) : 0u);
     if (blocks > 0) {
-        exact_fold_kernel<T><<<blocks, kXThreads, 0, st>>>(g, x, f);
-        if (cudaGetLastError() != cudaSuccess) return -5;
+        if (launch_dependent(exact_fold_kernel<T>, dim3(blocks), dim3(kXThreads), 0, st, g, x, f) != cudaSuccess) return -5;
     }
     return 0;
 }

@@ -4,10 +4,34 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
+#include <stdlib.h>
 
 #include "dcn_common.cuh"
 
 namespace dcn {
+
+// DCN_PDL=0: plain launches, in order.
+inline bool pdl_enabled() {
+    static const bool off = [] { const char* e = getenv("DCN_PDL"); return e != nullptr && e[0] == '0'; }();
+    return !off;
+}
+
+// Launch of a kernel that calls pdl_wait() before it reads or writes global memory (see dcn_common.cuh).
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
 
 // EXACT-precision (SIMT) launchers, dcn_simt.cu.  dtype: 0 fp32, 1 fp64.  Return 0 or -5 (launch failure).
 int simt_forward(const Geom& g, int dtype, int ndim, int deform, const void* x, const void* off, const void* w,

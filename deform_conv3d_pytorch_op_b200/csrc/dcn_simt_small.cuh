@@ -388,7 +388,7 @@ small_backward_kernel(const Geom g, const float* __restrict__ x, const float* __
     __syncthreads();
     // Everything above only reads inputs.  The outputs are zero-filled by the launch before this one, which this
     // kernel may overlap (programmatic dependent launch): wait for it here, before the first addition.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
 #pragma unroll 2
     for (int it = threadIdx.x; it < TP * g.Kg; it += kSmallThreads) {
         const int pl = it % TP, k = it / TP;
@@ -542,7 +542,7 @@ struct ZeroList {
 };
 __global__ void __launch_bounds__(256)
 small_zero_kernel(const Geom g, const float* __restrict__ dy, const ZeroList z) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_trigger();
     if (blockIdx.x >= z.blocks) {
         bias_grad_block(g, dy, z.dbias, (int)(blockIdx.x - z.blocks));
         return;
@@ -558,11 +558,6 @@ small_zero_kernel(const Geom g, const float* __restrict__ dy, const ZeroList z) 
         if (first < tail) z.p[b][h + 4 * n4 + first] = 0.f;
         for (size_t i = first; i < n4; i += stride) reinterpret_cast<float4*>(z.p[b] + h)[i] = zero;
     }
-}
-
-inline bool small_pdl_enabled() {
-    static const bool off = [] { const char* e = getenv("DCN_PDL"); return e != nullptr && e[0] == '0'; }();
-    return !off;
 }
 
 // dX, dW (dOffset with several convolution groups; the offset-producing convolution's gradients in layer mode) are
@@ -581,7 +576,7 @@ int launch_small_backward(const Geom& g, const float* x, const float* off, const
                       layer ? lay->db_off : nullptr};
     const size_t lens[5] = {(size_t)g.N * g.C * g.iv, (size_t)g.O * g.Cg * g.kv, (size_t)g.N * g.dg * g.kv * D * g.ov,
                             layer ? (size_t)gq->O * gq->Kg : 0, layer ? (size_t)gq->O : 0};
-    const bool pdl = small_pdl_enabled();
+    const bool pdl = pdl_enabled();
     ZeroList z;
     size_t most = 4;
     for (int b = 0; b < 5; ++b) {

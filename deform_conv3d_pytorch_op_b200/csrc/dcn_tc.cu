@@ -354,7 +354,7 @@ int tc_debug_points(const Geom& g, int ndim, int deform, const float* off, int n
     const B2Dims d = b2_dims(g);
     Passes p;
     p.points(g, off, pts, d.Wp, d.W2);
-    const int r = p.launch(st);
+    const int r = p.launch(st, true);
     if (r != 0) return r;
     const long long want = ((long long)g.dg * g.kv * g.ov + 255) / 256;
     const int blocks = (int)(want < 16ll * sm_count() ? want : 16ll * sm_count());
@@ -374,7 +374,7 @@ int tc_forward(const Geom& g, int ndim, int deform, const float* x, const float*
     p.copy_x(g, x, xcl);
     p.weight(g, kTilesFwd, w, wpk);
     add_zeros(p, plan);
-    const int r = p.launch(st);
+    const int r = p.launch(st, false);
     if (r != 0) return r;
     return launch_tc_forward(g, plan, ndim, deform, xcl, off, wpk, bias, y, st);
 }
@@ -391,11 +391,11 @@ int tc_backward_data(const Geom& g, int ndim, int deform, const float* x, const 
         p.copy_x(g, x, b.own_xcl());
         b.xcl = b.own_xcl();
     }
-    r = p.launch(st);
+    r = p.launch(st, false);
     if (r == 0) r = b.run(st);
     Passes q;
     b.fold_dx(q);
-    return r != 0 ? r : q.launch(st);
+    return r != 0 ? r : q.launch(st, true);
 }
 
 int tc_backward_weight(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* dy,
@@ -409,7 +409,7 @@ int tc_backward_weight(const Geom& g, int ndim, int deform, const float* x, cons
     Passes p;
     p.copy_x(g, x, xcl);
     p.pack_dy(g, dy, dpk, d.MT, d.PC, nullptr, nullptr);
-    int r = p.launch(st);
+    int r = p.launch(st, false);
     if (r != 0) return r;
     float* dwpk = reinterpret_cast<float*>(base + l.dwpk_off);
     if (ndim == 2) r = deform ? launch_tc_wgrad<2, true>(g, xcl, off, dpk, dwpk, st)
@@ -419,7 +419,7 @@ int tc_backward_weight(const Geom& g, int ndim, int deform, const float* x, cons
     if (r != 0) return r;
     Passes q;
     add_dw_fold(q, g, dwpk, dw, true);               // this entry point accumulates into dW
-    return q.launch(st);
+    return q.launch(st, true);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -445,13 +445,13 @@ int tc_backward(const Geom& g, int ndim, int deform, const float* x, const float
         b.xcl = b.own_xcl();
     }
     // (a call on its own keeps its passes apart, one name each on a profiler's timeline)
-    r = p.launch(st, xcl_in == nullptr);
+    r = p.launch(st, false, xcl_in == nullptr);
     if (r == 0) r = b.run(st);
     if (r != 0) return r;
     Passes q;
     b.fold_dx(q);
     b.epilogue(q);
-    return q.launch(st);
+    return q.launch(st, true);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -487,7 +487,7 @@ int tc_layer_forward(const Geom& g, const Geom& gq, int ndim, const float* x, co
     p.weight(g, kTilesFwd, w, base + l.wpk_off);
     add_zeros(p, pq);
     add_zeros(p, pl);
-    int r = p.launch(st);
+    int r = p.launch(st, false);
     if (r != 0) return r;
     r = launch_tc_forward(gq, pq, ndim, 0, xcl, nullptr, baseq + lq.wpk_off, b_off, offsets, st);
     if (r != 0) return r;
@@ -524,24 +524,24 @@ int tc_layer_backward(const Geom& g, const Geom& gq, int ndim, const float* x, c
     if (r != 0) return r;
     b.with_dy(p);
     if (second) r = q.before(p, st);
-    if (r == 0) r = p.launch(st);
+    if (r == 0) r = p.launch(st, false);
     if (r == 0) r = b.run(st);
     if (r != 0) return r;
     Passes mid, end;
     b.fold_dx(mid);                      // before anything is added to dX
     if (second) {
         q.with_dy(mid);
-        r = mid.launch(st);
+        r = mid.launch(st, false);
         if (r == 0) r = q.run(st);
         if (r != 0) return r;
         q.fold_dx(end);
         q.epilogue(end);
     } else {
-        r = mid.launch(st);
+        r = mid.launch(st, false);
         if (r != 0) return r;
     }
     b.epilogue(end);
-    return end.launch(st);
+    return end.launch(st, true);
 }
 
 // ---------------------------------------------------------------------------------------------------

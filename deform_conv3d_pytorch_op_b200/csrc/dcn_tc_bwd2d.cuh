@@ -209,6 +209,8 @@ tc_bwd2d_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const uint4
         mbar_init(&ctl->w_empty, 1);
         fence_barrier_init();
     }
+    pdl_trigger();
+    pdl_wait();
     if (warp == 0) {
         tmem_alloc(&ctl->tmem_base, 256);
         tmem_relinquish();
@@ -583,12 +585,11 @@ int launch_tc_bwd2d(const Geom& g, const __nv_bfloat16* xcl, const uint4* pts, c
     const bool full = dx != nullptr && doff != nullptr && g.kv % (kB2WQ * 3) == 0;
     auto go = [&](auto kern) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_bytes) != cudaSuccess) return false;
-        kern<<<grid, kB2Threads, d.smem_bytes, st>>>(g, xcl, pts, dpk, wpk, scale_bits, dx, doff, d, d_iw, d_w2);
-        return true;
+        return launch_dependent(kern, dim3(grid), dim3(kB2Threads), d.smem_bytes, st, g, xcl, pts, dpk, wpk, scale_bits, dx, doff,
+                                d, d_iw, d_w2) == cudaSuccess;
     };
     bool launched;
     if (accumulate) launched = full ? go(tc_bwd2d_kernel<true, true>) : go(tc_bwd2d_kernel<true, false>);
     else launched = full ? go(tc_bwd2d_kernel<false, true>) : go(tc_bwd2d_kernel<false, false>);
-    if (!launched) return -5;
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launched ? 0 : -5;
 }

@@ -54,6 +54,8 @@ tc_dgrad_rowwise_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, con
         }
         fence_barrier_init();
     }
+    pdl_trigger();
+    pdl_wait();
     if (warp == 0) {
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
@@ -271,6 +273,6 @@ int launch_tc_dgrad_rowwise(const Geom& g, const __nv_bfloat16* xcl, const float
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -5;
     const long long tiles = (long long)g.G * d.PT * d.NB;
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    kern<<<grid, kDgThreads, smem, st>>>(g, xcl, off, dpk, wpk, dxcl, doff, d.MT, d.NB, d.NW, d.OC, d.PC2, d.PT);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launch_dependent(kern, dim3(grid), dim3(kDgThreads), smem, st, g, xcl, off, dpk, wpk, dxcl, doff, d.MT, d.NB, d.NW,
+                            d.OC, d.PC2, d.PT) == cudaSuccess ? 0 : -5;
 }

@@ -74,6 +74,8 @@ tc_dgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
         }
         fence_barrier_init();
     }
+    pdl_trigger();
+    pdl_wait();
     if (warp == 0) {
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
@@ -414,8 +416,8 @@ int launch_tc_dgrad_t(const Geom& g, const __nv_bfloat16* xcl, const float* off,
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -5;
     const long long tiles = (long long)g.G * d.PT * d.NB;
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    kern<<<grid, 32 * (2 + EW), smem, st>>>(g, xcl, off, dpk, wpk, dxcl, doff, d.MT, d.NB, d.NW, d.OC, d.PC2, d.PT);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launch_dependent(kern, dim3(grid), dim3(32 * (2 + EW)), smem, st, g, xcl, off, dpk, wpk, dxcl, doff, d.MT, d.NB, d.NW,
+                            d.OC, d.PC2, d.PT) == cudaSuccess ? 0 : -5;
 }
 
 template <int D, bool DEFORM>

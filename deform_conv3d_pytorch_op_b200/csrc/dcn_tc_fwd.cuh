@@ -92,6 +92,7 @@ tc_forward_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const flo
         }
         fence_barrier_init();
     }
+    pdl_wait();
     if (warp == 0) {
         tmem_alloc(&ctl->tmem_base, 512);
         tmem_relinquish();
@@ -617,9 +618,8 @@ int launch_tc_forward(const Geom& g, const FwdPlan& pl, const __nv_bfloat16* xcl
     constexpr int GW = 16;
     auto kern = tc_forward_kernel<D, DEFORM, GW>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem) != cudaSuccess) return -5;
-    kern<<<pl.grid, fwd_threads(GW), pl.smem, st>>>(g, xcl, off, wpk, bias, y, d.KC, d.MT, d.MB, d.PT, pl.stages, pl.max_slots,
-                                                    pl.n_tabs, pl.sp);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launch_dependent(kern, dim3(pl.grid), dim3(fwd_threads(GW)), pl.smem, st, g, xcl, off, wpk, bias, y, d.KC, d.MT, d.MB,
+                            d.PT, pl.stages, pl.max_slots, pl.n_tabs, pl.sp) == cudaSuccess ? 0 : -5;
 }
 
 inline FwdPlan fwd_plan(const Geom& g, int ndim, int deform, float* y, bool accumulate) {

@@ -51,6 +51,7 @@ tc_forward_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, co
         }
         fence_barrier_init();
     }
+    pdl_wait();
     if (warp == 0) {
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
@@ -236,7 +237,7 @@ int launch_tc_forward_direct(const Geom& g, const __nv_bfloat16* xcl, const floa
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -5;
     const long long tiles = (long long)g.G * d.MB * d.PT;
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    kern<<<grid, kFwdDirectThreads, smem, st>>>(g, xcl, off, wpk, bias, y, d.KC, d.MT, d.MB, d.PT);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launch_dependent(kern, dim3(grid), dim3(kFwdDirectThreads), smem, st, g, xcl, off, wpk, bias, y, d.KC, d.MT, d.MB,
+                            d.PT) == cudaSuccess ? 0 : -5;
 }
 

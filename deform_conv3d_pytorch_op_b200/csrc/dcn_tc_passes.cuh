@@ -39,6 +39,7 @@ struct JobList {
     Geom g[kMaxGeoms];
     Job job[kMaxJobs];
     int n;
+    int last;                        // no kernel of the call follows
 };
 
 // x [N, C, iv] fp32 -> [N, iv, C] bf16: tiles of 64 channels x 64 positions, sixteen loads of a thread in flight, 128-byte
@@ -439,6 +440,8 @@ __device__ __forceinline__ void job_bias(const Geom& g, const Job& J, unsigned b
 __global__ void __launch_bounds__(kPassThreads, 6)
 tc_passes_kernel(const __grid_constant__ JobList L) {
     extern __shared__ float pass_smem[];
+    if (!L.last) pdl_trigger();
+    pdl_wait();
     unsigned b = blockIdx.x;
     int i = 0;
     while (b >= L.job[i].blocks) b -= L.job[i++].blocks;
@@ -562,9 +565,10 @@ public:
         J.blocks = (unsigned)((g.O + kPassThreads / 32 - 1) / (kPassThreads / 32));
     }
 
-    // one launch; apart: one launch per job
-    int launch(cudaStream_t st, bool apart = false) {
+    // one launch; last: of the call; apart: one launch per job
+    int launch(cudaStream_t st, bool last, bool apart = false) {
         if (error != 0) return error;
+        L.last = last ? 1 : 0;
         if (apart) {
             JobList one = L;
             for (int i = 0; i < L.n; ++i) {
@@ -605,7 +609,6 @@ private:
         if (smem > 48 * 1024 &&
             cudaFuncSetAttribute(tc_passes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return -5;
-        tc_passes_kernel<<<(unsigned)blocks, kPassThreads, smem, st>>>(l);
-        return cudaGetLastError() == cudaSuccess ? 0 : -5;
+        return launch_dependent(tc_passes_kernel, dim3((unsigned)blocks), dim3(kPassThreads), smem, st, l) == cudaSuccess ? 0 : -5;
     }
 };

@@ -57,6 +57,8 @@ tc_wgrad_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, cons
         mbar_init(acc_full, 1);
         fence_barrier_init();
     }
+    pdl_trigger();
+    pdl_wait();
     if (warp == 0) {
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
@@ -219,6 +221,6 @@ int launch_tc_wgrad_direct(const Geom& g, const __nv_bfloat16* xcl, const float*
     auto kern = tc_wgrad_direct_kernel<D, DEFORM>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -5;
     dim3 grid((unsigned)(g.G * d.MB * d.NB), (unsigned)d.splits);
-    kern<<<grid, kWgThreads, smem, st>>>(g, xcl, off, dpk, dw, d.MT, d.MB, d.NB, d.NW, d.PC, d.cps);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launch_dependent(kern, grid, dim3(kWgThreads), smem, st, g, xcl, off, dpk, dw, d.MT, d.MB, d.NB, d.NW, d.PC,
+                            d.cps) == cudaSuccess ? 0 : -5;
 }

@@ -66,6 +66,8 @@ tc_wgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
         }
         fence_barrier_init();
     }
+    pdl_trigger();
+    pdl_wait();
     if (warp == 0) {
         tmem_alloc(&ctl->tmem_base, 512);
         tmem_relinquish();
@@ -343,7 +345,6 @@ int launch_tc_wgrad(const Geom& g, const __nv_bfloat16* xcl, const float* off, c
     auto kern = tc_wgrad_kernel<D, DEFORM>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -5;
     dim3 grid((unsigned)(g.G * d.MB * d.NB), (unsigned)d.splits);
-    kern<<<grid, kWg2Threads, smem, st>>>(g, xcl, off, dpk, dw, d.MT, d.MB, d.NB, d.NW, d.PC, d.cps, stages, max_slots,
-                                          n_tabs, a_tiles);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return launch_dependent(kern, grid, dim3(kWg2Threads), smem, st, g, xcl, off, dpk, dw, d.MT, d.MB, d.NB, d.NW, d.PC, d.cps,
+                            stages, max_slots, n_tabs, a_tiles) == cudaSuccess ? 0 : -5;
 }
