@@ -379,6 +379,9 @@ struct Acc<float, R, C> {
 // Prologue of a pass, one launch: block ranges for the bias gradient, the input copy, the points, the weight and a zero fill.
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T>
+constexpr int kCopyTile = sizeof(T) == 4 ? 64 : 32;      // side of a transpose tile
+
+template <typename T>
 struct PrepArgs {
     const T *x, *off, *w, *dy;
     T *xcl, *wk, *zero, *dbias;      // wk: w2 (forward) or wt (backward)
@@ -393,7 +396,8 @@ struct PrepArgs {
 template <typename T, int D>
 __global__ void __launch_bounds__(kXThreads)
 exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
-    __shared__ T tile[32][33];
+    constexpr int TC = kCopyTile<T>;
+    __shared__ T tile[TC][TC + 1];
     pdl_trigger();
     pdl_wait();
     unsigned b = blockIdx.x;
@@ -415,28 +419,39 @@ exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
         return;
     }
     b -= a.nb;
-    if (b < a.nx) {                                                    // x -> xcl, 32 channels x 32 positions
+    if (b < a.nx) {                                                    // x -> xcl, TC channels x TC positions
         const unsigned px = b % a.tx, r = b / a.tx, cy = r % a.ty, n = r / a.ty;
         const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-        const int p0 = (int)px * 32, c0 = (int)cy * 32;
+        const int p0 = (int)px * TC, c0 = (int)cy * TC;
         const T* xn = a.x + (size_t)n * g.C * g.iv;
+        T v[TC / 8][TC / 32];                                          // all loads in flight together
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int c4 = c0 + ty + i * 8, p = p0 + tx;
-            T v = (T)0;
-            if (c4 < xg.C4 && p < g.iv) {
-                uint32_t seg, r4;
-                xg.d_S4.divmod((uint32_t)c4, seg, r4);
-                if ((int)r4 < xg.S) v = __ldg(xn + (size_t)(seg * xg.S + r4) * g.iv + p);
+        for (int i = 0; i < TC / 8; ++i) {
+            const int c4 = c0 + ty + i * 8;
+            uint32_t seg, r4;
+            xg.d_S4.divmod((uint32_t)c4, seg, r4);
+            const bool ok = c4 < xg.C4 && (int)r4 < xg.S;
+            const T* xc = xn + (size_t)(ok ? seg * xg.S + r4 : 0) * g.iv;
+#pragma unroll
+            for (int h = 0; h < TC / 32; ++h) {
+                const int p = p0 + h * 32 + tx;
+                v[i][h] = ok && p < g.iv ? __ldg(xc + p) : (T)0;
             }
-            tile[ty + i * 8][tx] = v;
         }
+#pragma unroll
+        for (int i = 0; i < TC / 8; ++i)
+#pragma unroll
+            for (int h = 0; h < TC / 32; ++h) tile[ty + i * 8][h * 32 + tx] = v[i][h];
         __syncthreads();
         T* on = a.xcl + (size_t)n * g.iv * xg.C4;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int p = p0 + ty + i * 8, c4 = c0 + tx;
-            if (p < g.iv && c4 < xg.C4) on[(size_t)p * xg.C4 + c4] = tile[tx][ty + i * 8];
+        for (int i = 0; i < TC / 8; ++i) {
+            const int p = p0 + ty + i * 8;
+#pragma unroll
+            for (int h = 0; h < TC / 32; ++h) {
+                const int c4 = c0 + h * 32 + tx;
+                if (p < g.iv && c4 < xg.C4) on[(size_t)p * xg.C4 + c4] = tile[h * 32 + tx][ty + i * 8];
+            }
         }
         return;
     }
@@ -1105,30 +1120,42 @@ struct FoldArgs {
 template <typename T>
 __global__ void __launch_bounds__(kXThreads)
 exact_fold_kernel(const Geom g, const ExactGeom xg, const FoldArgs<T> a) {
-    __shared__ T tile[32][33];
+    constexpr int TC = kCopyTile<T>;
+    __shared__ T tile[TC][TC + 1];
     pdl_wait();
     unsigned b = blockIdx.x;
     if (b < a.nx) {
         const unsigned px = b % a.tx, r = b / a.tx, cy = r % a.ty, n = r / a.ty;
         const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-        const int p0 = (int)px * 32, c0 = (int)cy * 32;
+        const int p0 = (int)px * TC, c0 = (int)cy * TC;
         const T* in = a.dxcl + (size_t)n * g.iv * xg.C4;
+        T v[TC / 8][TC / 32];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int p = p0 + ty + i * 8, c4 = c0 + tx;
-            tile[ty + i * 8][tx] = (p < g.iv && c4 < xg.C4) ? __ldg(in + (size_t)p * xg.C4 + c4) : (T)0;
+        for (int i = 0; i < TC / 8; ++i) {
+            const int p = p0 + ty + i * 8;
+#pragma unroll
+            for (int h = 0; h < TC / 32; ++h) {
+                const int c4 = c0 + h * 32 + tx;
+                v[i][h] = (p < g.iv && c4 < xg.C4) ? __ldg(in + (size_t)p * xg.C4 + c4) : (T)0;
+            }
         }
+#pragma unroll
+        for (int i = 0; i < TC / 8; ++i)
+#pragma unroll
+            for (int h = 0; h < TC / 32; ++h) tile[ty + i * 8][h * 32 + tx] = v[i][h];
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int c4 = c0 + ty + i * 8, p = p0 + tx;
-            if (c4 >= xg.C4 || p >= g.iv) continue;
+        for (int i = 0; i < TC / 8; ++i) {
+            const int c4 = c0 + ty + i * 8;
             uint32_t seg, r4;
             xg.d_S4.divmod((uint32_t)c4, seg, r4);
-            if ((int)r4 >= xg.S) continue;
-            T* dst = a.dx + ((size_t)n * g.C + seg * xg.S + r4) * g.iv + p;
-            const T v = tile[tx][ty + i * 8];
-            *dst = a.add ? *dst + v : v;
+            if (c4 >= xg.C4 || (int)r4 >= xg.S) continue;
+            T* dst = a.dx + ((size_t)n * g.C + seg * xg.S + r4) * g.iv;
+#pragma unroll
+            for (int h = 0; h < TC / 32; ++h) {
+                const int p = p0 + h * 32 + tx;
+                if (p < g.iv) dst[p] = a.add ? dst[p] + tile[h * 32 + tx][ty + i * 8] : tile[h * 32 + tx][ty + i * 8];
+            }
         }
         return;
     }
@@ -1273,8 +1300,8 @@ int launch_prep(const Geom& g, const ExactGeom& x, PrepArgs<T> a, cudaStream_t s
     a.nb = a.dbias != nullptr ? (unsigned)g.O : 0u;
     a.nx = a.np = a.nw = a.nz = 0;
     a.bpk = 1;
-    a.tx = (unsigned)((g.iv + 31) / 32);
-    a.ty = (unsigned)((x.C4 + 31) / 32);
+    a.tx = (unsigned)((g.iv + kCopyTile<T> - 1) / kCopyTile<T>);
+    a.ty = (unsigned)((x.C4 + kCopyTile<T> - 1) / kCopyTile<T>);
     if (a.xcl != nullptr) a.nx = a.tx * a.ty * (unsigned)g.N;
     if (a.pts != nullptr) {
         a.bpk = (unsigned)((g.P + kPtsPerThread * kXThreads - 1) / (kPtsPerThread * kXThreads));
@@ -1402,8 +1429,8 @@ int run_backward(const Geom& g, const ExactGeom& x, int pass, int add, const voi
         r = pick_weight<T, D, DEFORM, V>(t, g, x, grid, a.xcl, a.pts, (const T*)dy, (T*)(ws + l.dwp), per, st);
         if (r != 0) return r;
     }
-    f.tx = (unsigned)((g.iv + 31) / 32);
-    f.ty = (unsigned)((x.C4 + 31) / 32);
+    f.tx = (unsigned)((g.iv + kCopyTile<T> - 1) / kCopyTile<T>);
+    f.ty = (unsigned)((x.C4 + kCopyTile<T> - 1) / kCopyTile<T>);
     if (dx != nullptr) {
         f.dxcl = a.zero;
         f.dx = (T*)dx;

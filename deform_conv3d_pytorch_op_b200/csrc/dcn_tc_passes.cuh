@@ -385,42 +385,39 @@ __device__ __forceinline__ void job_dx(const Geom& g, const Job& J, unsigned blk
     }
 }
 
-// dwpk[split][G][rows][cols] (k' = tap * Cg + c along the columns) -> dW [O][Cg][kv], the position splits added in split
-// order (deterministic).  A block takes one output channel and 32 input channels: slices read along the channels
-// (128-byte runs), dW written along the taps.  (Runs of 8 taps per block, and four taps or sixteen splits per thread,
-// measured 15 to 50 % slower.)  a: rows, b: cols, c: add, d: splits, e: channel runs; z: slice elements
-constexpr int kFoldChannels = 32, kFoldTaps = 32;
+// dwpk[split][k' / 4][rows][4] (k' = tap * Cg + c) -> dW [O][Cg][kv], the position splits added in split order
+// (deterministic).  A block takes 8 output channels, 32 input channels and a run of up to 4 taps, one 16-byte vector of
+// channels per thread and split: slices read along the rows (128-byte runs), dW written along the taps.
+// a: rows of a group, c: add, d: splits, e: channel runs; z: slice elements, z2: tap runs
+constexpr int kFoldChannels = 32, kFoldRows = 8, kFoldTaps = 4;
 __device__ __forceinline__ void job_dw(const Geom& g, const Job& J, unsigned blk, float* sm) {
-    const int c0 = (int)(blk % J.e) * kFoldChannels, o = (int)(blk / J.e);
-    const int j = o / g.Og, ol = o - j * g.Og, kv = g.kv;
-    const int nc = g.Cg - c0 < kFoldChannels ? g.Cg - c0 : kFoldChannels;
-    const float* src = static_cast<const float*>(J.src) + ((size_t)j * J.a + ol) * J.b + c0;
-    float* dst = static_cast<float*>(J.dst) + ((size_t)o * g.Cg + c0) * kv;
-    for (int t0 = 0; t0 < kv; t0 += kFoldTaps) {
-        const int nt = kv - t0 < kFoldTaps ? kv - t0 : kFoldTaps;
-        if (t0 > 0) __syncthreads();
-        for (int e = threadIdx.x; e < nt * kFoldChannels; e += kPassThreads) {
-            const int c = e % kFoldChannels, t = e / kFoldChannels;
-            if (c >= nc) continue;
-            const float* s = src + (size_t)(t0 + t) * g.Cg + c;
-            // loads in batches of eight (independent, all in flight), additions in split order
-            float v = 0.f;
-            for (int s0 = 0; s0 < J.d; s0 += 8) {
-                float q[8];
+    const int kv = g.kv, runs = (int)J.z2, per = (kv + runs - 1) / runs, orun = (g.Og + kFoldRows - 1) / kFoldRows;
+    const int t0 = (int)(blk % runs) * per, c0 = (int)(blk / runs % J.e) * kFoldChannels;
+    const int ro = (int)(blk / runs / J.e), j = ro / orun, o0 = (ro - j * orun) * kFoldRows;
+    const int nc = g.Cg - c0 < kFoldChannels ? g.Cg - c0 : kFoldChannels, nt = kv - t0 < per ? kv - t0 : per;
+    const int r = threadIdx.x % kFoldRows, c4 = threadIdx.x / kFoldRows % (kFoldChannels / 4), t = threadIdx.x / (2 * kFoldChannels);
+    if (o0 + r < g.Og && c4 * 4 < nc && t < nt) {
+        const size_t rows = (size_t)g.G * J.a;
+        const float4* s = static_cast<const float4*>(J.src) + (size_t)(((t0 + t) * g.Cg + c0) / 4 + c4) * rows + j * J.a + o0 + r;
+        // loads in batches of four (independent, all in flight), additions in split order
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s0 = 0; s0 < J.d; s0 += 4) {
+            float4 q[4];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) q[u] = (s0 + u < J.d) ? __ldg(s + (size_t)(s0 + u) * J.z) : 0.f;
+            for (int u = 0; u < 4; ++u) q[u] = (s0 + u < J.d) ? __ldg(s + (size_t)(s0 + u) * (J.z / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (s0 + u < J.d) v = (s0 + u == 0) ? q[u] : v + q[u];
-            }
-            sm[c * (kFoldTaps + 1) + t] = v;
+            for (int u = 0; u < 4; ++u) { v.x += q[u].x; v.y += q[u].y; v.z += q[u].z; v.w += q[u].w; }
         }
-        __syncthreads();
-        for (int e = threadIdx.x; e < nc * nt; e += kPassThreads) {
-            const int t = e % nt, c = e / nt;
-            float* d = dst + (size_t)c * kv + t0 + t;
-            *d = J.c ? *d + sm[c * (kFoldTaps + 1) + t] : sm[c * (kFoldTaps + 1) + t];
-        }
+        float* d = sm + (r * kFoldChannels + c4 * 4) * (kFoldTaps + 1) + t;
+        d[0] = v.x; d[kFoldTaps + 1] = v.y; d[2 * (kFoldTaps + 1)] = v.z; d[3 * (kFoldTaps + 1)] = v.w;
+    }
+    __syncthreads();
+    const int rn = g.Og - o0 < kFoldRows ? g.Og - o0 : kFoldRows;
+    for (int e = threadIdx.x; e < rn * nc * nt; e += kPassThreads) {
+        const int wt = e % nt, q = e / nt, wc = q % nc, wr = q / nc;
+        float* d = static_cast<float*>(J.dst) + ((size_t)(j * g.Og + o0 + wr) * g.Cg + c0 + wc) * kv + t0 + wt;
+        const float v = sm[(wr * kFoldChannels + wc) * (kFoldTaps + 1) + wt];
+        *d = J.c ? *d + v : v;
     }
 }
 
@@ -547,16 +544,16 @@ public:
         J.blocks = (unsigned)J.a * (unsigned)J.b * (unsigned)g.N;
         need(64 * 65 * 4);
     }
-    void fold_dw(const Geom& g, const float* dwpk, float* dw, int rows, int cols, int splits, size_t slice, bool add_to) {
+    void fold_dw(const Geom& g, const float* dwpk, float* dw, int rows, int splits, size_t slice, bool add_to) {
         Job& J = add(g, kJobDw, dwpk, dw);
         J.a = rows;
-        J.b = cols;
         J.c = add_to ? 1 : 0;
         J.d = splits;
         J.e = (g.Cg + kFoldChannels - 1) / kFoldChannels;
         J.z = slice;
-        J.blocks = (unsigned)g.O * (unsigned)J.e;
-        need(kFoldChannels * (kFoldTaps + 1) * 4);
+        J.z2 = (size_t)(g.kv + kFoldTaps - 1) / kFoldTaps;
+        J.blocks = (unsigned)(g.G * ((g.Og + kFoldRows - 1) / kFoldRows)) * (unsigned)J.e * (unsigned)J.z2;
+        need(kFoldRows * kFoldChannels * (kFoldTaps + 1) * 4);
     }
     void fold_bias(const Geom& g, const float* row_sums, float* dbias, int MT, long long PC) {
         Job& J = add(g, kJobBias, row_sums, dbias);

@@ -16,6 +16,13 @@ constexpr int kWgStages = 3;
 constexpr int kWgNMax = 256;
 // elements of one position split's slice of the packed dW scratch; `items` = G * MB * NB (the kernels' gridDim.x)
 __host__ __device__ inline size_t wg_slice_elems(unsigned items) { return (size_t)items * 256 * kWgNMax; }
+// Where a split keeps the sums of row (group, output channel) and columns kq..kq+3: [split][columns / 4][rows][4], so that
+// the lanes of an epilogue warp (32 consecutive rows, four columns each) write 512 contiguous bytes.  (Rows of columns
+// instead cost 32 lines per store: 4 us of every launch per 128 rows, whatever the size.)
+__device__ __forceinline__ float4* wg_dw_ptr(float* dw, unsigned split, unsigned items, int NB, int row, int kq) {
+    const size_t rows = (size_t)(items / (unsigned)NB) * 256;
+    return reinterpret_cast<float4*>(dw + split * wg_slice_elems(items)) + (size_t)(kq / 4) * rows + row;
+}
 constexpr int kWgThreads = 32 * (2 + kProducerWarps + kEpilogueWarps);
 
 struct WgSmem {
@@ -148,10 +155,8 @@ tc_wgrad_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, cons
             for (int mt = 0; mt < mtb; ++mt) {
                 const int ol = (mb * 2 + mt) * 128 + q * 32 + lane;
                 const bool o_ok = ol < g.Og;
-                // partial sums of this position split: plain stores into its slice of the packed scratch
-                // dwpk[split][G][MB*256 rows][NB*256 columns] (added up in split order by the dW fold)
-                float* dwo = dw + (size_t)blockIdx.y * wg_slice_elems(gridDim.x) +
-                             ((size_t)j * MB * 256 + (o_ok ? ol : 0)) * ((size_t)NB * kWgNMax) + (size_t)nb * kWgNMax;
+                // partial sums of this position split: plain stores into its slice of the packed scratch (wg_dw_ptr;
+                // added up in split order by the dW fold)
                 for (int cc = 0; cc < NW / 32; ++cc) {
                     uint32_t v[32];
                     tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + mt * 256 + cc * 32, v);
@@ -161,7 +166,7 @@ tc_wgrad_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, cons
                     for (int i = 0; i < 8; ++i) {
                         const int kq = nb * kWgNMax + cc * 32 + 4 * i;
                         if (kq < g.kv * g.Cg)
-                            *reinterpret_cast<float4*>(dwo + cc * 32 + 4 * i) =
+                            *wg_dw_ptr(dw, blockIdx.y, gridDim.x, NB, j * MB * 256 + ol, kq) =
                                 make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
                                             __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
                     }
@@ -210,7 +215,7 @@ inline size_t dwpk_bytes(const Geom& g) {
 // the fold of the position splits' sums into dW (add: accumulate)
 inline void add_dw_fold(Passes& p, const Geom& g, const float* dwpk, float* dw, bool add) {
     const WgDims d = wg_dims(g);
-    p.fold_dw(g, dwpk, dw, d.MB * 256, d.NB * kWgNMax, d.splits, wg_slice_elems(g.G * d.MB * d.NB), add);
+    p.fold_dw(g, dwpk, dw, d.MB * 256, d.splits, wg_slice_elems(g.G * d.MB * d.NB), add);
 }
 
 template <int D, bool DEFORM>
