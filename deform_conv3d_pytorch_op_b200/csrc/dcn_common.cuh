@@ -40,8 +40,9 @@ struct FastDiv {
 };
 
 // Programmatic dependent launch.  Kernels of one call are launched so that the next one's blocks may take their place on
-// the SMs while the last blocks of this one still run (launch_dependent): every such kernel lets its successor start at
-// once (the last one of a call does not: what follows it is not ours) and waits, before it touches global memory, until its predecessor has completed and its writes are visible.  As
+// the SMs while the last blocks of this one still run (launch_dependent): every such kernel lets its successor start
+// (passes at once, the long kernels towards their end; the last one of a call does not: what follows it is not ours) and
+// waits, before it touches global memory, until its predecessor has completed and its writes are visible.  As
 // every kernel of the chain waits, completion carries over from the first to the last.  It hides the launch latency and
 // the set-up of each kernel, 1 to 2 us a boundary.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -830,7 +830,6 @@ exact_weight_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl,
 
     Acc<T, TM, TN> acc;
     acc.clear();
-    pdl_trigger();
     pdl_wait();
     if (ch0 < ch1) {
         long long ci = ch0, cf = ch0;                                 // chunks of the next item to issue / entry to fetch
@@ -879,6 +878,7 @@ exact_weight_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl,
             if (more) store_dy(buf ^ 1);
         }
     }
+    pdl_trigger();
 #pragma unroll
     for (int h = 0; h < TN / 4; ++h) {
         const int k0 = blockIdx.x * BN + tile_col(tx, h);
@@ -964,7 +964,6 @@ exact_data_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl, c
     Acc<T, TM, TN> acc;
     acc.clear();
     const int nch = (g.Og + kBK - 1) / kBK;
-    pdl_trigger();
     pdl_wait();
     load(0);
     store(0);
@@ -996,6 +995,7 @@ exact_data_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl, c
         }
     }
     T (*con)[NG][BN] = reinterpret_cast<T (*)[NG][BN]>(smem);
+    pdl_trigger();
     if constexpr (DEFORM) {
         __syncthreads();                                   // the operand tiles are done with
         if (ty == 0) {                                     // (two warps hold such threads: all sixteen tx)

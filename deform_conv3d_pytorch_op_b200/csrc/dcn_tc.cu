@@ -156,7 +156,7 @@ BwdDataWorkspace bwd_data_workspace(const Geom& g) {
     size_t wpk_bytes = (size_t)g.G * d.NB * d.OC * 2 * kTileBytes;
     if (g.Cg % 8 == 0 && b2_wpk_bytes(g) > wpk_bytes) wpk_bytes = b2_wpk_bytes(g);   // slab-wise tiles of dcn_tc_bwd2d.cuh
     w.scale_off = w.wpk_off + align_up(wpk_bytes, 256);
-    w.dxcl_off = w.scale_off + 256;                    // two words: bit patterns of max|dy| and max|W|
+    w.dxcl_off = w.scale_off + 256;                    // two words: bit patterns of max|dy| and max|W|; or the tile counter
     w.dxcl_bytes = align_up((size_t)g.N * g.iv * g.C * 4, 256);
     // the shared-memory-accumulating kernel has no channels-last dX scratch; its sampling-point entries live there
     if (g.Cg % 8 == 0 && b2_points_bytes(g) > w.dxcl_bytes) w.dxcl_bytes = align_up(b2_points_bytes(g), 256);
@@ -261,7 +261,7 @@ struct Backward {
         }
         if (scatter) {
             if (dx_cl && dx != nullptr && (reinterpret_cast<uintptr_t>(dx) & 15) != 0) return -7;   // 16-byte reductions
-            p.weight(g, kTilesBwd, w, base + l.wpk_off);
+            p.weight(g, kTilesBwd, w, base + l.wpk_off, nullptr, scale());      // (clears the kernel's tile counter)
             if (dx != nullptr && !(dx_cl && dx_partial)) p.zero(dxcl(), (size_t)g.N * g.iv * g.C);
         }
         if (doff != nullptr) p.zero(doff, (size_t)g.N * g.dg * g.kv * ndim * g.ov);
@@ -287,10 +287,10 @@ struct Backward {
             r = launch_tc_bwd2d(g, xcl, reinterpret_cast<uint4*>(base + l.dxcl_off), dpk, base + l.wpk_off, scale(), dx, doff,
                                 dx_partial, st);
         if (scatter) {
-            if (ndim == 2) r = deform ? launch_tc_dgrad<2, true>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, st)
-                                      : launch_tc_dgrad<2, false>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, st);
-            else r = deform ? launch_tc_dgrad<3, true>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, st)
-                            : launch_tc_dgrad<3, false>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, st);
+            if (ndim == 2) r = deform ? launch_tc_dgrad<2, true>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, scale(), st)
+                                      : launch_tc_dgrad<2, false>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, scale(), st);
+            else r = deform ? launch_tc_dgrad<3, true>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, scale(), st)
+                            : launch_tc_dgrad<3, false>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, scale(), st);
         }
         if (r == 0 && gather) {
             const FwdWorkspace f = fwd_workspace(gt);

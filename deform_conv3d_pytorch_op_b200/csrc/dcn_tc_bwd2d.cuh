@@ -209,7 +209,6 @@ tc_bwd2d_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const uint4
         mbar_init(&ctl->w_empty, 1);
         fence_barrier_init();
     }
-    pdl_trigger();
     pdl_wait();
     if (warp == 0) {
         tmem_alloc(&ctl->tmem_base, 256);
@@ -566,6 +565,7 @@ tc_bwd2d_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const uint4
         }
     }
 
+    pdl_trigger();              // (late: a waiting block of the next kernel would take shared memory from this one's L1)
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {

@@ -54,7 +54,6 @@ tc_dgrad_rowwise_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, con
         }
         fence_barrier_init();
     }
-    pdl_trigger();
     pdl_wait();
     if (warp == 0) {
         tmem_alloc(tmem_slot, 512);
@@ -239,6 +238,7 @@ tc_dgrad_rowwise_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, con
         }
     }
 
+    pdl_trigger();              // (late: a waiting block of the next kernel would take shared memory from this one's L1)
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {

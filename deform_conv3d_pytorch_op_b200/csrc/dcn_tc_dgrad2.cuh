@@ -36,7 +36,7 @@ struct Dg2Smem {
     static constexpr int kEntryBytes = kSlots * 32 * (int)sizeof(DgEntry<D, DEFORM>);   // per warp: slots x 32 rows
     static constexpr int kWarpBytes = (kColFloats + kTotFloats) * 4 + kEntryBytes;
     static constexpr int kBarOffset = kStagesBytes + EW * kWarpBytes;
-    static constexpr int kTotal = kBarOffset + (2 * kDg2Stages + 4) * 8 + 16;
+    static constexpr int kTotal = kBarOffset + (2 * kDg2Stages + 8) * 8 + 16;
 };
 
 // EW epilogue warps: 8 (each 128 columns of the tile) or 16 (each 64 columns).
@@ -45,8 +45,8 @@ template <int D, bool DEFORM, int EW, int U>
 __global__ void __launch_bounds__(32 * (2 + EW), 1)
 tc_dgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float* __restrict__ off,
                 const uint8_t* __restrict__ dpk, const uint8_t* __restrict__ wpk, float* __restrict__ dxcl,
-                float* __restrict__ doff, const int MT, const int NB, const int NW, const int OC,
-                const long long PC2, const long long PT) {
+                float* __restrict__ doff, unsigned int* __restrict__ next_tile, const int MT, const int NB, const int NW,
+                const int OC, const long long PC2, const long long PT) {
     using SM = Dg2Smem<D, DEFORM, EW, U>;
     using Entry = DgEntry<D, DEFORM>;
     constexpr int NC = 1 << D;
@@ -59,7 +59,13 @@ tc_dgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
     uint64_t* empty = full + kDg2Stages;
     uint64_t* acc_full = empty + kDg2Stages;
     uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    // Tiles are handed out in order as CTAs get free (next_tile, zero at the start): the rate at which an SM reduces into
+    // L2 differs between SMs, and with a fixed share each the fastest were done 10 % of the kernel's time before the
+    // slowest.  The loader draws the tiles and passes them on through a ring of two, so it is at most two ahead.
+    uint64_t* tile_full = acc_empty + 2;
+    uint64_t* tile_empty = tile_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tile_empty + 2);
+    volatile int* tile_of = reinterpret_cast<volatile int*>(tmem_slot + 1);     // [2]; < 0: no more
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
@@ -71,10 +77,11 @@ tc_dgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], EW);
+            mbar_init(&tile_full[b], 1);
+            mbar_init(&tile_empty[b], EW + 1);           // the epilogue warps and the MMA thread
         }
         fence_barrier_init();
     }
-    pdl_trigger();
     pdl_wait();
     if (warp == 0) {
         tmem_alloc(tmem_slot, 512);
@@ -92,8 +99,11 @@ tc_dgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
         if (lane == 0) {
             uint32_t it = 0, tl = 0;
             bool ok = true;
-            for (long long t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++tl) {
+            for (; ok; ++tl) {
                 const uint32_t b = tl & 1;
+                ok = mbar_wait(&tile_full[b], (tl >> 1) & 1);
+                if (!ok || tile_of[b] < 0) break;
+                mbar_arrive(&tile_empty[b]);
                 ok = mbar_wait(&acc_empty[b], ((tl >> 1) & 1) ^ 1);
                 tc_fence_after();
                 for (int oc = 0; oc < OC && ok; ++oc, ++it) {
@@ -116,9 +126,16 @@ tc_dgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            uint32_t it = 0;
+            uint32_t it = 0, tl = 0;
             bool ok = true;
-            for (long long t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+            for (; ok; ++tl) {
+                const uint32_t tb = tl & 1;
+                ok = mbar_wait(&tile_empty[tb], ((tl >> 1) & 1) ^ 1);
+                if (!ok) break;
+                const long long t = atomicAdd(next_tile, 1u);
+                tile_of[tb] = t < n_tiles ? (int)t : -1;
+                mbar_arrive(&tile_full[tb]);
+                if (t >= n_tiles) break;
                 const int nb = (int)(t % NB);
                 const long long pt = (t / NB) % PT;
                 const int j = (int)(t / NB / PT);
@@ -153,11 +170,16 @@ tc_dgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
         const bool want_x = DEFORM && doff != nullptr;
         uint32_t tl = 0;
         bool ok = true;
-        for (long long t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++tl) {
+        for (; ok; ++tl) {
+            const uint32_t b = tl & 1;
+            ok = mbar_wait(&tile_full[b], (tl >> 1) & 1);
+            if (!ok) break;
+            const long long t = tile_of[b];
+            if (t < 0) break;
+            mbar_arrive_warp(&tile_empty[b]);
             const int nb = (int)(t % NB);
             const long long pt = (t / NB) % PT;
             const int j = (int)(t / NB / PT);
-            const uint32_t b = tl & 1;
             const long long P = pt * 128 + q * 32 + lane;          // phase-A position of this thread
             const bool p_ok = P < g.P;
             const OutPos op = decompose_pos(g, p_ok ? P : 0);
@@ -387,6 +409,7 @@ tc_dgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
         }
     }
 
+    pdl_trigger();              // (late: a waiting block of the next kernel would take shared memory from this one's L1)
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -408,7 +431,7 @@ inline int dgrad_key_unit(const Geom& g, int deform) {
 
 template <int D, bool DEFORM, int EW, int U>
 int launch_tc_dgrad_t(const Geom& g, const __nv_bfloat16* xcl, const float* off, const uint8_t* dpk,
-                      const uint8_t* wpk, float* dxcl, float* doff, cudaStream_t st) {
+                      const uint8_t* wpk, float* dxcl, float* doff, unsigned int* next_tile, cudaStream_t st) {
     const DgDims d = dg_dims(g);
     const int smem = Dg2Smem<D, DEFORM, EW, U>::kTotal;
     static_assert(Dg2Smem<D, DEFORM, EW, U>::kTotal <= kSmemLimit, "dgrad epilogue staging does not fit");
@@ -416,16 +439,17 @@ int launch_tc_dgrad_t(const Geom& g, const __nv_bfloat16* xcl, const float* off,
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -5;
     const long long tiles = (long long)g.G * d.PT * d.NB;
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    return launch_dependent(kern, dim3(grid), dim3(32 * (2 + EW)), smem, st, g, xcl, off, dpk, wpk, dxcl, doff, d.MT, d.NB, d.NW,
-                            d.OC, d.PC2, d.PT) == cudaSuccess ? 0 : -5;
+    return launch_dependent(kern, dim3(grid), dim3(32 * (2 + EW)), smem, st, g, xcl, off, dpk, wpk, dxcl, doff, next_tile, d.MT,
+                            d.NB, d.NW, d.OC, d.PC2, d.PT) == cudaSuccess ? 0 : -5;
 }
 
+// next_tile: a word that the prologue has zeroed
 template <int D, bool DEFORM>
 int launch_tc_dgrad(const Geom& g, const __nv_bfloat16* xcl, const float* off, const uint8_t* dpk,
-                    const uint8_t* wpk, float* dxcl, float* doff, cudaStream_t st) {
+                    const uint8_t* wpk, float* dxcl, float* doff, unsigned int* next_tile, cudaStream_t st) {
     const int u = dgrad_key_unit(g, DEFORM ? 1 : 0);
-    if (u == 32) return launch_tc_dgrad_t<D, DEFORM, 16, 32>(g, xcl, off, dpk, wpk, dxcl, doff, st);
+    if (u == 32) return launch_tc_dgrad_t<D, DEFORM, 16, 32>(g, xcl, off, dpk, wpk, dxcl, doff, next_tile, st);
     // two keys per chunk double the per-warp staging: 8 epilogue warps
-    if (u == 16) return launch_tc_dgrad_t<D, DEFORM, 8, 16>(g, xcl, off, dpk, wpk, dxcl, doff, st);
+    if (u == 16) return launch_tc_dgrad_t<D, DEFORM, 8, 16>(g, xcl, off, dpk, wpk, dxcl, doff, next_tile, st);
     return launch_tc_dgrad_rowwise<D, DEFORM>(g, xcl, off, dpk, wpk, dxcl, doff, st);
 }

@@ -95,6 +95,7 @@ __device__ __forceinline__ void job_weight(const Geom& g, const Job& J, unsigned
     const int stride = CC * kv + 1;
     const float* w = static_cast<const float*>(J.src);
     uint8_t* dst = static_cast<uint8_t*>(J.dst);
+    if (J.aux != nullptr && blk == 0 && threadIdx.x == 0) *static_cast<unsigned int*>(J.aux) = 0u;
     float mx = 0.f;
 #pragma unroll 4
     for (int e = threadIdx.x; e < R * CC * kv; e += kPassThreads) {        // (div: by CC * kv)
@@ -478,9 +479,11 @@ public:
             need(64 * 65 * 4);
         }
     }
-    void weight(const Geom& g, WeightTiles tiles, const float* w, void* dst, unsigned int* mx = nullptr) {
+    // clear: a word to set to zero on the way
+    void weight(const Geom& g, WeightTiles tiles, const float* w, void* dst, unsigned int* mx = nullptr, unsigned int* clear = nullptr) {
         Job& J = add(g, kJobWeight, w, dst);
         J.mx = mx;
+        J.aux = clear;
         J.a = tiles;
         int rows = g.Og, chans = g.Cg;
         if (tiles == kTilesFwd) {

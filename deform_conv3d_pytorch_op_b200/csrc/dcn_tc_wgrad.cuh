@@ -64,7 +64,6 @@ tc_wgrad_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, cons
         mbar_init(acc_full, 1);
         fence_barrier_init();
     }
-    pdl_trigger();
     pdl_wait();
     if (warp == 0) {
         tmem_alloc(tmem_slot, 512);
@@ -175,6 +174,7 @@ tc_wgrad_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, cons
         }
     }
 
+    pdl_trigger();              // (late: a waiting block of the next kernel would take shared memory from this one's L1)
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {

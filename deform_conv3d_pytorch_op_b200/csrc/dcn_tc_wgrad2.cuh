@@ -66,7 +66,6 @@ tc_wgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
         }
         fence_barrier_init();
     }
-    pdl_trigger();
     pdl_wait();
     if (warp == 0) {
         tmem_alloc(&ctl->tmem_base, 512);
@@ -308,6 +307,7 @@ tc_wgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
         }
     }
 
+    pdl_trigger();              // (late: a waiting block of the next kernel would take shared memory from this one's L1)
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
