@@ -17,12 +17,14 @@ constexpr int kWgNMax = 256;
 // elements of one position split's slice of the packed dW scratch; `items` = G * MB * NB (the kernels' gridDim.x)
 __host__ __device__ inline size_t wg_slice_elems(unsigned items) { return (size_t)items * 256 * kWgNMax; }
 // Where a split keeps the sums of row (group, output channel) and columns kq..kq+3: [split][columns / 4][rows][4], so that
-// the lanes of an epilogue warp (32 consecutive rows, four columns each) write 512 contiguous bytes.  (Rows of columns
-// instead cost 32 lines per store: 4 us of every launch per 128 rows, whatever the size.)
-__device__ __forceinline__ float4* wg_dw_ptr(float* dw, unsigned split, unsigned items, int NB, int row, int kq) {
-    const size_t rows = (size_t)(items / (unsigned)NB) * 256;
-    return reinterpret_cast<float4*>(dw + split * wg_slice_elems(items)) + (size_t)(kq / 4) * rows + row;
-}
+// the lanes of an epilogue warp (32 consecutive rows, four columns each) write 512 contiguous bytes.
+struct WgDst {
+    float4* base;
+    size_t rows;
+    __device__ __forceinline__ WgDst(float* dw, unsigned split, unsigned items, int NB, int row)
+        : base(reinterpret_cast<float4*>(dw + split * wg_slice_elems(items)) + row), rows((size_t)(items / (unsigned)NB) * 256) {}
+    __device__ __forceinline__ float4& at(int kq) const { return base[(size_t)(kq / 4) * rows]; }
+};
 constexpr int kWgThreads = 32 * (2 + kProducerWarps + kEpilogueWarps);
 
 struct WgSmem {
@@ -154,8 +156,9 @@ tc_wgrad_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, cons
             for (int mt = 0; mt < mtb; ++mt) {
                 const int ol = (mb * 2 + mt) * 128 + q * 32 + lane;
                 const bool o_ok = ol < g.Og;
-                // partial sums of this position split: plain stores into its slice of the packed scratch (wg_dw_ptr;
-                // added up in split order by the dW fold)
+                // partial sums of this position split: plain stores into its slice of the packed scratch (added
+                // up in split order by the dW fold)
+                const WgDst dst(dw, blockIdx.y, gridDim.x, NB, j * MB * 256 + ol);
                 for (int cc = 0; cc < NW / 32; ++cc) {
                     uint32_t v[32];
                     tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + mt * 256 + cc * 32, v);
@@ -165,7 +168,7 @@ tc_wgrad_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, cons
                     for (int i = 0; i < 8; ++i) {
                         const int kq = nb * kWgNMax + cc * 32 + 4 * i;
                         if (kq < g.kv * g.Cg)
-                            *wg_dw_ptr(dw, blockIdx.y, gridDim.x, NB, j * MB * 256 + ol, kq) =
+                            dst.at(kq) =
                                 make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
                                             __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
                     }

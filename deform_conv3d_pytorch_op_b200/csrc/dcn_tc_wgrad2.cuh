@@ -196,9 +196,10 @@ tc_wgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
             for (int mt = 0; mt < mtb; ++mt) {
                 const int ol = (mb * 2 + mt) * 128 + q * 32 + lane;
                 const bool o_ok = ol < g.Og;
-                // The partial sums of this position split go to ITS slice of the packed scratch (wg_dw_ptr) with
+                // The partial sums of this position split go to ITS slice of the packed scratch with
                 // plain 16-byte stores: every element a slice's reader touches is written exactly once, and the dW
                 // fold adds the slices in split order, so dW does not depend on the order in which the CTAs finish.
+                const WgDst dst(dw, blockIdx.y, gridDim.x, NB, j * MB * 256 + ol);
                 for (int cc = 0; cc < NW / 16; ++cc) {
                     uint32_t v[16];
                     tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + mt * 256 + cc * 16, v);
@@ -208,7 +209,7 @@ tc_wgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
                     for (int i = 0; i < 4; ++i) {
                         const int kq = nb * kWgNMax + cc * 16 + 4 * i;
                         if (kq < g.kv * g.Cg)
-                            *wg_dw_ptr(dw, blockIdx.y, gridDim.x, NB, j * MB * 256 + ol, kq) =
+                            dst.at(kq) =
                                 make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
                                             __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
                     }
