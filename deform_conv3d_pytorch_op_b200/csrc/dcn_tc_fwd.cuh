@@ -24,6 +24,7 @@ constexpr int kFwdStageBytes = 3 * kTileBytes;      // A0 | A1 | B
 constexpr int kSmemLimit = 232448;                   // 227 KB opt-in maximum per CTA
 
 constexpr int kFwdMaxTabs = 6;
+constexpr int kFwdOutBytes = kFwdCoordWarps * 32 * 33 * (int)sizeof(float);
 constexpr int kFwdOffRing = 2 * kFwdCoordWarps;   // two private offset staging buffers per coordinate warp
 
 struct FwdCtl {            // lives behind the stages, the tables and the offset staging ring
@@ -59,7 +60,8 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdSplit& sp, long long t, int
     return it;
 }
 
-template <int D, bool DEFORM, int GW>
+// TURN: see FwdPlan::turn (a kernel of its own: with both epilogues in one the 3-D kernel spills, 1000 -> 1095 us)
+template <int D, bool DEFORM, int GW, bool TURN>
 __global__ void __launch_bounds__(fwd_threads(GW), 1)
 tc_forward_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float* __restrict__ off,
                   const uint8_t* __restrict__ wpk, const float* __restrict__ bias, float* __restrict__ y,
@@ -74,6 +76,7 @@ tc_forward_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const flo
     float* ostage = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(tab) +
                                              (size_t)n_tabs * max_slots * 128 * sizeof(Entry));   // [kFwdOffRing][max_slots][D][128]
     FwdCtl* ctl = reinterpret_cast<FwdCtl*>(ostage + (size_t)kFwdOffRing * max_slots * D * 128);
+    float* obuf = reinterpret_cast<float*>(ctl + 1);                // turn: [kFwdCoordWarps][32][33], see the epilogue
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
@@ -265,6 +268,41 @@ tc_forward_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const flo
                     const bool o_ok = ol < g.Og;
                     const int o = j * g.Og + ol;
                     const float bv = (bias != nullptr && o_ok && ks == 0) ? __ldg(bias + o) : 0.f;
+                    if constexpr (TURN) {
+                        // Channel-first y whose rows are not 16-byte aligned: 32 x 32 pieces are turned in shared memory
+                        // and leave as 128-byte runs along the positions.  (A lane storing its own row of an odd size
+                        // value by value touches 32 lines per instruction: 2 x 128 channels at 101x151, 67 us against
+                        // 57 us.  Aligned rows stay with the 16-byte stores below, which are faster still.)
+                        float* ob = obuf + cw * 32 * 33;
+#pragma unroll 1
+                        for (int cc = 0; cc < kTileN / 32; ++cc) {
+                            const long long P = pt * kTileN + cc * 32 + lane;
+                            if (pt * kTileN + cc * 32 >= g.P) break;
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                uint32_t v[16];
+                                tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + b * 256 + mt * 128 + cc * 32 + h * 16, v);
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) ob[lane * 33 + h * 16 + i] = __uint_as_float(v[i]) + bv;
+                            }
+                            __syncwarp();
+                            uint32_t n, opos;
+                            g.d_ov.divmod((uint32_t)(P < g.P ? P : 0), n, opos);
+                            const int o0 = (mb * 2 + mt) * 128 + q * 32;
+                            float* d1 = y + ((size_t)n * g.O + j * g.Og + o0) * g.ov + opos;
+                            const int rows = g.Og - o0 < 32 ? g.Og - o0 : 32;
+                            if (P < g.P) {
+#pragma unroll 4
+                                for (int r = 0; r < rows; ++r, d1 += g.ov) {
+                                    const float val = ob[r * 33 + lane];
+                                    if (plain) *d1 = val;
+                                    else atomicAdd(d1, val);
+                                }
+                            }
+                            __syncwarp();
+                        }
+                    } else {
 #pragma unroll 1
                     for (int cc = 0; cc < kTileN / 16; ++cc) {
                         uint32_t v[16];
@@ -309,6 +347,7 @@ tc_forward_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const flo
                                 }
                             }
                         }
+                    }
                     }
                 }
                 tc_fence_before();
@@ -526,6 +565,7 @@ inline int max_slots_per_chunk(const Geom& g, int cols_per_chunk) {
 struct FwdPlan {
     FwdSplit sp;
     int stages, n_tabs, smem, max_slots, grid;
+    int turn;                            // rows of a channel-first y are not 16-byte aligned
     bool direct;                         // the corner table does not fit beside the stages
     struct { float* p; size_t len; int rows, pitch; } zero[2];
     int zeros;
@@ -537,10 +577,11 @@ FwdPlan fwd_plan(const Geom& g, float* y, bool accumulate) {
     const TcDims d = tc_dims(g);
     FwdPlan pl = {};
     pl.max_slots = max_slots_per_chunk(g, 8);
+    pl.turn = !g.cl && (g.ov % 4 != 0 || (reinterpret_cast<uintptr_t>(y) & 15) != 0) ? 1 : 0;
     const size_t tab_one = (size_t)pl.max_slots * 128 * sizeof(TabEntry<D, DEFORM>);
     const size_t ost_bytes = (size_t)kFwdOffRing * pl.max_slots * D * 128 * sizeof(float);
     auto need = [&](int stages, int tabs) {
-        return (long long)stages * kFwdStageBytes + (long long)tabs * tab_one + ost_bytes + sizeof(FwdCtl) + 1024;
+        return (long long)stages * kFwdStageBytes + (long long)tabs * tab_one + ost_bytes + sizeof(FwdCtl) + (pl.turn ? kFwdOutBytes : 0) + 1024;
     };
     // The four coordinate warps work on four tables at once and wait on the barriers of a table buffer by phase
     // parity, which is only sound while no warp runs two laps of the ring ahead of another: with the tables
@@ -616,7 +657,7 @@ int launch_tc_forward(const Geom& g, const FwdPlan& pl, const __nv_bfloat16* xcl
     if (pl.direct) return launch_tc_forward_direct<D, DEFORM>(g, xcl, off, wpk, bias, y, st);
     const TcDims d = tc_dims(g);
     constexpr int GW = 16;
-    auto kern = tc_forward_kernel<D, DEFORM, GW>;
+    auto kern = pl.turn ? tc_forward_kernel<D, DEFORM, GW, true> : tc_forward_kernel<D, DEFORM, GW, false>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem) != cudaSuccess) return -5;
     return launch_dependent(kern, dim3(pl.grid), dim3(fwd_threads(GW)), pl.smem, st, g, xcl, off, wpk, bias, y, d.KC, d.MT, d.MB,
                             d.PT, pl.stages, pl.max_slots, pl.n_tabs, pl.sp) == cudaSuccess ? 0 : -5;
