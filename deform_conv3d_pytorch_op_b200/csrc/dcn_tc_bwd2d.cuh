@@ -378,6 +378,15 @@ tc_bwd2d_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const uint4
                 const uint32_t opos = p_ok ? (uint32_t)(P - pbeg) : 0u;
                 // the warps of a quarter take turns at the tap residues, so that the uneven share evens out over tiles
                 const int k3 = (kq + (int)tl) % WQ, k3n = (kq + (int)tl + 1) % WQ;
+                if (!FULL && k3 >= g.kv) {
+                    // fewer taps than warps of a quarter: no tap of this tile is this warp's, but the accumulator is
+                    // released only when every warp has arrived
+                    if (t + 1 < wi.tiles) fetch_points(P + 128, k3n);
+                    ok = mbar_wait(&ctl->acc_full[b], (tl >> 1) & 1);
+                    if (!ok) break;
+                    mbar_arrive_warp(&ctl->acc_empty[b]);
+                    continue;
+                }
                 for (int tg = k3; tg < g.kv; tg += WQ * TG) {
                     // ---- sampling points of this group from the entries fetched a group ago.  An invalid point is an
                     // all-zero entry: first block of the plane, zero weights, so the code below runs without
