@@ -596,55 +596,74 @@ FwdPlan fwd_plan(const Geom& g, float* y, bool accumulate) {
         return pl;
     }
     pl.smem = (int)need(pl.stages, pl.n_tabs);
-    // split the K range when there are fewer tiles than SMs (small batches / late layers of a network)
+    // Two ways of splitting tiles along K so that the SMs are busy to the end; both are weighed in K chunks of work, an
+    // item costing six beside its own (its sums are added to y), and no item gets under three (B200, 2 x 128 channels 40x41, 26 tiles of 18
+    // chunks, kernel time at 9 / 6 / 5 / 3 chunks an item: 18.3 / 15.6 / 14.8 / 13.9 us):
+    //   every tile into KS0 pieces (few tiles, or a badly filled last wave), all of y zero-filled;
+    //   the R tiles left after the last full wave into KS1 pieces, as many as there are SMs to take them.  They have to
+    //   lie in the last (group, channel block), so that they are a position range [P0, P) of its channels and only that
+    //   part of y is zero-filled.
     const long long base_tiles = (long long)g.G * d.MB * d.PT;
     const int S = sm_count();
+    auto waves = [&](long long items) { return (items + S - 1) / S; };
+    auto cost = [&](long long items, int chunks) { return waves(items) * (chunks + 6); };
+    auto pieces = [&](int want, int& chunks) {           // of a tile; chunks: of one piece
+        chunks = (d.KC + want - 1) / want;
+        return (d.KC + chunks - 1) / chunks;
+    };
     FwdSplit& sp = pl.sp;
     sp.acc = accumulate ? 1 : 0;
     sp.KS0 = 1;
-    if (base_tiles * 2 <= S) {
-        sp.KS0 = (int)(S / base_tiles);
-        if (sp.KS0 > d.KC / 8) sp.KS0 = d.KC / 8;          // at least 8 chunks per split
-        if (sp.KS0 < 1) sp.KS0 = 1;
+    sp.cpk0 = d.KC;
+    long long best = cost(base_tiles, d.KC);
+    for (int k = 2; k <= d.KC / 3 && base_tiles * k <= 3ll * S; ++k) {
+        int chunks;
+        const int ks = pieces(k, chunks);
+        const long long c = cost(base_tiles * ks, chunks) + 2;       // (the zero fill)
+        if (c * 20 < best * 19) { best = c; sp.KS0 = ks; sp.cpk0 = chunks; }
     }
-    sp.cpk0 = (d.KC + sp.KS0 - 1) / sp.KS0;
-    sp.KS0 = (d.KC + sp.cpk0 - 1) / sp.cpk0;
-    sp.T0 = base_tiles * sp.KS0;
-    sp.tile1 = base_tiles;
-    sp.KS1 = 1;
-    sp.cpk1 = d.KC;
-    sp.n_items = sp.T0;
+    const long long R = base_tiles % S;
+    const int oA = (g.G - 1) * g.Og + (d.MB - 1) * 256, Ob = g.O - oA;      // channels of the last block
+    int ks1 = 1, cpk1 = d.KC;
+    if (base_tiles > S && R != 0 && R <= d.PT && (long long)g.O * g.ov < (1ll << 31)) {
+        long long want = S / R;
+        if (want > d.KC / 3) want = d.KC / 3;
+        if (want >= 2) {
+            ks1 = pieces((int)want, cpk1);
+            if (base_tiles / S * (d.KC + 6) + cost(R * ks1, cpk1) + 1 < best) {
+                sp.KS0 = 1;
+                sp.cpk0 = d.KC;
+            } else {
+                ks1 = 1;
+            }
+        }
+    }
+    const bool tail = ks1 > 1;
+    sp.T0 = tail ? base_tiles - R : base_tiles * sp.KS0;
+    sp.tile1 = tail ? sp.T0 : base_tiles;
+    sp.KS1 = ks1;
+    sp.cpk1 = tail ? cpk1 : d.KC;
+    sp.n_items = tail ? sp.T0 + R * ks1 : sp.T0;
     auto zero = [&](float* p, size_t len, int rows, int pitch) {
         auto& z = pl.zero[pl.zeros++];
         z.p = p; z.len = len; z.rows = rows; z.pitch = pitch;
     };
-    if (sp.KS0 > 1) {
-        if (!accumulate) zero(y, (size_t)g.N * g.O * g.ov, 1, 0);
-    } else if (!accumulate && g.G * d.MB == 1 && base_tiles > S && base_tiles % S != 0) {
-        // Tail of an uneven grid: the R tiles left after the last full wave are split along K into as many pieces
-        // as there are SMs to take them.  With one (group, channel block) the tile index is the position tile, so
-        // the tail is the position range [P0, P) and only that part of y is zero-filled.
-        const long long R = base_tiles % S;
-        int ks1 = (int)(S / R);
-        if (ks1 > d.KC / 8) ks1 = d.KC / 8;
-        if (ks1 >= 2) {
-            sp.cpk1 = (d.KC + ks1 - 1) / ks1;
-            sp.KS1 = (d.KC + sp.cpk1 - 1) / sp.cpk1;
-            sp.T0 = base_tiles - R;
-            sp.tile1 = sp.T0;
-            sp.n_items = sp.T0 + R * sp.KS1;
-            const long long P0 = sp.T0 * kTileN;
-            if (g.cl) {
-                zero(y + (size_t)P0 * g.O, (size_t)(g.P - P0) * g.O, 1, 0);
-            } else {
-                long long n0 = P0 / g.ov;
-                const long long o0 = P0 % g.ov;
-                if (o0 != 0) {      // the sample the tail starts in: the positions [o0, ov) of every channel
-                    zero(y + (size_t)n0 * g.O * g.ov + o0, (size_t)(g.ov - o0), g.O, g.ov);
-                    ++n0;
-                }
-                if (n0 < g.N) zero(y + (size_t)n0 * g.O * g.ov, (size_t)(g.N - n0) * g.O * g.ov, 1, 0);
+    if (!accumulate && sp.KS0 > 1) zero(y, (size_t)g.N * g.O * g.ov, 1, 0);
+    if (!accumulate && tail) {
+        const long long P0 = (d.PT - R) * kTileN;
+        if (g.cl) {
+            if (Ob == g.O) zero(y + (size_t)P0 * g.O, (size_t)(g.P - P0) * g.O, 1, 0);
+            else zero(y + (size_t)P0 * g.O + oA, (size_t)Ob, (int)(g.P - P0), g.O);
+        } else {
+            long long n0 = P0 / g.ov;
+            const long long o0 = P0 % g.ov;
+            if (o0 != 0) {      // the sample the tail starts in: the positions [o0, ov) of every channel
+                zero(y + ((size_t)n0 * g.O + oA) * g.ov + o0, (size_t)(g.ov - o0), Ob, g.ov);
+                ++n0;
             }
+            float* rest = y + ((size_t)n0 * g.O + oA) * g.ov;
+            if (n0 < g.N && Ob == g.O) zero(rest, (size_t)(g.N - n0) * g.O * g.ov, 1, 0);
+            else if (n0 < g.N) zero(rest, (size_t)Ob * g.ov, (int)(g.N - n0), g.O * g.ov);
         }
     }
     pl.grid = (int)(sp.n_items < S ? sp.n_items : S);

@@ -201,10 +201,14 @@ inline WgDims wg_dims(const Geom& g) {
     d.NW = kq >= kWgNMax ? kWgNMax : ((kq + 63) / 64) * 64;
     d.PC = 2 * ((g.P + 127) / 128);     // 64-position chunks, even count (shared tile layout with dgrad)
     const long long items = (long long)g.G * d.MB * d.NB;
-    long long splits = sm_count() / items;      // floor: the whole grid must fit in one wave (one CTA per SM)
-    if (splits > d.PC) splits = d.PC;
-    if (splits < 1) splits = 1;
-    if (splits > 65535) splits = 65535;
+    // position slices: CTAs in up to three waves, weighed in chunks of 64 positions, a CTA costing five beside its own
+    // (set-up and epilogue; 2 us a chunk)
+    const int S = sm_count();
+    long long splits = 1, best = 0;
+    for (long long k = 1; k <= d.PC && k <= 65535 && (k == 1 || items * k <= 3ll * S); ++k) {
+        const long long c = (items * k + S - 1) / S * ((d.PC + k - 1) / k + 5);
+        if (k == 1 || c < best) { best = c; splits = k; }
+    }
     d.cps = (int)((d.PC + splits - 1) / splits);
     d.splits = (int)((d.PC + d.cps - 1) / d.cps);
     return d;
