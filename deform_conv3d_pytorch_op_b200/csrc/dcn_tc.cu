@@ -444,7 +444,7 @@ int tc_backward(const Geom& g, int ndim, int deform, const float* x, const float
         p.copy_x(g, x, b.own_xcl());
         b.xcl = b.own_xcl();
     }
-    // (a call on its own keeps its passes apart, one name each on a profiler's timeline)
+    // (a call on its own launches its passes one by one, as dcn_launch_count states; autograd always hands the copy in)
     r = p.launch(st, false, xcl_in == nullptr);
     if (r == 0) r = b.run(st);
     if (r != 0) return r;
