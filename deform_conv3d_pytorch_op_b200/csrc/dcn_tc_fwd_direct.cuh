@@ -18,12 +18,13 @@ constexpr int kFwdDirectThreads = 32 * (2 + kProducerWarps + kEpilogueWarps);
 // K chunk is shared by both 128-row halves of the output-channel block.
 // ---------------------------------------------------------------------------------------------------
 struct FwdDirectSmem {
+    // (with the CTA's reserved kilobyte this stays under 196 KB, which leaves 60 KB of L1 to the gathers; 17 KB more for
+    // turning unaligned outputs, as tc_forward_kernel does, left 28 KB: config 4 forward 539 -> 575 us)
     // per stage: A0 | A1 | B, 16 KB each
     static constexpr int kStageBytes = 3 * kTileBytes;
     static constexpr int kBarOffset = kDirectStages * kStageBytes;
     // barriers: full[S], empty[S], acc_full[2], acc_empty[2]; then the tensor-memory base address
-    static constexpr int kOutOffset = kBarOffset + (2 * kDirectStages + 4) * 8 + 16;     // [4 epilogue warps][32][33] floats
-    static constexpr int kTotal = kOutOffset + 4 * 32 * 33 * 4;
+    static constexpr int kTotal = kBarOffset + (2 * kDirectStages + 4) * 8 + 16;
 };
 
 template <int D, bool DEFORM>
@@ -162,8 +163,6 @@ tc_forward_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, co
     } else {
         // ------------------------------------------------ epilogue
         const int q = warp & 3;                     // tensor-memory lane quarter this warp may access
-        float* ob = reinterpret_cast<float*>(smem + FwdDirectSmem::kOutOffset) + q * 32 * 33;
-        const bool turn = !g.cl && (g.ov % 4 != 0 || (reinterpret_cast<uintptr_t>(y) & 15) != 0);
         uint32_t tl = 0;
         bool ok = true;
         for (long long t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++tl) {
@@ -186,30 +185,12 @@ tc_forward_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, co
                     tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + b * 256 + mt * 128 + cc * 32, v);
                     tmem_ld_wait();
                     const long long P0 = pt * kTileN + cc * 32;
-                    if (P0 >= g.P || (!o_ok && !turn)) continue;
+                    if (!o_ok || P0 >= g.P) continue;
                     if (g.cl) {
                         // channels-last y: the 32 lanes of the warp hold 32 consecutive channels of a position
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
                             if (P0 + i < g.P) y[(size_t)(P0 + i) * g.O + o] = __uint_as_float(v[i]) + bv;
-                        continue;
-                    }
-                    if (turn) {
-                        // rows not 16-byte aligned: 32 x 32 pieces turned in shared memory (see tc_forward_kernel)
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) ob[lane * 33 + i] = __uint_as_float(v[i]) + bv;
-                        __syncwarp();
-                        const long long P = P0 + lane;
-                        if (P < g.P) {
-                            uint32_t n, opos;
-                            g.d_ov.divmod((uint32_t)P, n, opos);
-                            const int o0 = (mb * 2 + mt) * 128 + q * 32;
-                            float* d1 = y + ((size_t)n * g.O + j * g.Og + o0) * g.ov + opos;
-                            const int rows = g.Og - o0 < 32 ? g.Og - o0 : 32;
-#pragma unroll 8
-                            for (int r = 0; r < rows; ++r, d1 += g.ov) *d1 = ob[r * 33 + lane];
-                        }
-                        __syncwarp();
                         continue;
                     }
                     uint32_t n0, opos0;
