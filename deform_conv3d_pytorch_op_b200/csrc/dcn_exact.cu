@@ -254,7 +254,11 @@ __device__ __forceinline__ void load_row(const T* p, T (&r)[N]) {
 // into slots of shared memory that only the issuing thread reads, so that kAhead further items can be in flight without
 // registers to hold them: with one item in registers the forward and weight kernels waited for corners half of the time
 // (config 4: 0.80 and 0.73 ms, FMA pipe 40 % busy).
-constexpr int kAhead = 2, kStages = kAhead + 1;
+// 3-D fp32 keeps one item ahead, not two: eight corners an item, and at three CTAs per SM the third stage would push the
+// shared-memory carve-out from 196 to 228 KB and leave 28 KB of L1 instead of 60 (config 4: forward 0.69 -> 0.65, weight
+// 0.68 -> 0.64 ms; 2-D is 1 % slower with one).
+template <typename T, int D, bool DEFORM>
+constexpr int kAheadOf = sizeof(T) == 4 && D == 3 && DEFORM ? 1 : 2;
 
 template <int BYTES>
 __device__ __forceinline__ void cp_async_small(void* smem, const void* gmem, bool ok) {
@@ -268,6 +272,7 @@ __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.w
 
 template <typename T, int D, bool DEFORM, int V, int NT>
 struct Sampler {
+    static constexpr int kAhead = kAheadOf<T, D, DEFORM>, kStages = kAhead + 1;
     static constexpr int NC = DEFORM ? (1 << D) : 1, VB = V * (int)sizeof(T);
     static constexpr int kBytes = kStages * NC * NT * VB;
     char* slots;                     // [stage][corner][thread]
@@ -617,6 +622,7 @@ exact_forward_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl
         }
         return k;
     };
+    constexpr int kAhead = kAheadOf<T, D, DEFORM>, kStages = kAhead + 1;
     Sampler<T, D, DEFORM, V, NT> smp;
     smp.slots = smem_x + 2 * kBK * (BM + BN) * sizeof(T) + tid * V * sizeof(T);
     Entry<T> ent;
@@ -767,6 +773,7 @@ exact_weight_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl,
         xg.d_Cg4.divmod((uint32_t)(kp < xg.Kp ? kp : 0), tap[u], c[u]);
         if constexpr (DEFORM) pk[u] = pts + (size_t)(group_of(g, xg, j, c[u]) * g.kv + (int)tap[u]) * (size_t)g.P;
     }
+    constexpr int kAhead = kAheadOf<T, D, DEFORM>, kStages = kAhead + 1;
     Sampler<T, D, DEFORM, V, NT> smp;
     smp.slots = smem_x + 2 * kBK * (BM + PAD + BN) * sizeof(T) + tid * V * sizeof(T);
     Entry<T> ent;
