@@ -389,9 +389,9 @@ constexpr int kCopyTile = sizeof(T) == 4 ? 64 : 32;      // side of a transpose 
 template <typename T>
 struct PrepArgs {
     const T *x, *off, *w, *dy;
-    T *xcl, *wk, *zero, *dbias;      // wk: w2 (forward) or wt (backward)
+    T *xcl, *wk, *zero, *zero2, *dbias;      // wk: w2 (forward) or wt (backward)
     Entry<T>* pts;
-    size_t zero_n;                   // elements
+    size_t zero_n, zero2_n;          // elements
     unsigned nb, nx, np, nw, nz;     // blocks of each part
     unsigned tx, ty;                 // input copy: tiles along the positions / channels
     unsigned bpk;                    // points: blocks of one (deformable group, tap)
@@ -510,17 +510,21 @@ exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
         return;
     }
     b -= a.nw;
-    constexpr int W = 16 / (int)sizeof(T);                             // dX scratch, or y
-    const size_t whole = (reinterpret_cast<uintptr_t>(a.zero) & 15) == 0 ? a.zero_n / W : 0;
+    constexpr int W = 16 / (int)sizeof(T);                             // dX scratch, or y; dOffset
+    const bool second = b >= a.nz;
+    T* z = second ? a.zero2 : a.zero;
+    const size_t len = second ? a.zero2_n : a.zero_n;
+    if (second) b -= a.nz;
+    const size_t whole = (reinterpret_cast<uintptr_t>(z) & 15) == 0 ? len / W : 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const size_t e = ((size_t)b * 4 + i) * kXThreads + threadIdx.x;
         if (e < whole) {
-            reinterpret_cast<uint4*>(a.zero)[e] = make_uint4(0u, 0u, 0u, 0u);
+            reinterpret_cast<uint4*>(z)[e] = make_uint4(0u, 0u, 0u, 0u);
         } else {
 #pragma unroll
             for (int k = 0; k < W; ++k)
-                if (e * W + k < a.zero_n) a.zero[e * W + k] = (T)0;
+                if (e * W + k < len) z[e * W + k] = (T)0;
         }
     }
 }
@@ -1319,7 +1323,8 @@ int launch_prep(const Geom& g, const ExactGeom& x, PrepArgs<T> a, cudaStream_t s
         a.nw = (unsigned)((n + 4 * kXThreads - 1) / (4 * kXThreads));
     }
     if (a.zero != nullptr) a.nz = (unsigned)((a.zero_n * sizeof(T) + 64 * kXThreads - 1) / (64 * kXThreads));
-    const unsigned blocks = a.nb + a.nx + a.np + a.nw + a.nz;
+    const unsigned nz2 = a.zero2 != nullptr ? (unsigned)((a.zero2_n * sizeof(T) + 64 * kXThreads - 1) / (64 * kXThreads)) : 0u;
+    const unsigned blocks = a.nb + a.nx + a.np + a.nw + a.nz + nz2;
     if (blocks == 0) return 0;
     return launch_dependent(exact_prep_kernel<T, D>, dim3(blocks), dim3(kXThreads), 0, st, g, x, a) == cudaSuccess ? 0 : -5;
 }
@@ -1411,13 +1416,15 @@ int run_backward(const Geom& g, const ExactGeom& x, int pass, int add, const voi
     a.wk = data ? (T*)(ws + l.wk) : nullptr;
     a.zero = dx != nullptr ? (T*)(ws + l.dxcl) : nullptr;
     a.zero_n = (size_t)g.N * g.iv * x.C4;
+    // a 64-row tile of the data kernel holds whole segments: its offset sums are the offset gradient, else parts of it
+    const int plain = x.S4 <= 64 && 64 % x.S4 == 0 && !x.split;
+    if (DEFORM && doff != nullptr && !plain) {
+        a.zero2 = (T*)doff;
+        a.zero2_n = (size_t)g.N * g.dg * g.kv * D * g.ov;
+    }
     int r = launch_prep<T, D>(g, x, a, st);
     if (r != 0) return r;
     if (data) {
-        const int plain = x.S4 <= 64 && 64 % x.S4 == 0 && !x.split;
-        if (DEFORM && doff != nullptr && !plain &&
-            cudaMemsetAsync(doff, 0, (size_t)g.N * g.dg * g.kv * D * g.ov * sizeof(T), st) != cudaSuccess)
-            return -5;
         constexpr int BN = 16 * kDataTn<T, V>;
         const dim3 grid((unsigned)((g.P + BN - 1) / BN), (unsigned)(g.G * (x.Kp64 / 64)));
         if (launch_dependent(exact_data_kernel<T, D, DEFORM, V>, grid, dim3(kXThreads), 0, st, g, x, a.xcl, a.pts, a.wk,
