@@ -38,7 +38,7 @@ struct ExactGeom {
     int Kp, Kp16, Kp64;              // kv * Cg4, and rounded up to the tile depths
     int Og4;
     int split;                       // a deformable group spans several convolution groups
-    FastDiv d_Cg4, d_S4, d_S, d_Og4, d_C4, d_Kp64;
+    FastDiv d_Cg4, d_S4, d_Og4, d_Kp64;
 };
 
 template <typename T, int V>
@@ -1219,7 +1219,7 @@ ExactGeom exact_geom(const Geom& g, int dtype) {
     x.Kp16 = (x.Kp + 15) / 16 * 16;
     x.Kp64 = (x.Kp + 63) / 64 * 64;
     x.Og4 = (g.Og + 3) / 4 * 4;
-    x.d_Cg4.init(x.Cg4); x.d_S4.init(x.S4); x.d_S.init(x.S); x.d_Og4.init(x.Og4); x.d_C4.init(x.C4); x.d_Kp64.init(x.Kp64);
+    x.d_Cg4.init(x.Cg4); x.d_S4.init(x.S4); x.d_Og4.init(x.Og4); x.d_Kp64.init(x.Kp64);
     return x;
 }
 
