@@ -10,7 +10,8 @@
 //   wt  [G][Og][K']             (backward) weight in the same order, k' fastest
 // so that one corner costs one 16-byte load (or one 16-byte reduction) per four channels, and three FFMA kernels with
 // 16-deep double-buffered operand tiles do the rest:
-//   exact_forward_kernel   y[o, P]      = sum_k' w2[k', o] * sample(k', P)
+//   exact_forward_kernel   y[o, P]      = sum_k' w2[k', o] * sample(k', P), parts of the K range where tiles alone leave SMs
+//                                         idle, added in part order by the last of a tile to finish: reproducible
 //   exact_data_kernel      col[k', P]   = sum_o  wt[o, k'] * dy[o, P], consumed from registers: reductions into a
 //                                         channels-last dX, corner dot products for dOffset
 //   exact_weight_kernel    dW[o, k']    = sum_P  dy[o, P] * sample(k', P), position range split over CTAs, one slice of
@@ -351,6 +352,7 @@ struct Acc {
             for (int q = 0; q < C; ++q) v[i][q] += a[i] * b[q];
     }
     __device__ __forceinline__ T at(int i, int q) const { return v[i][q]; }
+    __device__ __forceinline__ void add(int i, int q, T a) { v[i][q] += a; }
 };
 template <int R, int C>
 struct Acc<float, R, C> {
@@ -378,6 +380,11 @@ struct Acc<float, R, C> {
         asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v[i / 2][q]));
         return (i & 1) ? hi : lo;
     }
+    __device__ __forceinline__ void add(int i, int q, float a) {
+        float lo, hi;
+        unpack2(v[i / 2][q], lo, hi);
+        v[i / 2][q] = (i & 1) ? pack2(lo, hi + a) : pack2(lo + a, hi);
+    }
 };
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -389,7 +396,7 @@ constexpr int kCopyTile = sizeof(T) == 4 ? 64 : 32;      // side of a transpose 
 template <typename T>
 struct PrepArgs {
     const T *x, *off, *w, *dy;
-    T *xcl, *wk, *zero, *zero2, *dbias;      // wk: w2 (forward) or wt (backward)
+    T *xcl, *wk, *zero, *zero2, *dbias;      // wk: w2 (forward) or wt (backward); zero: dX scratch, or the tiles' counters
     Entry<T>* pts;
     size_t zero_n, zero2_n;          // elements
     unsigned nb, nx, np, nw, nz;     // blocks of each part
@@ -510,7 +517,7 @@ exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
         return;
     }
     b -= a.nw;
-    constexpr int W = 16 / (int)sizeof(T);                             // dX scratch, or y; dOffset
+    constexpr int W = 16 / (int)sizeof(T);                             // dX scratch, or counters; dOffset
     const bool second = b >= a.nz;
     T* z = second ? a.zero2 : a.zero;
     const size_t len = second ? a.zero2_n : a.zero_n;
@@ -565,12 +572,58 @@ __device__ __forceinline__ void tile_step(Acc<T, TM, TN>& acc, const T* arow, co
     acc.fma(a, b);
 }
 
+// Parts of the K range (grid.z > 1): each stores its sums in a slice of its own, and the CTA that finishes a tile last --
+// `done` counts them; nobody waits -- adds the slices in part order and stores y.  Every output is thus written once and
+// has one order of summation; reductions into a zeroed y gave the last bits to whichever part came first.
+// A thread reads back what the same thread of the other parts stored, 16 bytes per lane and slice vector.  Costs 1.5 us of
+// a step against the reductions (6 x 96 -> 96 channels 33x45, four parts: 187.5 -> 189.0 us; plain 8 x 64 -> 128, 56x56
+// stride 2, three parts: 99.6 -> 101.3): a tile's slices pass through the one SM that finishes it.
+template <typename T, int TM, int TN, int NT>
+__device__ __forceinline__ bool fold_parts(Acc<T, TM, TN>& acc, T* slices, unsigned* done, char* smem) {
+    constexpr int W = 16 / (int)sizeof(T), E = TM * TN / W;            // 16-byte vectors of a thread
+    static_assert(TN % W == 0, "a vector lies within one row of the register tile");
+    const int tid = threadIdx.x;
+    const size_t tile = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+    T* all = slices + tile * gridDim.z * (TM * TN * NT) + tid * W;
+    T* mine = all + (size_t)blockIdx.z * (TM * TN * NT);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        T t[W];
+#pragma unroll
+        for (int k = 0; k < W; ++k) t[k] = acc.at(e * W / TN, e * W % TN + k);
+        uint4 q;
+        memcpy(&q, t, 16);
+        __stcg(reinterpret_cast<uint4*>(mine + e * (NT * W)), q);
+    }
+    __threadfence();                                                   // the slice is visible before it is counted
+    __syncthreads();                                                   // (also: the operand tiles are done with)
+    if (tid == 0) *reinterpret_cast<unsigned*>(smem) = atomicAdd(done + tile, 1u);
+    __syncthreads();
+    if (*reinterpret_cast<volatile unsigned*>(smem) + 1 != gridDim.z) return false;
+    __threadfence();
+    acc.clear();
+#pragma unroll 2
+    for (unsigned z = 0; z < gridDim.z; ++z, all += TM * TN * NT) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const uint4 q = __ldcg(reinterpret_cast<const uint4*>(all + e * (NT * W)));
+            T t[W];
+            memcpy(t, &q, 16);
+#pragma unroll
+            for (int k = 0; k < W; ++k) acc.add(e * W / TN, e * W % TN + k, t[k]);
+        }
+    }
+    return true;
+}
+
 // grid.x: tiles of 16 * TN positions; grid.y: G * ceil(Og / BM); grid.z: parts of the K range (more than one where the
-// tiles alone leave SMs idle; the parts are added into a y that the prologue has zeroed).
-template <typename T, int D, bool DEFORM, int V, int TM, int TN, int TY>
+// tiles alone leave SMs idle).  slices, done: see fold_parts; `done` is zeroed by the prologue.
+// SPLIT is a kernel of its own: with the fold's registers in the whole-tile one a step of config 4 took 2495 us, not 2408.
+template <typename T, int D, bool DEFORM, int V, int TM, int TN, int TY, bool SPLIT>
 __global__ void __launch_bounds__(16 * TY, kCtasPerSm<T, TN, TY>)
 exact_forward_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl, const Entry<T>* __restrict__ pts,
-                     const T* __restrict__ w2, const T* __restrict__ bias, T* __restrict__ y, int chunks_per_part) {
+                     const T* __restrict__ w2, const T* __restrict__ bias, T* __restrict__ y, int chunks_per_part,
+                     T* __restrict__ slices, unsigned* __restrict__ done) {
     constexpr int BM = TM * TY, BN = 16 * TN, NT = 16 * TY;
     constexpr int Q = kBK / V, ALL = BN * Q, ITEMS = (ALL + NT - 1) / NT, L16 = 16 / (int)sizeof(T);
     extern __shared__ __align__(16) char smem_x[];
@@ -710,9 +763,11 @@ exact_forward_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl
         }
     }
 
-    const bool split = gridDim.z > 1;
+    if constexpr (SPLIT) {
+        if (!fold_parts<T, TM, TN, NT>(acc, slices, done, smem_x)) return;
+    }
     // four positions of one sample, 16-byte aligned
-    const bool vec = sizeof(T) == 4 && !split && g.ov % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+    const bool vec = sizeof(T) == 4 && g.ov % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
 #pragma unroll
     for (int h = 0; h < TN / 4; ++h) {
         const long long P = P0 + tile_col(tx, h);
@@ -724,7 +779,7 @@ exact_forward_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl
             const int ol = o0 + ty * TM + i;
             if (ol >= g.Og) break;
             const int o = j * g.Og + ol;
-            const T bv = bias != nullptr && blockIdx.z == 0 ? __ldg(bias + o) : (T)0;
+            const T bv = bias != nullptr ? __ldg(bias + o) : (T)0;
             if (vec) {
                 *reinterpret_cast<float4*>(y + ((size_t)n * g.O + o) * g.ov + opos) =
                     make_float4((float)(acc.at(i, 4 * h) + bv), (float)(acc.at(i, 4 * h + 1) + bv),
@@ -736,9 +791,7 @@ exact_forward_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl
                 if (P + t >= g.P) break;
                 uint32_t nt, ot;
                 g.d_ov.divmod((uint32_t)(P + t), nt, ot);
-                T* dst = y + ((size_t)nt * g.O + o) * g.ov + ot;
-                if (split) atomicAdd(dst, acc.at(i, 4 * h + t) + bv);
-                else *dst = acc.at(i, 4 * h + t) + bv;
+                y[((size_t)nt * g.O + o) * g.ov + ot] = acc.at(i, 4 * h + t) + bv;
             }
         }
     }
@@ -1286,7 +1339,7 @@ int forward_parts(const Geom& g, const ExactGeom& x, int dtype, int& per) {
 }
 
 struct ExactLayout {
-    size_t xcl, wk, pts, dxcl, dwp, total;
+    size_t xcl, wk, pts, dxcl, dwp, slices, done, done_n, total;     // done_n: counters
 };
 ExactLayout exact_layout(const Geom& g, const ExactGeom& x, int dtype, int deform, int pass) {
     const size_t es = dtype == 1 ? 8 : 4;
@@ -1295,7 +1348,18 @@ ExactLayout exact_layout(const Geom& g, const ExactGeom& x, int dtype, int defor
     l.xcl = at; at += up256((size_t)g.N * g.iv * x.C4 * es);
     l.wk = at; at += up256((size_t)g.G * (pass == 0 ? (size_t)x.Kp16 * x.Og4 : (size_t)g.Og * x.Kp64) * es);
     l.pts = at; at += deform ? up256((size_t)g.dg * g.kv * g.P * (dtype == 1 ? sizeof(Entry<double>) : sizeof(Entry<float>))) : 0;
-    l.dxcl = at; l.dwp = at;
+    l.dxcl = at; l.dwp = at; l.slices = at; l.done = at; l.done_n = 0;
+    if (pass == 0) {
+        int per;
+        const int parts = forward_parts(g, x, dtype, per);
+        if (parts > 1) {             // no more CTAs than run at once: at most 14 MB
+            const ExactTiles t = exact_tiles(g, x, dtype);
+            l.done_n = (size_t)((g.P + t.bn - 1) / t.bn) * g.G * t.mt;
+            at += up256(l.done_n * parts * (size_t)(t.tm * t.ty) * t.bn * es);
+            l.done = at;
+            at += up256(l.done_n * sizeof(unsigned));
+        }
+    }
     if (pass == 1 || pass == 3) { l.dxcl = at; at += up256((size_t)g.N * g.iv * x.C4 * es); }
     if (pass == 2 || pass == 3) {
         int per;
@@ -1336,11 +1400,13 @@ bool allow_smem(K kernel, int bytes) {
 
 template <typename T, int D, bool DEFORM, int V, int TM, int TN, int TY>
 int launch_forward(const Geom& g, const ExactGeom& x, dim3 grid, const T* xcl, const Entry<T>* pts, const T* w2,
-                   const T* bias, T* y, int per, cudaStream_t st) {
-    auto kernel = exact_forward_kernel<T, D, DEFORM, V, TM, TN, TY>;
+                   const T* bias, T* y, int per, T* slices, unsigned* done, cudaStream_t st) {
+    auto kernel = grid.z > 1 ? exact_forward_kernel<T, D, DEFORM, V, TM, TN, TY, true>
+                             : exact_forward_kernel<T, D, DEFORM, V, TM, TN, TY, false>;
     const int smem = 2 * kBK * (TM * TY + 16 * TN) * (int)sizeof(T) + Sampler<T, D, DEFORM, V, 16 * TY>::kBytes;
     if (!allow_smem(kernel, smem)) return -5;
-    return launch_dependent(kernel, grid, dim3(16 * TY), smem, st, g, x, xcl, pts, w2, bias, y, per) == cudaSuccess ? 0 : -5;
+    return launch_dependent(kernel, grid, dim3(16 * TY), smem, st, g, x, xcl, pts, w2, bias, y, per, slices, done) == cudaSuccess
+               ? 0 : -5;
 }
 
 template <typename T, int D, bool DEFORM, int V, int TM, int TN, int TY>
@@ -1369,8 +1435,8 @@ int launch_weight(const Geom& g, const ExactGeom& x, dim3 grid, const T* xcl, co
 
 template <typename T, int D, bool DEFORM, int V>
 int pick_forward(const ExactTiles& t, const Geom& g, const ExactGeom& x, dim3 grid, const T* xcl, const Entry<T>* pts,
-                 const T* w2, const T* bias, T* y, int per, cudaStream_t st) {
-    DCN_EXACT_TILE(launch_forward, g, x, grid, xcl, pts, w2, bias, y, per, st);
+                 const T* w2, const T* bias, T* y, int per, T* slices, unsigned* done, cudaStream_t st) {
+    DCN_EXACT_TILE(launch_forward, g, x, grid, xcl, pts, w2, bias, y, per, slices, done, st);
 }
 template <typename T, int D, bool DEFORM, int V>
 int pick_weight(const ExactTiles& t, const Geom& g, const ExactGeom& x, dim3 grid, const T* xcl, const Entry<T>* pts,
@@ -1390,14 +1456,15 @@ int run_forward(const Geom& g, const ExactGeom& x, const void* x_in, const void*
     int per;
     const int parts = forward_parts(g, x, dtype, per);
     if (parts > 1) {
-        a.zero = (T*)y;
-        a.zero_n = (size_t)g.N * g.O * g.ov;
+        a.zero = (T*)(ws + l.done);
+        a.zero_n = (l.done_n * sizeof(unsigned) + sizeof(T) - 1) / sizeof(T);
     }
     const int r = launch_prep<T, D>(g, x, a, st);
     if (r != 0) return r;
     const ExactTiles t = exact_tiles(g, x, dtype);
     const dim3 grid((unsigned)((g.P + t.bn - 1) / t.bn), (unsigned)(g.G * t.mt), (unsigned)parts);
-    return pick_forward<T, D, DEFORM, V>(t, g, x, grid, a.xcl, a.pts, a.wk, (const T*)bias, (T*)y, per, st);
+    return pick_forward<T, D, DEFORM, V>(t, g, x, grid, a.xcl, a.pts, a.wk, (const T*)bias, (T*)y, per, (T*)(ws + l.slices),
+                                         (unsigned*)(ws + l.done), st);
 }
 
 // pass 1: backward data, 2: backward weight, 3: both.  add: dX and dW accumulate (else they are overwritten).

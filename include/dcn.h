@@ -106,7 +106,8 @@ size_t dcn_workspace_bytes(const dcn_problem* p, int pass);
 int dcn_launch_count(const dcn_problem* p, int pass);
 
 /* y = conv(x sampled at offset, weight) + bias.  `offset` may be NULL when deformable == 0, `bias` may
- * be NULL.  y is overwritten.  Replaces deform_conv_forward_cuda (deform3d/lib/deform_conv3d_cuda.cpp:90-165)
+ * be NULL.  y is overwritten; precision EXACT gives the same bits on every call with the same arguments.
+ * Replaces deform_conv_forward_cuda (deform3d/lib/deform_conv3d_cuda.cpp:90-165)
  * and the Python-side bias add (deform3d/deform_conv3d_functions/deform_conv3d_function.py:41-42). */
 int dcn_forward(const dcn_problem* p, const void* x, const void* offset, const void* weight, const void* bias,
                 void* y, void* workspace, size_t workspace_bytes, void* stream);
