@@ -193,7 +193,6 @@ int dcn_forward_static_scratch(const dcn_problem* p, const void* x, const void* 
     Geom g;
     make_geom(p, g);
     if (!dcn::tc_supported(g, p->ndim, p->deformable)) return DCN_ERR_UNSUPPORTED;
-    if (dcn::tc_workspace_bytes(g, p->ndim, DCN_PASS_FORWARD) > dcn::tc_static_scratch_bytes()) return DCN_ERR_LIMIT;
     return dcn::tc_forward_static(g, p->ndim, p->deformable, (const float*)x, (const float*)offset,
                                   (const float*)weight, (const float*)bias, (float*)y,
                                   static_cast<cudaStream_t>(stream));

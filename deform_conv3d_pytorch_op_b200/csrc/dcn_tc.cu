@@ -111,14 +111,18 @@ int sm_count() {
 #include "dcn_tc_fwd.cuh"
 
 struct FwdWorkspace {
-    size_t xcl_off, wpk_off, total;
+    size_t xcl_off, wpk_off, slices_off, total;       // slices: partial sums of split tiles
+    FwdSplit split;
 };
-FwdWorkspace fwd_workspace(const Geom& g) {
+// have: bytes there are at most
+FwdWorkspace fwd_workspace(const Geom& g, size_t have = SIZE_MAX) {
     const TcDims d = tc_dims(g);
     FwdWorkspace w;
     w.xcl_off = 0;
     w.wpk_off = align_up((size_t)g.N * g.iv * g.C * 2, 256);
-    w.total = w.wpk_off + align_up((size_t)g.G * d.MT * d.KC * kTileBytes, 256);
+    w.slices_off = w.wpk_off + align_up((size_t)g.G * d.MT * d.KC * kTileBytes, 256);
+    w.split = fwd_split(g, have > w.slices_off ? have - w.slices_off : 0);
+    w.total = w.slices_off + align_up((size_t)fwd_slices(w.split) * fwd_slice_bytes(g), 256);
     return w;
 }
 
@@ -230,6 +234,7 @@ struct Backward {
     bool b2, gather, scatter, tiles, bias_here;
     Geom gt, gk;                         // transposed convolution; with the layout of dX
     FwdPlan plan;                        // of the gather
+    FwdWorkspace f;
 
     Backward(const Geom& g_, int ndim_, int deform_, bool add_, const float* off_, const float* w_, const float* dy_, float* dx_,
              float* doff_, float* dw_, float* dbias_, void* ws)
@@ -266,19 +271,18 @@ struct Backward {
         }
         if (doff != nullptr) p.zero(doff, (size_t)g.N * g.dg * g.kv * ndim * g.ov);
         if (gather) {
-            const FwdWorkspace f = fwd_workspace(gt);
+            f = fwd_workspace(gt);
             gk = gt;
             gk.cl = dx_cl ? 1 : 0;
-            plan = fwd_plan(gk, ndim, 0, dx, dx_partial);
+            plan = fwd_plan(gk, f.split, ndim, 0, dx, dx_partial);
             if (plan.direct && dx_partial) return -5;
             p.weight(g, kTilesFlip, w, base + l.gath_off + f.wpk_off);
-            add_zeros(p, plan);
         }
         return 0;
     }
     void with_dy(Passes& p) {
         if (tiles) p.pack_dy(g, dy, base + l.dpk_off, d.MT, d.PC2, b2 ? scale() : nullptr, sums());
-        if (gather) p.copy_x(gt, dy, reinterpret_cast<__nv_bfloat16*>(base + l.gath_off + fwd_workspace(gt).xcl_off));
+        if (gather) p.copy_x(gt, dy, reinterpret_cast<__nv_bfloat16*>(base + l.gath_off + f.xcl_off));
     }
     int run(cudaStream_t st) {
         int r = 0;
@@ -292,11 +296,9 @@ struct Backward {
             else r = deform ? launch_tc_dgrad<3, true>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, scale(), st)
                             : launch_tc_dgrad<3, false>(g, xcl, off, dpk, base + l.wpk_off, dxcl(), doff, scale(), st);
         }
-        if (r == 0 && gather) {
-            const FwdWorkspace f = fwd_workspace(gt);
+        if (r == 0 && gather)            // (a split one is folded behind it, by fold_dx)
             r = launch_tc_forward(gk, plan, ndim, 0, reinterpret_cast<const __nv_bfloat16*>(base + l.gath_off + f.xcl_off), nullptr,
-                                  base + l.gath_off + f.wpk_off, nullptr, dx, st);
-        }
+                                  base + l.gath_off + f.wpk_off, nullptr, dx, slices(), st);
         if (r == 0 && dw != nullptr) {   // the weight kernel reads dy tiles with the same layout and stride (PC2 == wg_dims().PC)
             float* dwpk = reinterpret_cast<float*>(base + l.dwpk_off);
             if (ndim == 2) r = deform ? launch_tc_wgrad<2, true>(g, xcl, off, dpk, dwpk, st)
@@ -306,8 +308,11 @@ struct Backward {
         }
         return r;
     }
-    bool folds_dx() const { return scatter && dx != nullptr && !dx_cl; }
-    void fold_dx(Passes& p) const { if (folds_dx()) p.fold_dx(g, dxcl(), dx, dx_partial); }
+    float* slices() const { return reinterpret_cast<float*>(base + l.gath_off + f.slices_off); }
+    void fold_dx(Passes& p) const {
+        if (scatter && dx != nullptr && !dx_cl) p.fold_dx(g, dxcl(), dx, dx_partial);
+        if (gather && plan.folds()) p.fold_y(gk, y_fold(gk, plan, slices(), nullptr, dx));
+    }
     void epilogue(Passes& p) const {
         if (dw != nullptr) add_dw_fold(p, g, reinterpret_cast<const float*>(base + l.dwpk_off), dw, add);
         if (bias_here) p.fold_bias(g, sums(), dbias, d.MT, d.PC2);
@@ -336,12 +341,14 @@ int tc_launch_count(const Geom& g, int ndim, int deform, int pass) {
     const bool b2 = use_bwd2d(g, ndim, deform);
     Geom gt;
     const bool gather = use_gather_dgrad(g, ndim, deform, gt);
-    if (pass == 0) return 2;                               // prologue, implicit GEMM
-    if (pass == 1) return b2 || gather || g.cl ? 2 : 3;    // prologue, GEMM + scatter (or gather), (dX transpose)
+    auto folds = [&](const Geom& f, int df) { return fwd_plan(f, fwd_workspace(f).split, ndim, df, nullptr, false).folds() ? 1 : 0; };
+    if (pass == 0) return 2 + folds(g, deform);            // prologue, implicit GEMM, (fold of the split tiles)
+    if (pass == 1 && gather) return 2 + folds(gt, 0);
+    if (pass == 1) return b2 || g.cl ? 2 : 3;              // prologue, GEMM + scatter, (dX transpose)
     if (pass == 2) return 3;                               // prologue, implicit GEMM, dW fold
     // fused backward without the forward pass's workspace: the jobs of the prologue one by one, two GEMMs, epilogue
     if (b2) return 8;                                      // points, slab tiles, zero fill, dy pack, input copy
-    if (gather) return 7 + fwd_plan(gt, ndim, 0, nullptr, false).zeros;   // mirrored tiles, (zero fill,) dy pack, dy copy, input copy
+    // (gather: mirrored tiles, dy pack, dy copy, input copy)
     return 7;                                              // weight tiles, zero fill, dy pack, input copy
 }
 
@@ -364,19 +371,19 @@ int tc_debug_points(const Geom& g, int ndim, int deform, const float* off, int n
 
 int tc_forward(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
                const float* bias, float* y, void* ws, size_t ws_bytes, cudaStream_t st) {
-    const FwdWorkspace l = fwd_workspace(g);
+    const FwdWorkspace l = fwd_workspace(g, ws_bytes);
     if (ws_bytes < l.total) return -4;
     uint8_t* base = static_cast<uint8_t*>(ws);
     __nv_bfloat16* xcl = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
     uint8_t* wpk = base + l.wpk_off;
-    const FwdPlan plan = fwd_plan(g, ndim, deform, y, false);
+    const FwdPlan plan = fwd_plan(g, l.split, ndim, deform, y, false);
+    float* slices = reinterpret_cast<float*>(base + l.slices_off);
     Passes p;
     p.copy_x(g, x, xcl);
     p.weight(g, kTilesFwd, w, wpk);
-    add_zeros(p, plan);
-    const int r = p.launch(st, false);
-    if (r != 0) return r;
-    return launch_tc_forward(g, plan, ndim, deform, xcl, off, wpk, bias, y, st);
+    int r = p.launch(st, false);
+    if (r == 0) r = launch_tc_forward(g, plan, ndim, deform, xcl, off, wpk, bias, y, slices, st);
+    return r != 0 ? r : launch_y_fold(g, plan, slices, bias, y, true, st);
 }
 
 int tc_backward_data(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
@@ -468,30 +475,29 @@ static size_t layer_doff_bytes(const Geom& g, int ndim) {
 }
 
 size_t tc_layer_workspace_bytes(const Geom& g, const Geom& gq, int ndim, int pass) {
-    if (pass == 0) return fwd_workspace(g).total + align_up(fwd_workspace(gq).total, 256);
+    if (pass == 0) return fwd_workspace(g).total + fwd_workspace(gq).total;
     return layer_doff_bytes(g, ndim) + align_up(bwd_data_workspace(g).total, 256) + align_up(bwd_data_workspace(gq).total, 256);
 }
 
 int tc_layer_forward(const Geom& g, const Geom& gq, int ndim, const float* x, const float* w_off, const float* b_off,
                      const float* w, const float* bias, float* offsets, float* y, void* ws, size_t ws_bytes,
                      cudaStream_t st) {
-    if (ws_bytes < tc_layer_workspace_bytes(g, gq, ndim, 0)) return -4;
     const FwdWorkspace l = fwd_workspace(g), lq = fwd_workspace(gq);
+    if (ws_bytes < l.total + lq.total) return -4;
     uint8_t* base = static_cast<uint8_t*>(ws);
-    uint8_t* baseq = base + align_up(l.total, 256);
+    uint8_t* baseq = base + l.total;
+    float *slices = reinterpret_cast<float*>(base + l.slices_off), *slicesq = reinterpret_cast<float*>(baseq + lq.slices_off);
     __nv_bfloat16* xcl = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
-    const FwdPlan pq = fwd_plan(gq, ndim, 0, offsets, false), pl = fwd_plan(g, ndim, 1, y, false);
+    const FwdPlan pq = fwd_plan(gq, lq.split, ndim, 0, offsets, false), pl = fwd_plan(g, l.split, ndim, 1, y, false);
     Passes p;
     p.copy_x(g, x, xcl);
     p.weight(gq, kTilesFwd, w_off, baseq + lq.wpk_off);
     p.weight(g, kTilesFwd, w, base + l.wpk_off);
-    add_zeros(p, pq);
-    add_zeros(p, pl);
     int r = p.launch(st, false);
-    if (r != 0) return r;
-    r = launch_tc_forward(gq, pq, ndim, 0, xcl, nullptr, baseq + lq.wpk_off, b_off, offsets, st);
-    if (r != 0) return r;
-    return launch_tc_forward(g, pl, ndim, 1, xcl, offsets, base + l.wpk_off, bias, y, st);
+    if (r == 0) r = launch_tc_forward(gq, pq, ndim, 0, xcl, nullptr, baseq + lq.wpk_off, b_off, offsets, slicesq, st);
+    if (r == 0) r = launch_y_fold(gq, pq, slicesq, b_off, offsets, false, st);
+    if (r == 0) r = launch_tc_forward(g, pl, ndim, 1, xcl, offsets, base + l.wpk_off, bias, y, slices, st);
+    return r != 0 ? r : launch_y_fold(g, pl, slices, bias, y, true, st);
 }
 
 int tc_layer_backward(const Geom& g, const Geom& gq, int ndim, const float* x, const float* offsets, const float* w_off,
@@ -560,7 +566,7 @@ int tc_forward_static(const Geom& g, int ndim, int deform, const float* x, const
                       const float* bias, float* y, cudaStream_t st) {
     constexpr int kMaxDevices = 64;
     static void* volatile scratch_of_device[kMaxDevices] = {};
-    if (fwd_workspace(g).total > kStaticScratchBytes) return -8;
+    if (fwd_workspace(g, 0).total > kStaticScratchBytes) return -8;      // (without room for a split)
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess) return -5;
     if (dev < 0 || dev >= kMaxDevices) return -8;

@@ -36,27 +36,28 @@ struct FwdCtl {            // lives behind the stages, the tables and the offset
 // How the work items of the persistent CTAs map to (tile, K range).  Items [0, T0) split every tile KS0 ways
 // (KS0 = 1: whole tiles); items from T0 on split the tiles from tile1 on KS1 ways.  The second region is the
 // tail of a grid that does not divide evenly: the tiles left over after the last full wave are split along K so
-// that the last wave is a fraction of a tile long instead of a whole one.  Split tiles add into a zero-filled y.
+// that the last wave is a fraction of a tile long instead of a whole one.
+// The items of split tiles store their sums in a slice of scratch each (item order); a fold behind the kernel adds
+// the slices of a tile in K order and stores y (fold_y, dcn_tc_passes.cuh).
 struct FwdSplit {
     long long T0, tile1, n_items;
     int KS0, cpk0, KS1, cpk1;
-    int acc;            // y already holds a partial result: every tile is added to it with reductions
+    int acc;            // y already holds a partial result, which the tiles are added to (plain convolution only)
 };
 struct FwdItem {
     long long tt;       // tile index ((j * MB + mb) * PT + pt)
-    int ks, kc0, kc1;   // split number and its K chunks [kc0, kc1)
-    bool atomic;        // partial sum of a split tile
+    long long slice;    // of a split tile: where its sums go; else -1
+    int kc0, kc1;       // its K chunks [kc0, kc1)
 };
 __device__ __forceinline__ FwdItem fwd_item(const FwdSplit& sp, long long t, int KC) {
     const bool tail = t >= sp.T0;
     const long long r = tail ? t - sp.T0 : t;
     const int KS = tail ? sp.KS1 : sp.KS0, cpk = tail ? sp.cpk1 : sp.cpk0;
     FwdItem it;
-    it.ks = (int)(r % KS);
     it.tt = (tail ? sp.tile1 : 0) + r / KS;
-    it.kc0 = it.ks * cpk;
+    it.slice = KS > 1 ? r : -1;
+    it.kc0 = (int)(r % KS) * cpk;
     it.kc1 = (it.kc0 + cpk < KC) ? it.kc0 + cpk : KC;
-    it.atomic = KS > 1 || sp.acc != 0;
     return it;
 }
 
@@ -66,7 +67,7 @@ __global__ void __launch_bounds__(fwd_threads(GW), 1)
 tc_forward_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float* __restrict__ off,
                   const uint8_t* __restrict__ wpk, const float* __restrict__ bias, float* __restrict__ y,
                   const int KC, const int MT, const int MB, const long long PT, const int n_stages,
-                  const int max_slots, const int n_tabs, const FwdSplit sp) {
+                  const int max_slots, const int n_tabs, const FwdSplit sp, float* __restrict__ slices) {
     // Work items: see FwdSplit.  With few position tiles and a long K every tile is split (small batches, late
     // layers of a network); otherwise only the tiles of the last, partial wave are.
     using Entry = TabEntry<D, DEFORM>;
@@ -256,18 +257,31 @@ tc_forward_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const flo
                 tc_fence_after();
                 const uint32_t b = etl & 1;
                 const FwdItem wi = fwd_item(sp, et, KC);
-                const int ks = wi.ks;
-                const bool plain = !wi.atomic;
+                const bool plain = DEFORM || sp.acc == 0;
                 const long long tt = wi.tt;
                 const long long pt = tt % PT;
                 const int mb = (int)((tt / PT) % MB);
                 const int j = (int)(tt / PT / MB);
                 const int mtb = (MT - mb * 2) >= 2 ? 2 : 1;
+                if (wi.slice >= 0) {
+                    float* s = slices + (size_t)wi.slice * ((MT >= 2 ? 2 : 1) * kSliceHalf) + q * (kSliceHalf / 4) + lane * 4;
+#pragma unroll 1
+                    for (int c = 0; c < mtb * (kTileN / 16); ++c) {
+                        const int mt = c / (kTileN / 16), cc = c % (kTileN / 16);
+                        uint32_t v[16];
+                        tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + b * 256 + mt * 128 + cc * 16, v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            *reinterpret_cast<uint4*>(s + (size_t)mt * kSliceHalf + cc * kSliceGroup + i * 128) =
+                                make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    }
+                } else
                 for (int mt = 0; mt < mtb; ++mt) {
                     const int ol = (mb * 2 + mt) * 128 + q * 32 + lane;      // output channel within the group
                     const bool o_ok = ol < g.Og;
                     const int o = j * g.Og + ol;
-                    const float bv = (bias != nullptr && o_ok && ks == 0) ? __ldg(bias + o) : 0.f;
+                    const float bv = (bias != nullptr && o_ok) ? __ldg(bias + o) : 0.f;
                     if constexpr (TURN) {
                         // Channel-first y whose rows are not 16-byte aligned: 32 x 32 pieces are turned in shared memory
                         // and leave as 128-byte runs along the positions.  (A lane storing its own row of an odd size
@@ -560,21 +574,72 @@ inline int max_slots_per_chunk(const Geom& g, int cols_per_chunk) {
     return best;
 }
 
-// How a forward pass runs: stages, work split and what of y has to be zero before the kernel starts (parts of a split
-// tile are added to it).
+// The tiles' split along K, so that the SMs are busy to the end; both ways are weighed in K chunks of work (0.7 us each), an
+// item costing six beside its own (set-up and epilogue), the fold four, and no item gets under three (B200, 2 x 128 channels
+// 40x41, 26 tiles of 18 chunks, kernel time with reductions at 9 / 6 / 5 / 3 chunks an item: 18.3 / 15.6 / 14.8 / 13.9 us):
+//   every tile into KS0 pieces (few tiles, or a badly filled last wave);
+//   the R tiles left after the last full wave into KS1 pieces, as many as there are SMs to take them.
+// room: bytes there are for slices; a split that needs more is not taken.
+inline size_t fwd_slice_bytes(const Geom& g) { return (size_t)(g.Og > 128 ? 2 : 1) * kSliceHalf * sizeof(float); }
+inline long long fwd_slices(const FwdSplit& sp) { return sp.KS0 > 1 ? sp.T0 : (sp.KS1 > 1 ? sp.n_items - sp.T0 : 0); }
+inline FwdSplit fwd_split(const Geom& g, size_t room) {
+    const TcDims d = tc_dims(g);
+    const long long base_tiles = (long long)g.G * d.MB * d.PT;
+    FwdSplit sp = {};
+    sp.KS0 = sp.KS1 = 1;
+    sp.cpk0 = sp.cpk1 = d.KC;
+    sp.T0 = sp.tile1 = sp.n_items = base_tiles;
+    if (base_tiles >= (1 << 28)) return sp;              // (the fold counts tiles and pieces in 32 bits)
+    const int S = sm_count(), base = (int)base_tiles;
+    const size_t most = room / fwd_slice_bytes(g);
+    auto cost = [&](int items, int chunks) { return (items + S - 1) / S * (long long)(chunks + 6); };
+    auto pieces = [&](int want, int& chunks) {           // of a tile; chunks: of one piece
+        chunks = (d.KC + want - 1) / want;
+        return (d.KC + chunks - 1) / chunks;
+    };
+    long long best = cost(base, d.KC);
+    for (int k = 2; k <= d.KC / 3 && (long long)base * k <= 3ll * S; ++k) {
+        int chunks;
+        const int ks = pieces(k, chunks);
+        const long long c = cost(base * ks, chunks) + 4;
+        if (c * 20 < best * 19 && (size_t)base * ks <= most) { best = c; sp.KS0 = ks; sp.cpk0 = chunks; }
+    }
+    const int R = base % S;
+    int ks1 = 1, cpk1 = d.KC;
+    if (base > S && R != 0) {
+        int want = S / R;
+        if (want > d.KC / 3) want = d.KC / 3;
+        if (want >= 2) {
+            ks1 = pieces(want, cpk1);
+            if ((long long)(base / S) * (d.KC + 6) + cost(R * ks1, cpk1) + 4 < best && (size_t)R * ks1 <= most) {
+                sp.KS0 = 1;
+                sp.cpk0 = d.KC;
+            } else {
+                ks1 = 1;
+            }
+        }
+    }
+    const bool tail = ks1 > 1;
+    sp.T0 = tail ? base_tiles - R : base_tiles * sp.KS0;
+    sp.tile1 = tail ? sp.T0 : base_tiles;
+    sp.KS1 = ks1;
+    sp.cpk1 = tail ? cpk1 : d.KC;
+    sp.n_items = tail ? sp.T0 + R * ks1 : sp.T0;
+    return sp;
+}
+
+// How a forward pass runs: stages and work split.
 struct FwdPlan {
     FwdSplit sp;
     int stages, n_tabs, smem, max_slots, grid;
     int turn;                            // rows of a channel-first y are not 16-byte aligned
     bool direct;                         // the corner table does not fit beside the stages
-    struct { float* p; size_t len; int rows, pitch; } zero[2];
-    int zeros;
+    bool folds() const { return !direct && fwd_slices(sp) > 0; }
 };
 
-// accumulate: add to what y holds (every tile leaves through reductions; the direct variant cannot)
+// accumulate: add to what y holds (the direct variant cannot)
 template <int D, bool DEFORM>
-FwdPlan fwd_plan(const Geom& g, float* y, bool accumulate) {
-    const TcDims d = tc_dims(g);
+FwdPlan fwd_plan(const Geom& g, const FwdSplit& split, const float* y, bool accumulate) {
     FwdPlan pl = {};
     pl.max_slots = max_slots_per_chunk(g, 8);
     pl.turn = !g.cl && (g.ov % 4 != 0 || (reinterpret_cast<uintptr_t>(y) & 15) != 0) ? 1 : 0;
@@ -596,103 +661,54 @@ FwdPlan fwd_plan(const Geom& g, float* y, bool accumulate) {
         return pl;
     }
     pl.smem = (int)need(pl.stages, pl.n_tabs);
-    // Two ways of splitting tiles along K so that the SMs are busy to the end; both are weighed in K chunks of work, an
-    // item costing six beside its own (its sums are added to y), and no item gets under three (B200, 2 x 128 channels 40x41, 26 tiles of 18
-    // chunks, kernel time at 9 / 6 / 5 / 3 chunks an item: 18.3 / 15.6 / 14.8 / 13.9 us):
-    //   every tile into KS0 pieces (few tiles, or a badly filled last wave), all of y zero-filled;
-    //   the R tiles left after the last full wave into KS1 pieces, as many as there are SMs to take them.  They have to
-    //   lie in the last (group, channel block), so that they are a position range [P0, P) of its channels and only that
-    //   part of y is zero-filled.
-    const long long base_tiles = (long long)g.G * d.MB * d.PT;
-    const int S = sm_count();
-    auto waves = [&](long long items) { return (items + S - 1) / S; };
-    auto cost = [&](long long items, int chunks) { return waves(items) * (chunks + 6); };
-    auto pieces = [&](int want, int& chunks) {           // of a tile; chunks: of one piece
-        chunks = (d.KC + want - 1) / want;
-        return (d.KC + chunks - 1) / chunks;
-    };
-    FwdSplit& sp = pl.sp;
-    sp.acc = accumulate ? 1 : 0;
-    sp.KS0 = 1;
-    sp.cpk0 = d.KC;
-    long long best = cost(base_tiles, d.KC);
-    for (int k = 2; k <= d.KC / 3 && base_tiles * k <= 3ll * S; ++k) {
-        int chunks;
-        const int ks = pieces(k, chunks);
-        const long long c = cost(base_tiles * ks, chunks) + 2;       // (the zero fill)
-        if (c * 20 < best * 19) { best = c; sp.KS0 = ks; sp.cpk0 = chunks; }
-    }
-    const long long R = base_tiles % S;
-    const int oA = (g.G - 1) * g.Og + (d.MB - 1) * 256, Ob = g.O - oA;      // channels of the last block
-    int ks1 = 1, cpk1 = d.KC;
-    if (base_tiles > S && R != 0 && R <= d.PT && (long long)g.O * g.ov < (1ll << 31)) {
-        long long want = S / R;
-        if (want > d.KC / 3) want = d.KC / 3;
-        if (want >= 2) {
-            ks1 = pieces((int)want, cpk1);
-            if (base_tiles / S * (d.KC + 6) + cost(R * ks1, cpk1) + 1 < best) {
-                sp.KS0 = 1;
-                sp.cpk0 = d.KC;
-            } else {
-                ks1 = 1;
-            }
-        }
-    }
-    const bool tail = ks1 > 1;
-    sp.T0 = tail ? base_tiles - R : base_tiles * sp.KS0;
-    sp.tile1 = tail ? sp.T0 : base_tiles;
-    sp.KS1 = ks1;
-    sp.cpk1 = tail ? cpk1 : d.KC;
-    sp.n_items = tail ? sp.T0 + R * ks1 : sp.T0;
-    auto zero = [&](float* p, size_t len, int rows, int pitch) {
-        auto& z = pl.zero[pl.zeros++];
-        z.p = p; z.len = len; z.rows = rows; z.pitch = pitch;
-    };
-    if (!accumulate && sp.KS0 > 1) zero(y, (size_t)g.N * g.O * g.ov, 1, 0);
-    if (!accumulate && tail) {
-        const long long P0 = (d.PT - R) * kTileN;
-        if (g.cl) {
-            if (Ob == g.O) zero(y + (size_t)P0 * g.O, (size_t)(g.P - P0) * g.O, 1, 0);
-            else zero(y + (size_t)P0 * g.O + oA, (size_t)Ob, (int)(g.P - P0), g.O);
-        } else {
-            long long n0 = P0 / g.ov;
-            const long long o0 = P0 % g.ov;
-            if (o0 != 0) {      // the sample the tail starts in: the positions [o0, ov) of every channel
-                zero(y + ((size_t)n0 * g.O + oA) * g.ov + o0, (size_t)(g.ov - o0), Ob, g.ov);
-                ++n0;
-            }
-            float* rest = y + ((size_t)n0 * g.O + oA) * g.ov;
-            if (n0 < g.N && Ob == g.O) zero(rest, (size_t)(g.N - n0) * g.O * g.ov, 1, 0);
-            else if (n0 < g.N) zero(rest, (size_t)Ob * g.ov, (int)(g.N - n0), g.O * g.ov);
-        }
-    }
-    pl.grid = (int)(sp.n_items < S ? sp.n_items : S);
+    pl.sp = split;
+    pl.sp.acc = accumulate ? 1 : 0;
+    pl.grid = (int)(pl.sp.n_items < sm_count() ? pl.sp.n_items : sm_count());
     return pl;
 }
 
 template <int D, bool DEFORM>
 int launch_tc_forward(const Geom& g, const FwdPlan& pl, const __nv_bfloat16* xcl, const float* off, const uint8_t* wpk,
-                      const float* bias, float* y, cudaStream_t st) {
+                      const float* bias, float* y, float* slices, cudaStream_t st) {
     if (pl.direct) return launch_tc_forward_direct<D, DEFORM>(g, xcl, off, wpk, bias, y, st);
     const TcDims d = tc_dims(g);
     constexpr int GW = 16;
     auto kern = pl.turn ? tc_forward_kernel<D, DEFORM, GW, true> : tc_forward_kernel<D, DEFORM, GW, false>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem) != cudaSuccess) return -5;
     return launch_dependent(kern, dim3(pl.grid), dim3(fwd_threads(GW)), pl.smem, st, g, xcl, off, wpk, bias, y, d.KC, d.MT, d.MB,
-                            d.PT, pl.stages, pl.max_slots, pl.n_tabs, pl.sp) == cudaSuccess ? 0 : -5;
+                            d.PT, pl.stages, pl.max_slots, pl.n_tabs, pl.sp, slices) == cudaSuccess ? 0 : -5;
 }
 
-inline FwdPlan fwd_plan(const Geom& g, int ndim, int deform, float* y, bool accumulate) {
-    if (ndim == 2) return deform ? fwd_plan<2, true>(g, y, accumulate) : fwd_plan<2, false>(g, y, accumulate);
-    return deform ? fwd_plan<3, true>(g, y, accumulate) : fwd_plan<3, false>(g, y, accumulate);
-}
-inline void add_zeros(Passes& p, const FwdPlan& pl) {
-    for (int i = 0; i < pl.zeros; ++i) p.zero(pl.zero[i].p, pl.zero[i].len, pl.zero[i].rows, pl.zero[i].pitch);
+inline FwdPlan fwd_plan(const Geom& g, const FwdSplit& split, int ndim, int deform, const float* y, bool accumulate) {
+    if (ndim == 2) return deform ? fwd_plan<2, true>(g, split, y, accumulate) : fwd_plan<2, false>(g, split, y, accumulate);
+    return deform ? fwd_plan<3, true>(g, split, y, accumulate) : fwd_plan<3, false>(g, split, y, accumulate);
 }
 inline int launch_tc_forward(const Geom& g, const FwdPlan& pl, int ndim, int deform, const __nv_bfloat16* xcl,
-                             const float* off, const uint8_t* wpk, const float* bias, float* y, cudaStream_t st) {
-    if (ndim == 2) return deform ? launch_tc_forward<2, true>(g, pl, xcl, off, wpk, bias, y, st)
-                                 : launch_tc_forward<2, false>(g, pl, xcl, off, wpk, bias, y, st);
-    return deform ? launch_tc_forward<3, true>(g, pl, xcl, off, wpk, bias, y, st)
-                  : launch_tc_forward<3, false>(g, pl, xcl, off, wpk, bias, y, st);
+                             const float* off, const uint8_t* wpk, const float* bias, float* y, float* slices, cudaStream_t st) {
+    if (ndim == 2) return deform ? launch_tc_forward<2, true>(g, pl, xcl, off, wpk, bias, y, slices, st)
+                                 : launch_tc_forward<2, false>(g, pl, xcl, off, wpk, bias, y, slices, st);
+    return deform ? launch_tc_forward<3, true>(g, pl, xcl, off, wpk, bias, y, slices, st)
+                  : launch_tc_forward<3, false>(g, pl, xcl, off, wpk, bias, y, slices, st);
+}
+// the fold of the split tiles' slices into y (`bias` and `y` of the launch)
+inline FoldY y_fold(const Geom& g, const FwdPlan& pl, const float* slices, const float* bias, float* y) {
+    const TcDims d = tc_dims(g);
+    const bool tail = pl.sp.KS0 == 1;
+    FoldY f = {};
+    f.slices = slices; f.bias = bias; f.y = y;
+    f.parts = tail ? pl.sp.KS1 : pl.sp.KS0;
+    f.tiles = (unsigned)(fwd_slices(pl.sp) / f.parts);
+    f.tile1 = tail ? (unsigned)pl.sp.tile1 : 0u;
+    f.halves = g.Og > 128 ? 2 : 1;
+    f.MB = d.MB;
+    f.add = pl.sp.acc;
+    f.d_PT.init((uint32_t)d.PT);
+    return f;
+}
+inline int launch_y_fold(const Geom& g, const FwdPlan& pl, const float* slices, const float* bias, float* y, bool last,
+                         cudaStream_t st) {
+    if (!pl.folds()) return 0;
+    const FoldY f = y_fold(g, pl, slices, bias, y);
+    return launch_dependent(tc_fold_y_kernel, dim3(f.tiles, 16u * (unsigned)f.halves), dim3(kPassThreads), 0, st, g, f,
+                            last ? 1 : 0) == cudaSuccess ? 0 : -5;
 }

@@ -2,7 +2,7 @@
 // has to happen before the first contraction of a call goes out as ONE launch, everything after the last as another.
 //
 // A pass is a list of jobs, each a range of blocks: input copy, weight tiles, packed dy, sampling points, zero fills; or
-// dX transpose, dW fold, bias-gradient fold.  The jobs of a list are independent of one another.  Each job moves its
+// dX transpose, dW fold, bias-gradient fold, fold of a forward pass's partial sums.  The jobs of a list are independent of one another.  Each job moves its
 // tensor once with coalesced accesses, so what is left to save at small and medium sizes is launches and the gaps
 // between them: a batch-1 inference call spent 10 of its 32 us of GPU time and most of its 36 us of host time in four
 // launches in front of the kernel, a layer step 28 launches (199 us busy, 237 us elapsed).
@@ -10,7 +10,7 @@
 
 
 
-enum JobType { kJobCopyX, kJobCastX, kJobWeight, kJobPackDy, kJobPackDyCl, kJobPoints, kJobZero, kJobDx, kJobDw, kJobBias };
+enum JobType { kJobCopyX, kJobCastX, kJobWeight, kJobPackDy, kJobPackDyCl, kJobPoints, kJobZero, kJobDx, kJobDw, kJobBias, kJobY };
 // operand tiles a weight job cuts (see the kernels for who reads which)
 enum WeightTiles {
     kTilesFwd,      // [G][MT][KC] 128 o x 64 k', k' = tap * Cg + c                          forward
@@ -35,9 +35,21 @@ constexpr int kMaxJobs = 12, kMaxGeoms = 3;
 constexpr int kPassThreads = 256;
 constexpr int kWeightSmem = 20 * 1024;       // of one weight job's block: ten blocks per SM stay resident
 
+// Partial sums of the split tiles of a forward pass, as its epilogue stores them; see fold_y.
+// Floats of a slice: [128-row half][lane quarter][16-position group][4 of them][lane][4].
+constexpr int kSliceGroup = 4 * 32 * 4, kSliceHalf = 4 * (kTileN / 16) * kSliceGroup;
+struct FoldY {
+    const float *slices, *bias;
+    float* y;
+    unsigned tiles, tile1;           // split tiles, the first of them
+    int parts, halves, MB, add;
+    FastDiv d_PT;
+};
+
 struct JobList {
     Geom g[kMaxGeoms];
     Job job[kMaxJobs];
+    FoldY fy;                        // of the kJobY job
     int n;
     int last;                        // no kernel of the call follows
 };
@@ -322,31 +334,24 @@ __device__ __forceinline__ void job_points(const Geom& g, const Job& J, unsigned
     }
 }
 
-// Zero fill of z floats at dst and z2 floats at aux (16-byte stores where aligned), or (a > 1) of a rows of z floats,
-// c floats apart.  b: blocks of the first range
+// Zero fill of z floats at dst and z2 floats at aux (16-byte stores where aligned).  b: blocks of the first range
 constexpr int kZeroPerBlock = 16 * kPassThreads;
 __device__ __forceinline__ void job_zero(const Job& J, unsigned blk) {
     const bool second = blk >= (unsigned)J.b;
     float* p = static_cast<float*>(second ? J.aux : J.dst);
     const size_t base = (size_t)(second ? blk - J.b : blk) * kZeroPerBlock, len = second ? J.z2 : J.z;
-    if (J.a == 1) {
-        const size_t n4 = (reinterpret_cast<uintptr_t>(p) & 15) == 0 ? len / 4 : 0;
+    const size_t n4 = (reinterpret_cast<uintptr_t>(p) & 15) == 0 ? len / 4 : 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const size_t e = base / 4 + i * kPassThreads + threadIdx.x;
-            if (e < n4) {
-                reinterpret_cast<float4*>(p)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-            } else {
+    for (int i = 0; i < 4; ++i) {
+        const size_t e = base / 4 + i * kPassThreads + threadIdx.x;
+        if (e < n4) {
+            reinterpret_cast<float4*>(p)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (e * 4 + k < len) p[e * 4 + k] = 0.f;
-            }
+            for (int k = 0; k < 4; ++k)
+                if (e * 4 + k < len) p[e * 4 + k] = 0.f;
         }
-        return;
     }
-    const size_t all = (size_t)J.a * J.z;
-    for (size_t e = base + threadIdx.x; e < base + kZeroPerBlock && e < all; e += kPassThreads)
-        p[e / J.z * (size_t)J.c + e % J.z] = 0.f;
 }
 
 // dx[n, c, p] (+)= dx_cl[n, p, c], tiles of 64 x 64.  a, b: tiles along positions / channels; c: add
@@ -435,6 +440,70 @@ __device__ __forceinline__ void job_bias(const Geom& g, const Job& J, unsigned b
     if (lane == 0) static_cast<float*>(J.dst)[o] = v;
 }
 
+// y of the split tiles of a forward pass: the slices of a tile added in K order, plus the bias.  (Reductions into a zeroed y
+// left the order, and with it the last bits, to whichever part came first.)  A block takes 32 output channels x 32 positions,
+// one 16-byte vector of every slice per thread, in the order in which the epilogue stored them; y leaves in 128-byte runs,
+// along the positions or the channels.
+// Bound by latency (launch, one read of L2, one turn).  Against the reductions, B200: one image 256 -> 256 channels 50x76,
+// 30 tiles in 4 parts: kernel 26.3 -> 20.0 us and 4.2 us of fold, call 28.5 -> 29.1; 8 x 128 -> 128, 28x28 as a layer, three
+// forward kernels in 3 parts: step 140 -> 152 us; config 2, 44 of 784 tiles in 3 parts: 1211 -> 1219; 2 x 128, 101x151, a tail
+// over two groups that could not be split before: 264 -> 256.  Folding in the CTA that finishes a tile last is slower: its
+// slices then pass through one SM (kernel 34.6 us for the first, step 170 us for the second).
+// piece: [half][lane quarter][32 positions]
+__device__ __forceinline__ void fold_y(const Geom& g, const FoldY& a, unsigned slot, unsigned piece, float* sm) {
+    const int cg = (int)(piece % 4), q = (int)(piece / 4 % 4), mt = (int)(piece / 16);
+    uint32_t jm, pt;
+    a.d_PT.divmod(a.tile1 + slot, jm, pt);
+    const int j = (int)(jm / (unsigned)a.MB), mb = (int)jm - j * a.MB;
+    const int o0 = (mb * 2 + mt) * 128 + q * 32, lane = threadIdx.x % 32, wp = threadIdx.x / 32;
+    const long long P0 = (long long)pt * kTileN + cg * 32;
+    if (o0 >= g.Og || P0 >= g.P) return;
+    const size_t step = (size_t)a.halves * kSliceHalf / 4;
+    const float4* s = reinterpret_cast<const float4*>(a.slices) + (size_t)slot * a.parts * step +
+                      (mt * kSliceHalf + q * (kSliceHalf / 4) + cg * 2 * kSliceGroup) / 4 + threadIdx.x;
+    const float bv = a.bias != nullptr && o0 + lane < g.Og ? __ldg(a.bias + j * g.Og + o0 + lane) : 0.f;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k0 = 0; k0 < a.parts; k0 += 4) {    // loads in batches of four (all in flight), additions in order
+        float4 t[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) t[u] = k0 + u < a.parts ? __ldg(s + (k0 + u) * step) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { v.x += t[u].x; v.y += t[u].y; v.z += t[u].z; v.w += t[u].w; }
+    }
+    float* row = sm + lane * 33 + wp * 4;        // positions 4 * wp .. of channel `lane`
+    row[0] = v.x + bv; row[1] = v.y + bv; row[2] = v.z + bv; row[3] = v.w + bv;
+    __syncthreads();
+    const int o = j * g.Og + o0;
+    if (g.cl) {
+        float* d = a.y + (size_t)(P0 + wp) * g.O + o + lane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i, d += 8 * (size_t)g.O) {
+            if (o0 + lane >= g.Og || P0 + wp + 8 * i >= g.P) continue;
+            const float r = sm[lane * 33 + wp + 8 * i];
+            *d = a.add ? *d + r : r;
+        }
+    } else if (P0 + lane < g.P) {
+        uint32_t n, opos;
+        g.d_ov.divmod((uint32_t)P0 + lane, n, opos);
+        float* d = a.y + ((size_t)n * g.O + o + wp) * g.ov + opos;
+#pragma unroll
+        for (int i = 0; i < 4; ++i, d += 8 * (size_t)g.ov) {
+            if (o0 + wp + 8 * i >= g.Og) continue;
+            const float r = sm[(wp + 8 * i) * 33 + lane];
+            *d = a.add ? *d + r : r;
+        }
+    }
+}
+
+// behind a forward pass, a launch of its own: grid (tiles, pieces).  last: no kernel of the call follows
+__global__ void __launch_bounds__(kPassThreads)
+tc_fold_y_kernel(const __grid_constant__ Geom g, const __grid_constant__ FoldY a, const int last) {
+    __shared__ float sm[32 * 33];
+    if (!last) pdl_trigger();
+    pdl_wait();
+    fold_y(g, a, blockIdx.x, blockIdx.y, sm);
+}
+
 __global__ void __launch_bounds__(kPassThreads, 6)
 tc_passes_kernel(const __grid_constant__ JobList L) {
     extern __shared__ float pass_smem[];
@@ -455,7 +524,8 @@ tc_passes_kernel(const __grid_constant__ JobList L) {
         case kJobZero: job_zero(J, b); break;
         case kJobDx: job_dx(g, J, b, pass_smem); break;
         case kJobDw: job_dw(g, J, b, pass_smem); break;
-        default: job_bias(g, J, b); break;
+        case kJobBias: job_bias(g, J, b); break;
+        default: fold_y(g, L.fy, b / (unsigned)J.a, b % (unsigned)J.a, pass_smem); break;
     }
 }
 
@@ -519,13 +589,12 @@ public:
         J.b = W2;
         J.blocks = (unsigned)(((long long)g.N * g.dg * g.kv * g.ov + 4 * kPassThreads - 1) / (4 * kPassThreads));
     }
-    // rows of len floats, pitch apart
-    void zero(float* p, size_t len, int rows = 1, int pitch = 0) {
-        if (p == nullptr || len == 0 || rows == 0) return;
-        const unsigned blocks = (unsigned)(((size_t)rows * len + kZeroPerBlock - 1) / kZeroPerBlock);
-        if (L.n > 0 && rows == 1) {                    // beside another contiguous one in the same job
+    void zero(float* p, size_t len) {
+        if (p == nullptr || len == 0) return;
+        const unsigned blocks = (unsigned)((len + kZeroPerBlock - 1) / kZeroPerBlock);
+        if (L.n > 0) {                                 // beside another one in the same job
             Job& last = L.job[L.n - 1];
-            if (last.type == kJobZero && last.a == 1 && last.aux == nullptr) {
+            if (last.type == kJobZero && last.aux == nullptr) {
                 last.aux = p;
                 last.z2 = len;
                 last.blocks += blocks;
@@ -533,8 +602,6 @@ public:
             }
         }
         Job& J = add(L.g[0], kJobZero, nullptr, p);
-        J.a = rows;
-        J.c = pitch;
         J.z = len;
         J.b = (int)blocks;
         J.blocks = blocks;
@@ -563,6 +630,15 @@ public:
         J.a = MT;
         J.z = (size_t)PC;
         J.blocks = (unsigned)((g.O + kPassThreads / 32 - 1) / (kPassThreads / 32));
+    }
+
+    // (one per launch)
+    void fold_y(const Geom& g, const FoldY& f) {
+        Job& J = add(g, kJobY, f.slices, f.y);
+        J.a = 16 * f.halves;
+        J.blocks = f.tiles * (unsigned)J.a;
+        L.fy = f;
+        need(32 * 33 * 4);
     }
 
     // one launch; last: of the call; apart: one launch per job

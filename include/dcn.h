@@ -106,7 +106,7 @@ size_t dcn_workspace_bytes(const dcn_problem* p, int pass);
 int dcn_launch_count(const dcn_problem* p, int pass);
 
 /* y = conv(x sampled at offset, weight) + bias.  `offset` may be NULL when deformable == 0, `bias` may
- * be NULL.  y is overwritten; precision EXACT gives the same bits on every call with the same arguments.
+ * be NULL.  y is overwritten, with the same bits on every call with the same arguments.
  * Replaces deform_conv_forward_cuda (deform3d/lib/deform_conv3d_cuda.cpp:90-165)
  * and the Python-side bias add (deform3d/deform_conv3d_functions/deform_conv3d_function.py:41-42). */
 int dcn_forward(const dcn_problem* p, const void* x, const void* offset, const void* weight, const void* bias,
@@ -119,8 +119,9 @@ int dcn_forward(const dcn_problem* p, const void* x, const void* offset, const v
  * Same arithmetic and results as dcn_forward with precision DCN_PREC_BF16 (other precisions are refused
  * with DCN_ERR_UNSUPPORTED).  The scratch is a fixed array inside the library image of
  * dcn_static_scratch_bytes() bytes (32 MiB), held on every device that loads the library until the process
- * exits; a problem whose forward workspace (dcn_workspace_bytes) exceeds it is refused with DCN_ERR_LIMIT
- * before anything is launched.  The first call on each device resolves the array's device address (this
+ * exits; a problem whose bf16 input copy and weight tiles exceed it is refused with DCN_ERR_LIMIT before anything
+ * is launched.  (Where they fit and the rest of the forward workspace does not, the sums of a tile are made in one
+ * piece instead of in parts, and y may differ from dcn_forward's in the last bits.)  The first call on each device resolves the array's device address (this
  * may load the library's device code), so make that first call outside any stream capture.  All calls on a
  * device share the one array, which keeps the previous call's contents; this pass overwrites every byte it
  * later reads, so nothing needs clearing, but two calls whose kernels overlap on the GPU (different

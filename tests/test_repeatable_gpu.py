@@ -44,3 +44,42 @@ def test_exact_forward_is_repeatable(case):
     tol = 1e-4 if case.dtype == "float32" else 1e-10
     assert cases.rel_err(first.cpu().numpy().astype(np.float64), _oracle(case, tensors)) <= tol
     assert all(torch.equal(_forward(case, tensors, "exact"), first) for _ in range(20))
+
+
+BF16 = [
+    Case("three_chunks_a_part", 2, 1, 64, 64, (19, 21), (3, 3), (1, 1), (1, 1), (1, 1), 1, 64, offset_std=2.0, bias=True),
+    Case("two_halves", 2, 2, 128, 136, (40, 40), (3, 3), (1, 1), (1, 1), (1, 1), 1, 32, offset_std=2.0, bias=True),
+    Case("tail_two_groups", 2, 4, 128, 96, (49, 50), (3, 3), (1, 1), (1, 1), (1, 1), 2, 64, offset_std=2.0, bias=True),
+    Case("tail_three_blocks", 2, 4, 64, 648, (50, 48), (3, 3), (1, 1), (1, 1), (1, 1), 1, 64, offset_std=2.0, bias=True),
+    Case("three_d", 3, 3, 64, 40, (2, 7, 7), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), 1, 64, offset_std=1.0),
+    Case("plain", 2, 2, 64, 192, (23, 21), (3, 3), (1, 1), (1, 1), (1, 1), 1, 64, deformable=False, bias=True),
+]
+
+
+@pytest.mark.parametrize("channels_last", [False, True])
+@pytest.mark.parametrize("case", BF16, ids=[c.name for c in BF16])
+def test_bf16_forward_is_repeatable(case, channels_last):
+    tensors = list(cases.make_inputs(case))
+    ref = _oracle(case, tensors)
+    if channels_last:
+        tensors[0] = tensors[0].contiguous(memory_format=torch.channels_last if case.ndim == 2 else torch.channels_last_3d)
+    first = _forward(case, tensors, "bf16")
+    assert cases.rel_err(first.cpu().numpy().astype(np.float64), ref) <= 2e-2
+    assert all(torch.equal(_forward(case, tensors, "bf16"), first) for _ in range(20))
+
+
+def test_bf16_plain_input_gradient_is_repeatable():
+    """The input gradient of a stride-1 plain convolution is a forward pass of the transposed one, split like it."""
+    import deform_conv3d_pytorch_op_b200 as dcn
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn((2, 64, 23, 21), generator=g, device="cuda").requires_grad_(True)
+    w = torch.randn((192, 64, 3, 3), generator=g, device="cuda") * 0.05
+    dy = torch.randn((2, 192, 23, 21), generator=g, device="cuda")
+
+    def dx():
+        return torch.autograd.grad(dcn.Conv2dFunction.apply(x, w, None, 1, 1, 1, 1, "bf16"), x, dy)[0]
+
+    first = dx()
+    want = torch.nn.grad.conv2d_input(x.shape, w.double(), dy.double(), padding=1)
+    assert cases.rel_err(first.cpu().numpy().astype(np.float64), want.cpu().numpy()) <= 2e-2
+    assert all(torch.equal(dx(), first) for _ in range(20))

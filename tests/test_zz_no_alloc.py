@@ -118,3 +118,29 @@ def test_static_scratch_address_is_resolved_per_device():
             torch.cuda.synchronize(dev)
             outs.append(y.cpu().numpy())
     assert np.isfinite(outs[0]).all() and np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.gpu
+def test_static_scratch_without_room_for_partial_sums():
+    """A problem whose input copy and weights fit the fixed array while the partial sums of a split do not is served, with
+    whole tiles.  Both calls round the same operands and sum K = 2304 products in fp32, in another order: they differ by
+    at most about K * 2^-24 = 1.4e-4 of the largest sum of magnitudes, which is a few times max|y|."""
+    from deform_conv3d_pytorch_op_b200 import _lib
+    L = _lib.lib()
+    dev = torch.device("cuda")
+    stream = _lib.current_stream(dev)
+    prob = _lib.make_problem(2, torch.float32, 9, 256, 256, (56, 56), (3, 3), 1, 1, 1, 1, 256, True, False, True, _lib.PREC_BF16)
+    nbytes = L.dcn_workspace_bytes(ctypes.byref(prob), 0)
+    assert nbytes > L.dcn_static_scratch_bytes()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.rand((9, 256, 56, 56), generator=g, device=dev) * 2 - 1
+    w = torch.randn((256, 256, 3, 3), generator=g, device=dev) * 0.03
+    off = torch.randn((9, 18, 56, 56), generator=g, device=dev)
+    y_ws, y_st = torch.full((2, 9, 256, 56, 56), float("nan"), device=dev)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    _lib.check(L.dcn_forward(ctypes.byref(prob), _lib.ptr(x), _lib.ptr(off), _lib.ptr(w), None, _lib.ptr(y_ws), _lib.ptr(ws),
+                             nbytes, stream), "dcn_forward")
+    _lib.check(L.dcn_forward_static_scratch(ctypes.byref(prob), _lib.ptr(x), _lib.ptr(off), _lib.ptr(w), None,
+                                            _lib.ptr(y_st), stream), "dcn_forward_static_scratch")
+    torch.cuda.synchronize()
+    assert cases.rel_err(y_st.cpu().numpy(), y_ws.cpu().numpy()) <= 1e-3
