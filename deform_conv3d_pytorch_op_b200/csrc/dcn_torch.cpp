@@ -19,6 +19,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <cuda_runtime_api.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -291,7 +292,10 @@ struct DcnBackward : public Node {
     Tensor fwd_ws;
     bool freed = false;
 
-    std::string name() const override { return kind == kLayer ? "DeformLayerFunctionBackward" : kind == kPlain ? "ConvFunctionBackward" : "ConvOffsetFunctionBackward"; }
+    std::string name() const override {
+        if (kind == kLayer) return "DeformLayerFunctionBackward";
+        return std::string(kind == kPlain ? "Conv" : "ConvOffset") + (q.p.ndim == 2 ? "2d" : "3d") + "FunctionBackward";
+    }
 
     variable_list apply(variable_list&& grads) override {
         const std::lock_guard<std::mutex> lock(mutex_);
@@ -354,8 +358,6 @@ Tensor call(const Spec& s, CallTensors& t) {
     for (int i = 0; i < kSlots; ++i) {
         has[i] = slot[i]->defined();
         need = need || (has[i] && slot[i]->requires_grad());
-        if (has[i] && torch::autograd::isFwGradDefined(*slot[i]))
-            throw std::runtime_error("forward-mode derivatives are not implemented for this operator");
     }
     need = need && at::GradMode::is_enabled();
     const Problem q = make_problem(s, t.x, t.w);
@@ -383,6 +385,17 @@ Tensor call(const Spec& s, CallTensors& t) {
     if (t.ow.defined()) node->ow = SavedVariable(t.ow, false);
     torch::autograd::set_history(y, node);
     return y;
+}
+
+// Calls that have to go through a torch.autograd.Function: a trace records it as one operation (a direct call would leave
+// its result in the trace as a constant), and function transforms and forward-mode derivatives ask it for rules.
+bool transformed(const CallTensors& t) {
+    if (torch::jit::tracer::isTracing() ||
+        c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+        return true;
+    for (const Tensor* v : {&t.x, &t.off, &t.w, &t.b, &t.ow, &t.ob})
+        if (v->defined() && torch::autograd::isFwGradDefined(*v)) return true;
+    return false;
 }
 
 // ---- arguments ------------------------------------------------------------------------------------------------
@@ -447,6 +460,7 @@ PyObject* entry(Parse&& parse) {
         Spec s;
         CallTensors t;
         parse(s, t);
+        if (transformed(t)) Py_RETURN_NOTIMPLEMENTED;          // functions.py takes the other way
         Tensor y;
         {
             pybind11::gil_scoped_release no_gil;

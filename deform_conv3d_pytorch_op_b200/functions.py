@@ -15,15 +15,83 @@ together), and two optional trailing arguments select the arithmetic (``precisio
 and the 3-D out-of-bounds offset pseudo-gradient (``oob_offset_grad``).
 
 The work behind ``.apply`` -- checks, allocation, the library call, the graph node of the backward pass -- is C++
-(``csrc/dcn_torch.cpp``): in Python it cost more than the kernels of a small layer.
+(``csrc/dcn_torch.cpp``): in Python it cost more than the kernels of a small layer.  The classes are therefore no
+subclasses of ``torch.autograd.Function``; where a trace, a function transform (``torch.func``) or a forward-mode
+derivative needs one, the call goes through the ``_...Function`` of the same arguments below.
 """
 from __future__ import annotations
 
+from torch.autograd import Function
+from torch.autograd.function import once_differentiable
+
 from . import _lib
+from .ops import Op, check_status, status_check_enabled
 
 
 def _tup(v, n):
     return tuple(v) if isinstance(v, (tuple, list)) else (v,) * n
+
+
+def _check(x):
+    if status_check_enabled():
+        check_status(x.device)
+
+
+class _DeformFunction(Function):
+    @staticmethod
+    def forward(ctx, ndim, inputs, offset, weight, bias=None, stride=1, padding=0, dilation=1, channel_per_group=1,
+                group=1, precision=None, oob_offset_grad=None):
+        if inputs.dim() != ndim + 2:
+            raise RuntimeError("input dim")
+        ctx.op = Op(inputs, weight, _tup(stride, ndim), _tup(padding, ndim), _tup(dilation, ndim), channel_per_group,
+                    group, oob_offset_grad=oob_offset_grad, precision=precision)
+        ctx.save_for_backward(inputs, offset, weight)
+        return ctx.op.forward(inputs, offset, weight, bias)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dy):
+        grads = ctx.op.backward(*ctx.saved_tensors, dy, *ctx.needs_input_grad[1:5])
+        _check(dy)
+        return (None,) + grads + (None,) * 7
+
+
+class _PlainFunction(Function):
+    @staticmethod
+    def forward(ctx, ndim, inputs, weight, bias=None, stride=1, padding=0, dilation=1, group=1, precision=None):
+        if inputs.dim() != ndim + 2:
+            raise RuntimeError("input dim")
+        ctx.op = Op(inputs, weight, _tup(stride, ndim), _tup(padding, ndim), _tup(dilation, ndim), inputs.size(1),
+                    group, deformable=False, std_size_rule=True, precision=precision)
+        ctx.save_for_backward(inputs, weight)
+        return ctx.op.forward(inputs, None, weight, bias)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dy):
+        inputs, weight = ctx.saved_tensors
+        _, need_x, need_w, need_b = ctx.needs_input_grad[:4]
+        dx, _, dw, db = ctx.op.backward(inputs, None, weight, dy, need_x, False, need_w, need_b)
+        return (None, dx, dw, db) + (None,) * 5
+
+
+class _LayerFunction(Function):
+    @staticmethod
+    def forward(ctx, inputs, offset_weight, offset_bias, weight, bias, stride, padding, dilation, channel_per_group=1,
+                group=1, precision=None, oob_offset_grad=None):
+        ndim = inputs.dim() - 2
+        ctx.op = Op(inputs, weight, _tup(stride, ndim), _tup(padding, ndim), _tup(dilation, ndim), channel_per_group,
+                    group, oob_offset_grad=oob_offset_grad, precision=precision)
+        y, offset = ctx.op.layer_forward(inputs, offset_weight, offset_bias, weight, bias)
+        ctx.save_for_backward(inputs, offset, offset_weight, weight)
+        return y
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dy):
+        grads = ctx.op.layer_backward(*ctx.saved_tensors, dy, *ctx.needs_input_grad[:5])
+        _check(dy)
+        return grads + (None,) * 7
 
 
 class ConvOffset3dFunction:
@@ -32,7 +100,8 @@ class ConvOffset3dFunction:
 
     @staticmethod
     def apply(*args):
-        return _lib.native().conv_offset3d(*args)
+        y = _lib.native().conv_offset3d(*args)
+        return _DeformFunction.apply(3, *args) if y is NotImplemented else y
 
 
 class ConvOffset2dFunction:
@@ -41,7 +110,8 @@ class ConvOffset2dFunction:
 
     @staticmethod
     def apply(*args):
-        return _lib.native().conv_offset2d(*args)
+        y = _lib.native().conv_offset2d(*args)
+        return _DeformFunction.apply(2, *args) if y is NotImplemented else y
 
 
 class Conv2dFunction:
@@ -50,7 +120,8 @@ class Conv2dFunction:
 
     @staticmethod
     def apply(*args):
-        return _lib.native().conv2d(*args)
+        y = _lib.native().conv2d(*args)
+        return _PlainFunction.apply(2, *args) if y is NotImplemented else y
 
 
 class Conv3dFunction:
@@ -59,7 +130,8 @@ class Conv3dFunction:
 
     @staticmethod
     def apply(*args):
-        return _lib.native().conv3d(*args)
+        y = _lib.native().conv3d(*args)
+        return _PlainFunction.apply(3, *args) if y is NotImplemented else y
 
 
 class DeformLayerFunction:
@@ -70,7 +142,8 @@ class DeformLayerFunction:
 
     @staticmethod
     def apply(*args):
-        return _lib.native().deform_layer(*args)
+        y = _lib.native().deform_layer(*args)
+        return _LayerFunction.apply(*args) if y is NotImplemented else y
 
 
 class LegacyConvOffset2dFunction:

@@ -40,6 +40,11 @@ def check_status(device=None) -> None:
         _lib.check(_lib.lib().dcn_check_status(_lib.current_stream(dev)), "device status")
 
 
+def status_check_enabled() -> bool:
+    """Whether a backward pass checks the status word (``DCN_CHECK_STATUS=1``, and not while a stream is captured)."""
+    return os.environ.get("DCN_CHECK_STATUS", "0") not in ("", "0") and not torch.cuda.is_current_stream_capturing()
+
+
 def _nvtx_enabled() -> bool:
     """``DCN_NVTX=1``: wrap every library call of :class:`Op` in an NVTX range named after the entry point, so that
     the passes show up by name on a profiler's timeline (the reference has only wall-clock prints,

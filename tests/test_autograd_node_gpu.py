@@ -1,0 +1,71 @@
+"""The operator's place in torch's machinery: its graph node, traces, function transforms, forward mode."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _make(kind, precision="exact"):
+    """(callable, its tensor arguments as leaves that want gradients)"""
+    import deform_conv3d_pytorch_op_b200 as dcn
+    g = torch.Generator(device="cuda").manual_seed(7)
+
+    def leaf(*shape, std=1.0):
+        return (torch.randn(shape, generator=g, device="cuda") * std).requires_grad_(True)
+
+    x, w, b = leaf(2, 16, 13, 12), leaf(24, 16, 3, 3, std=0.1), leaf(24)
+    if kind == "deform":
+        return (lambda x, off, w, b: dcn.ConvOffset2dFunction.apply(x, off, w, b, 1, 1, 1, 16, 1, precision),
+                [x, leaf(2, 18, 13, 12), w, b])
+    if kind == "plain":
+        return lambda x, w, b: dcn.Conv2dFunction.apply(x, w, b, 1, 1, 1, 1, precision), [x, w, b]
+    return (lambda x, ow, ob, w, b: dcn.DeformLayerFunction.apply(x, ow, ob, w, b, 1, 1, 1, 16, 1, precision),
+            [x, leaf(18, 16, 3, 3, std=0.05), leaf(18, std=0.1), w, b])
+
+
+def _close(a, b):
+    # exact precision: the same sums of at most 16 * 9 products, the gradients' in another order
+    return torch.allclose(a, b, rtol=1e-4, atol=1e-4 * float(b.abs().max()))
+
+
+KINDS = ["deform", "plain", "layer"]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_trace_records_the_operation(kind):
+    fn, args = _make(kind)
+    traced = torch.jit.trace(fn, tuple(a.detach() for a in args), check_trace=False)
+    other = [(a.detach() * 0.5 + 0.1).requires_grad_(True) for a in args]
+    y, want = traced(*other), fn(*other)
+    assert _close(y, want)
+    dy = torch.randn_like(y)
+    for a, b in zip(torch.autograd.grad(y, other, dy), torch.autograd.grad(want, other, dy)):
+        assert _close(a, b)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_transforms_and_forward_mode_are_refused_by_torch(kind):
+    import torch.autograd.forward_ad as fw
+    fn, args = _make(kind)
+    args = [a.detach() for a in args]
+    for i in (0, len(args) - 1):
+        def of(v):
+            return fn(*args[:i], v, *args[i + 1:])
+        with pytest.raises(RuntimeError, match="setup_context"):
+            torch.func.grad(lambda v: of(v).sum())(args[i])
+        with pytest.raises(RuntimeError, match="setup_context"):
+            torch.vmap(of)(torch.stack([args[i]] * 2))
+        with pytest.raises(RuntimeError, match="setup_context"):
+            torch.func.functionalize(of)(args[i])
+        with fw.dual_level(), pytest.raises(NotImplementedError):
+            of(fw.make_dual(args[i], torch.ones_like(args[i])))
+    assert torch.isfinite(fn(*args)).all()
+
+
+def test_compiled_callers_keep_the_operation():
+    fn, args = _make("deform")
+    compiled = torch.compile(lambda x, *rest: fn(x * 2, *rest).relu(), backend="aot_eager")
+    y, want = compiled(*args), fn(args[0] * 2, *args[1:]).relu()
+    assert _close(y, want)
+    for a, b in zip(torch.autograd.grad(y.sum(), args), torch.autograd.grad(want.sum(), args)):
+        assert _close(a, b)
