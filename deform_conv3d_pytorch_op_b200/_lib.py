@@ -43,7 +43,7 @@ GENERIC_SYMBOLS = [
     "dcn_workspace_bytes", "dcn_launch_count", "dcn_forward", "dcn_backward_data", "dcn_backward_weight", "dcn_backward", "dcn_debug_points",
     "dcn_debug_tc_points", "dcn_debug_expire_wait",
     "dcn_check_status", "dcn_static_scratch_bytes", "dcn_forward_static_scratch",
-    "dcn_offset_conv_problem", "dcn_layer_workspace_bytes", "dcn_layer_forward", "dcn_layer_backward", "dcn_layer_launch_count",
+    "dcn_input_copy_bytes", "dcn_forward_keep", "dcn_layer_forward_keep", "dcn_offset_conv_problem", "dcn_layer_workspace_bytes", "dcn_layer_forward", "dcn_layer_backward", "dcn_layer_launch_count",
 ]
 LEGACY_SYMBOLS = [
     "dcn_deform3d_deform_conv_forward_cuda", "dcn_deform3d_deform_conv_backward_input_offset_cuda",
@@ -76,6 +76,10 @@ def lib() -> ctypes.CDLL:
         L.dcn_workspace_bytes.argtypes = [pp, ctypes.c_int]
         L.dcn_launch_count.argtypes = [pp, ctypes.c_int]
         L.dcn_forward.argtypes = [pp, vp, vp, vp, vp, vp, vp, ctypes.c_size_t, vp]
+        L.dcn_input_copy_bytes.restype = ctypes.c_size_t
+        L.dcn_input_copy_bytes.argtypes = [pp]
+        L.dcn_forward_keep.argtypes = [pp, vp, vp, vp, vp, vp, vp, vp, ctypes.c_size_t, vp]
+        L.dcn_layer_forward_keep.argtypes = [pp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ctypes.c_size_t, vp]
         L.dcn_backward_data.argtypes = [pp, vp, vp, vp, vp, vp, vp, vp, ctypes.c_size_t, vp]
         L.dcn_backward_weight.argtypes = [pp, vp, vp, vp, vp, vp, vp, ctypes.c_size_t, vp]
         L.dcn_backward.argtypes = [pp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ctypes.c_size_t, vp]

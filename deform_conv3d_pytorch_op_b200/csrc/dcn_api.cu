@@ -85,6 +85,9 @@ bool exact_ready(const dcn_problem* p, const Geom& g, int pass, const void* ws, 
            workspace_ok(ws, ws_bytes, dcn::exact_workspace_bytes(g, p->dtype, p->deformable, pass));
 }
 
+// bytes that a forward workspace needs less where the caller takes the input copy elsewhere
+size_t kept(const Geom& g, const void* x_channels_last) { return x_channels_last != nullptr ? dcn::tc_input_copy_bytes(g) : 0; }
+
 int check_ptrs(const dcn_problem* p, std::initializer_list<const void*> ptrs) {
     const size_t es = p->dtype == DCN_F64 ? 8 : 4;
     for (const void* q : ptrs)
@@ -157,8 +160,20 @@ int dcn_launch_count(const dcn_problem* p, int pass) {
     return dcn::tc_launch_count(g, p->ndim, p->deformable, pass);
 }
 
+size_t dcn_input_copy_bytes(const dcn_problem* p) {
+    if (validate(p) != DCN_OK || p->precision != DCN_PREC_BF16) return 0;
+    Geom g;
+    make_geom(p, g);
+    return dcn::tc_supported(g, p->ndim, p->deformable) ? dcn::tc_input_copy_bytes(g) : 0;
+}
+
 int dcn_forward(const dcn_problem* p, const void* x, const void* offset, const void* weight, const void* bias,
                 void* y, void* ws, size_t ws_bytes, void* stream) {
+    return dcn_forward_keep(p, x, offset, weight, bias, y, nullptr, ws, ws_bytes, stream);
+}
+
+int dcn_forward_keep(const dcn_problem* p, const void* x, const void* offset, const void* weight, const void* bias,
+                     void* y, void* x_channels_last, void* ws, size_t ws_bytes, void* stream) {
     const int v = validate(p);
     if (v != DCN_OK) return v;
     if (x == nullptr || weight == nullptr || y == nullptr || (p->deformable && offset == nullptr)) return DCN_ERR_NULL;
@@ -169,9 +184,11 @@ int dcn_forward(const dcn_problem* p, const void* x, const void* offset, const v
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (p->precision == DCN_PREC_BF16) {
         if (!dcn::tc_supported(g, p->ndim, p->deformable)) return DCN_ERR_UNSUPPORTED;
-        if (!workspace_ok(ws, ws_bytes, dcn::tc_workspace_bytes(g, p->ndim, DCN_PASS_FORWARD))) return DCN_ERR_WORKSPACE;
+        if (!workspace_ok(ws, ws_bytes + kept(g, x_channels_last), dcn::tc_workspace_bytes(g, p->ndim, DCN_PASS_FORWARD)))
+            return DCN_ERR_WORKSPACE;
+        if (!aligned(x_channels_last, 16)) return DCN_ERR_ALIGN;
         return dcn::tc_forward(g, p->ndim, p->deformable, (const float*)x, (const float*)offset,
-                               (const float*)weight, (const float*)bias, (float*)y, ws, ws_bytes, st);
+                               (const float*)weight, (const float*)bias, (float*)y, x_channels_last, ws, ws_bytes, st);
     }
     if (exact_ready(p, g, DCN_PASS_FORWARD, ws, ws_bytes))
         return dcn::exact_forward(g, p->dtype, p->ndim, p->deformable, x, offset, weight, bias, y, ws, st);
@@ -422,6 +439,12 @@ int dcn_layer_launch_count(const dcn_problem* p, int pass) {
 int dcn_layer_forward(const dcn_problem* p, const void* x, const void* offset_weight, const void* offset_bias,
                       const void* weight, const void* bias, void* offset, void* y, void* ws, size_t ws_bytes,
                       void* stream) {
+    return dcn_layer_forward_keep(p, x, offset_weight, offset_bias, weight, bias, offset, y, nullptr, ws, ws_bytes, stream);
+}
+
+int dcn_layer_forward_keep(const dcn_problem* p, const void* x, const void* offset_weight, const void* offset_bias,
+                           const void* weight, const void* bias, void* offset, void* y, void* x_channels_last, void* ws,
+                           size_t ws_bytes, void* stream) {
     dcn_problem q;
     const int v = dcn_offset_conv_problem(p, &q);
     if (v != DCN_OK) return v;
@@ -445,10 +468,12 @@ int dcn_layer_forward(const dcn_problem* p, const void* x, const void* offset_we
     make_geom(p, g);
     make_geom(&q, gq);
     if (!dcn::tc_supported(g, p->ndim, 1) || !dcn::tc_supported(gq, p->ndim, 0)) return DCN_ERR_UNSUPPORTED;
-    if (!workspace_ok(ws, ws_bytes, dcn::tc_layer_workspace_bytes(g, gq, p->ndim, 0))) return DCN_ERR_WORKSPACE;
+    if (!workspace_ok(ws, ws_bytes + kept(g, x_channels_last), dcn::tc_layer_workspace_bytes(g, gq, p->ndim, 0)))
+        return DCN_ERR_WORKSPACE;
+    if (!aligned(x_channels_last, 16)) return DCN_ERR_ALIGN;
     return dcn::tc_layer_forward(g, gq, p->ndim, (const float*)x, (const float*)offset_weight, (const float*)offset_bias,
-                                 (const float*)weight, (const float*)bias, (float*)offset, (float*)y, ws, ws_bytes,
-                                 static_cast<cudaStream_t>(stream));
+                                 (const float*)weight, (const float*)bias, (float*)offset, (float*)y, x_channels_last, ws,
+                                 ws_bytes, static_cast<cudaStream_t>(stream));
 }
 
 int dcn_layer_backward(const dcn_problem* p, const void* x, const void* offset, const void* offset_weight,

@@ -73,8 +73,10 @@ int exact_backward(const Geom& g, int dtype, int ndim, int deform, int pass, int
 // BF16 tensor-core (tcgen05) path, dcn_tc.cu.  fp32 tensors only.
 bool tc_supported(const Geom& g, int ndim, int deform);
 size_t tc_workspace_bytes(const Geom& g, int ndim, int pass);
+// xcl_out: where the channels-last copy of x goes, tc_input_copy_bytes() that the workspace then needs less (null: its start)
+size_t tc_input_copy_bytes(const Geom& g);
 int tc_forward(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
-               const float* bias, float* y, void* ws, size_t ws_bytes, cudaStream_t st);
+               const float* bias, float* y, void* xcl_out, void* ws, size_t ws_bytes, cudaStream_t st);
 int tc_backward_data(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
                      const float* dy, float* dx, float* doff, void* ws, size_t ws_bytes, cudaStream_t st);
 int tc_backward_weight(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* dy,
@@ -87,7 +89,7 @@ int tc_backward(const Geom& g, int ndim, int deform, const float* x, const float
 // deformable layer = offset-producing plain convolution (gq) + deformable convolution (g) of the same input
 size_t tc_layer_workspace_bytes(const Geom& g, const Geom& gq, int ndim, int pass);
 int tc_layer_forward(const Geom& g, const Geom& gq, int ndim, const float* x, const float* w_off, const float* b_off,
-                     const float* w, const float* bias, float* offsets, float* y, void* ws, size_t ws_bytes,
+                     const float* w, const float* bias, float* offsets, float* y, void* xcl_out, void* ws, size_t ws_bytes,
                      cudaStream_t st);
 int tc_layer_backward(const Geom& g, const Geom& gq, int ndim, const float* x, const float* offsets, const float* w_off,
                       const float* w, const float* dy, const void* xcl_in, float* dx, float* dw_off, float* db_off, float* dw,

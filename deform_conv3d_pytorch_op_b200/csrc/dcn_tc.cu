@@ -119,7 +119,7 @@ FwdWorkspace fwd_workspace(const Geom& g, size_t have = SIZE_MAX) {
     const TcDims d = tc_dims(g);
     FwdWorkspace w;
     w.xcl_off = 0;
-    w.wpk_off = align_up((size_t)g.N * g.iv * g.C * 2, 256);
+    w.wpk_off = tc_input_copy_bytes(g);
     w.slices_off = w.wpk_off + align_up((size_t)g.G * d.MT * d.KC * kTileBytes, 256);
     w.split = fwd_split(g, have > w.slices_off ? have - w.slices_off : 0);
     w.total = w.slices_off + align_up((size_t)fwd_slices(w.split) * fwd_slice_bytes(g), 256);
@@ -369,15 +369,18 @@ int tc_debug_points(const Geom& g, int ndim, int deform, const float* off, int n
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
+size_t tc_input_copy_bytes(const Geom& g) { return align_up((size_t)g.N * g.iv * g.C * 2, 256); }
+
 int tc_forward(const Geom& g, int ndim, int deform, const float* x, const float* off, const float* w,
-               const float* bias, float* y, void* ws, size_t ws_bytes, cudaStream_t st) {
-    const FwdWorkspace l = fwd_workspace(g, ws_bytes);
-    if (ws_bytes < l.total) return -4;
+               const float* bias, float* y, void* xcl_out, void* ws, size_t ws_bytes, cudaStream_t st) {
+    const size_t less = xcl_out != nullptr ? tc_input_copy_bytes(g) : 0;      // of the workspace, which starts behind the copy
+    const FwdWorkspace l = fwd_workspace(g, ws_bytes + less);
+    if (ws_bytes + less < l.total) return -4;
     uint8_t* base = static_cast<uint8_t*>(ws);
-    __nv_bfloat16* xcl = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
-    uint8_t* wpk = base + l.wpk_off;
+    __nv_bfloat16* xcl = static_cast<__nv_bfloat16*>(xcl_out != nullptr ? xcl_out : ws);
+    uint8_t* wpk = base + (l.wpk_off - less);
     const FwdPlan plan = fwd_plan(g, l.split, ndim, deform, y, false);
-    float* slices = reinterpret_cast<float*>(base + l.slices_off);
+    float* slices = reinterpret_cast<float*>(base + (l.slices_off - less));
     Passes p;
     p.copy_x(g, x, xcl);
     p.weight(g, kTilesFwd, w, wpk);
@@ -480,23 +483,24 @@ size_t tc_layer_workspace_bytes(const Geom& g, const Geom& gq, int ndim, int pas
 }
 
 int tc_layer_forward(const Geom& g, const Geom& gq, int ndim, const float* x, const float* w_off, const float* b_off,
-                     const float* w, const float* bias, float* offsets, float* y, void* ws, size_t ws_bytes,
+                     const float* w, const float* bias, float* offsets, float* y, void* xcl_out, void* ws, size_t ws_bytes,
                      cudaStream_t st) {
     const FwdWorkspace l = fwd_workspace(g), lq = fwd_workspace(gq);
-    if (ws_bytes < l.total + lq.total) return -4;
+    const size_t less = xcl_out != nullptr ? tc_input_copy_bytes(g) : 0;
+    if (ws_bytes + less < l.total + lq.total) return -4;
     uint8_t* base = static_cast<uint8_t*>(ws);
-    uint8_t* baseq = base + l.total;
-    float *slices = reinterpret_cast<float*>(base + l.slices_off), *slicesq = reinterpret_cast<float*>(baseq + lq.slices_off);
-    __nv_bfloat16* xcl = reinterpret_cast<__nv_bfloat16*>(base + l.xcl_off);
+    uint8_t *wpk = base + (l.wpk_off - less), *baseq = base + (l.total - less);
+    float *slices = reinterpret_cast<float*>(base + (l.slices_off - less)), *slicesq = reinterpret_cast<float*>(baseq + lq.slices_off);
+    __nv_bfloat16* xcl = static_cast<__nv_bfloat16*>(xcl_out != nullptr ? xcl_out : ws);
     const FwdPlan pq = fwd_plan(gq, lq.split, ndim, 0, offsets, false), pl = fwd_plan(g, l.split, ndim, 1, y, false);
     Passes p;
     p.copy_x(g, x, xcl);
     p.weight(gq, kTilesFwd, w_off, baseq + lq.wpk_off);
-    p.weight(g, kTilesFwd, w, base + l.wpk_off);
+    p.weight(g, kTilesFwd, w, wpk);
     int r = p.launch(st, false);
     if (r == 0) r = launch_tc_forward(gq, pq, ndim, 0, xcl, nullptr, baseq + lq.wpk_off, b_off, offsets, slicesq, st);
     if (r == 0) r = launch_y_fold(gq, pq, slicesq, b_off, offsets, false, st);
-    if (r == 0) r = launch_tc_forward(g, pl, ndim, 1, xcl, offsets, base + l.wpk_off, bias, y, slices, st);
+    if (r == 0) r = launch_tc_forward(g, pl, ndim, 1, xcl, offsets, wpk, bias, y, slices, st);
     return r != 0 ? r : launch_y_fold(g, pl, slices, bias, y, true, st);
 }
 
@@ -576,7 +580,7 @@ int tc_forward_static(const Geom& g, int ndim, int deform, const float* x, const
         if (cudaGetSymbolAddress(&ptr, g_static_scratch) != cudaSuccess || ptr == nullptr) return -5;
         scratch_of_device[dev] = ptr;      // racing first calls resolve the same address
     }
-    return tc_forward(g, ndim, deform, x, off, w, bias, y, ptr, kStaticScratchBytes, st);
+    return tc_forward(g, ndim, deform, x, off, w, bias, y, nullptr, ptr, kStaticScratchBytes, st);
 }
 
 // A wait that cannot complete: one thread waits, with a limit of about a millisecond, on a barrier nothing ever

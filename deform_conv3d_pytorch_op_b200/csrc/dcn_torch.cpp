@@ -204,9 +204,8 @@ struct CallTensors {
     Tensor x, off, w, b, ow, ob;         // off: kDeform; ow, ob: kLayer
 };
 
-// Forward pass; on the bf16 path `keep` receives the workspace, whose start holds the input copy (half the input's
-// size) that the backward pass takes over.
-// For a layer t.off receives the offsets.
+// Forward pass; on the bf16 path `keep` (if not null) receives the input copy, half the input's size, that the backward pass
+// takes over.  For a layer t.off receives the offsets.
 Tensor run_forward(const Problem& q, Kind kind, CallTensors& t, Tensor* keep) {
     const Tensor x = prep(t.x, "input", t.x, q.act);
     const Tensor w = prep(t.w, "weight", x), b = prep(t.b, "bias", x);
@@ -230,25 +229,30 @@ Tensor run_forward(const Problem& q, Kind kind, CallTensors& t, Tensor* keep) {
     const c10::cuda::CUDAGuard guard(x.device());
     void* st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
     Tensor y = at::empty(with_out(q, q.p.N, q.p.O), x.options().memory_format(q.act));
+    const size_t copy = keep != nullptr ? dcn_input_copy_bytes(&q.p) : 0;
+    if (copy != 0) {
+        *keep = scratch(copy, x);
+        bytes -= copy;
+    }
+    void* xcl = copy != 0 ? wptr(*keep) : nullptr;
     const Tensor ws = scratch(bytes, x);
     if (kind == kLayer) {
         Range range("dcn_layer_forward");
         off = at::empty(with_out(q, q.p.N, offset_channels(q)), x.options());
-        check(dcn_layer_forward(&q.p, ptr(x), ptr(ow), ptr(ob), ptr(w), ptr(b), wptr(off), wptr(y), wptr(ws), bytes, st),
-              "dcn_layer_forward");
+        check(dcn_layer_forward_keep(&q.p, ptr(x), ptr(ow), ptr(ob), ptr(w), ptr(b), wptr(off), wptr(y), xcl, wptr(ws), bytes,
+                                     st), "dcn_layer_forward");
         t.off = off;
     } else {
         Range range("dcn_forward");
-        check(dcn_forward(&q.p, ptr(x), ptr(off), ptr(w), ptr(b), wptr(y), wptr(ws), bytes, st), "dcn_forward");
+        check(dcn_forward_keep(&q.p, ptr(x), ptr(off), ptr(w), ptr(b), wptr(y), xcl, wptr(ws), bytes, st), "dcn_forward");
     }
-    if (keep != nullptr && q.p.precision == DCN_PREC_BF16) *keep = ws;
     return y;
 }
 
 // Gradient slots, in the order of the node's edges.
 enum Slot { kGx, kGoff, kGw, kGb, kGow, kGob, kSlots };
 
-void run_backward(const Problem& q, Kind kind, const CallTensors& t, const Tensor& grad, const Tensor& fwd_ws,
+void run_backward(const Problem& q, Kind kind, const CallTensors& t, const Tensor& grad, const Tensor& xcl,
                   const bool (&want)[kSlots], Tensor (&g)[kSlots]) {
     const Tensor x = prep(t.x, "input", t.x, q.act);
     const Tensor w = prep(t.w, "weight", x), off = prep(t.off, "offset", x), ow = prep(t.ow, "offset_weight", x);
@@ -266,14 +270,14 @@ void run_backward(const Problem& q, Kind kind, const CallTensors& t, const Tenso
         const size_t bytes = dcn_layer_workspace_bytes(&q.p, DCN_PASS_BACKWARD);
         const Tensor ws = scratch(bytes, x);
         Range range("dcn_layer_backward");
-        check(dcn_layer_backward(&q.p, ptr(x), ptr(off), ptr(ow), ptr(w), ptr(dy), ptr(fwd_ws), wptr(g[kGx]), wptr(g[kGow]),
+        check(dcn_layer_backward(&q.p, ptr(x), ptr(off), ptr(ow), ptr(w), ptr(dy), ptr(xcl), wptr(g[kGx]), wptr(g[kGow]),
                                  wptr(g[kGob]), wptr(g[kGw]), wptr(g[kGb]), wptr(ws), bytes, stream.stream()),
               "dcn_layer_backward");
     } else {
         const size_t bytes = dcn_workspace_bytes(&q.p, DCN_PASS_BACKWARD);
         const Tensor ws = scratch(bytes, x);
         Range range("dcn_backward");
-        check(dcn_backward(&q.p, ptr(x), ptr(off), ptr(w), ptr(dy), ptr(fwd_ws), wptr(g[kGx]), wptr(g[kGoff]),
+        check(dcn_backward(&q.p, ptr(x), ptr(off), ptr(w), ptr(dy), ptr(xcl), wptr(g[kGx]), wptr(g[kGoff]),
                            wptr(g[kGw]), wptr(g[kGb]), wptr(ws), bytes, stream.stream()),
               "dcn_backward");
     }
@@ -289,7 +293,7 @@ struct DcnBackward : public Node {
     Kind kind = kDeform;
     bool has[kSlots] = {};               // inputs the call had; their edges come in slot order
     SavedVariable x, off, w, ow;
-    Tensor fwd_ws;
+    Tensor xcl;
     bool freed = false;
 
     std::string name() const override {
@@ -319,7 +323,7 @@ struct DcnBackward : public Node {
             differentiated = at::GradMode::is_enabled() && dy.defined() && dy.requires_grad();
             at::NoGradGuard no_grad;
             if (!dy.defined()) dy = at::zeros(with_out(q, q.p.N, q.p.O), t.x.options());
-            run_backward(q, kind, t, dy, fwd_ws, want, g);
+            run_backward(q, kind, t, dy, xcl, want, g);
         } catch (const DcnFailure& e) {
             pybind11::gil_scoped_acquire gil;
             PyErr_SetString(g_error, e.text.c_str());
@@ -347,7 +351,7 @@ struct DcnBackward : public Node {
         off.reset_data();
         w.reset_data();
         ow.reset_data();
-        fwd_ws.reset();
+        xcl.reset();
     }
 };
 
@@ -377,7 +381,13 @@ Tensor call(const Spec& s, CallTensors& t) {
     Tensor y;
     {
         at::NoGradGuard no_grad;
-        y = run_forward(q, s.kind, t, &node->fwd_ws);
+        // the input copy is kept only where a gradient needs it, and never past saved-tensor hooks: a program that moves or
+        // drops what is saved (offloading, checkpoints) gets the tensors named below and nothing beside them
+        bool kept = t.w.requires_grad();
+        if (s.kind != kPlain)
+            for (int i : {kGx, kGoff, kGow, kGob}) kept = kept || (has[i] && slot[i]->requires_grad());
+        kept = kept && !at::SavedTensorDefaultHooks::get_hooks().has_value();
+        y = run_forward(q, s.kind, t, kept ? &node->xcl : nullptr);
     }
     node->x = SavedVariable(t.x, false);
     node->w = SavedVariable(t.w, false);

@@ -112,6 +112,14 @@ int dcn_launch_count(const dcn_problem* p, int pass);
 int dcn_forward(const dcn_problem* p, const void* x, const void* offset, const void* weight, const void* bias,
                 void* y, void* workspace, size_t workspace_bytes, void* stream);
 
+/* dcn_forward that leaves the channels-last bf16 copy of x in a buffer of the caller instead of the workspace, so that the
+ * copy can be kept for dcn_backward without the rest: x_channels_last has dcn_input_copy_bytes(p) bytes (16-byte aligned),
+ * the workspace that many bytes less than dcn_workspace_bytes(p, DCN_PASS_FORWARD).  With x_channels_last == NULL it is
+ * dcn_forward; precision EXACT makes no such copy (dcn_input_copy_bytes is 0) and leaves the buffer alone. */
+size_t dcn_input_copy_bytes(const dcn_problem* p);
+int dcn_forward_keep(const dcn_problem* p, const void* x, const void* offset, const void* weight, const void* bias,
+                     void* y, void* x_channels_last, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Forward pass that allocates nothing and needs no workspace (no counterpart in the reference, which
  * leaves all allocation to its Python layer).  It is for callers that cannot hand over scratch memory:
  * code running where device allocation is forbidden or would stall the pipeline -- an inference plugin's
@@ -152,7 +160,7 @@ int dcn_backward_weight(const dcn_problem* p, const void* x, const void* offset,
  * calls above, EVERY output is OVERWRITTEN: no zero fill by the caller.  The passes share their scratch
  * (workspace of dcn_workspace_bytes(p, DCN_PASS_BACKWARD) bytes).  `x_channels_last`, if not NULL, is the
  * channels-last bf16 copy of x that dcn_forward (precision BF16, same problem, same x) left at the START of
- * its workspace; passing it saves rebuilding it.  It is ignored by the EXACT precision.
+ * its workspace, or dcn_forward_keep in its buffer; passing it saves rebuilding it.  It is ignored by the EXACT precision.
  * Replaces deform_conv_backward_input_offset_cuda + deform_conv_backward_weight_cuda + the Python-side bias
  * gradient (deform3d/deform_conv3d_functions/deform_conv3d_function.py:46-77) as one unit. */
 int dcn_backward(const dcn_problem* p, const void* x, const void* offset, const void* weight, const void* dy,
@@ -191,6 +199,11 @@ int dcn_layer_launch_count(const dcn_problem* p, int pass);
 int dcn_layer_forward(const dcn_problem* p, const void* x, const void* offset_weight, const void* offset_bias,
                       const void* weight, const void* bias, void* offset, void* y, void* workspace,
                       size_t workspace_bytes, void* stream);
+
+/* dcn_layer_forward with the input copy in a buffer of the caller, as dcn_forward_keep. */
+int dcn_layer_forward_keep(const dcn_problem* p, const void* x, const void* offset_weight, const void* offset_bias,
+                           const void* weight, const void* bias, void* offset, void* y, void* x_channels_last,
+                           void* workspace, size_t workspace_bytes, void* stream);
 
 /* Gradients of the layer: dx (through the sampled values AND through the offsets), doffset_weight,
  * doffset_bias, dweight, dbias; any may be NULL, every output is OVERWRITTEN.  The offset gradient itself
