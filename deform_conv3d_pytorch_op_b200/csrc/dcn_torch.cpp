@@ -200,6 +200,18 @@ Tensor scratch(size_t bytes, const Tensor& x) {
     return bytes == 0 ? Tensor() : at::empty({(int64_t)bytes}, x.options().dtype(at::kByte));
 }
 
+// Workspace of a pass.  The exact precision also runs without one, on slower kernels that need no memory beside the tensors:
+// where the allocator has no room for `bytes` the call goes on with the `least` that it cannot do without.
+Tensor workspace(const Problem& q, size_t& bytes, size_t least, const Tensor& x) {
+    if (q.p.precision != DCN_PREC_EXACT) return scratch(bytes, x);
+    try {
+        return scratch(bytes, x);
+    } catch (const c10::OutOfMemoryError&) {
+        bytes = least;
+    }
+    return scratch(bytes, x);
+}
+
 struct CallTensors {
     Tensor x, off, w, b, ow, ob;         // off: kDeform; ow, ob: kLayer
 };
@@ -235,10 +247,10 @@ Tensor run_forward(const Problem& q, Kind kind, CallTensors& t, Tensor* keep) {
         bytes -= copy;
     }
     void* xcl = copy != 0 ? wptr(*keep) : nullptr;
-    const Tensor ws = scratch(bytes, x);
+    if (kind == kLayer) off = at::empty(with_out(q, q.p.N, offset_channels(q)), x.options());
+    const Tensor ws = workspace(q, bytes, 0, x);
     if (kind == kLayer) {
         Range range("dcn_layer_forward");
-        off = at::empty(with_out(q, q.p.N, offset_channels(q)), x.options());
         check(dcn_layer_forward_keep(&q.p, ptr(x), ptr(ow), ptr(ob), ptr(w), ptr(b), wptr(off), wptr(y), xcl, wptr(ws), bytes,
                                      st), "dcn_layer_forward");
         t.off = off;
@@ -267,15 +279,15 @@ void run_backward(const Problem& q, Kind kind, const CallTensors& t, const Tenso
     if (want[kGow]) g[kGow] = at::empty(ow.sizes(), opts);
     if (want[kGob]) g[kGob] = at::empty({offset_channels(q)}, opts);
     if (kind == kLayer) {
-        const size_t bytes = dcn_layer_workspace_bytes(&q.p, DCN_PASS_BACKWARD);
-        const Tensor ws = scratch(bytes, x);
+        size_t bytes = dcn_layer_workspace_bytes(&q.p, DCN_PASS_BACKWARD);
+        const Tensor ws = workspace(q, bytes, (off.nbytes() + 255) / 256 * 256, x);        // (the offset gradient)
         Range range("dcn_layer_backward");
         check(dcn_layer_backward(&q.p, ptr(x), ptr(off), ptr(ow), ptr(w), ptr(dy), ptr(xcl), wptr(g[kGx]), wptr(g[kGow]),
                                  wptr(g[kGob]), wptr(g[kGw]), wptr(g[kGb]), wptr(ws), bytes, stream.stream()),
               "dcn_layer_backward");
     } else {
-        const size_t bytes = dcn_workspace_bytes(&q.p, DCN_PASS_BACKWARD);
-        const Tensor ws = scratch(bytes, x);
+        size_t bytes = dcn_workspace_bytes(&q.p, DCN_PASS_BACKWARD);
+        const Tensor ws = workspace(q, bytes, 0, x);
         Range range("dcn_backward");
         check(dcn_backward(&q.p, ptr(x), ptr(off), ptr(w), ptr(dy), ptr(xcl), wptr(g[kGx]), wptr(g[kGoff]),
                            wptr(g[kGw]), wptr(g[kGb]), wptr(ws), bytes, stream.stream()),

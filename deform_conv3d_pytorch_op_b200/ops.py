@@ -155,12 +155,20 @@ class Op:
         t = torch.empty(tuple(shape), dtype=like.dtype, device=like.device, memory_format=mf)
         return t.zero_() if zero else t
 
-    def _ws(self, which: int):
-        nbytes = _lib.lib().dcn_workspace_bytes(ctypes.byref(self.p), which)
+    def _scratch(self, nbytes: int, least: int = 0):
+        """(workspace, its bytes).  The exact precision also runs without one, on slower kernels: it goes on with the
+        ``least`` that a call cannot do without where the allocator has no room for ``nbytes``."""
         if nbytes == 0:
             return None, 0
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
-        return ws, nbytes
+        try:
+            return torch.empty(nbytes, dtype=torch.uint8, device=self.device), nbytes
+        except torch.OutOfMemoryError:
+            if self.p.precision != _lib.PREC_EXACT or nbytes == least:
+                raise
+        return self._scratch(least, least)
+
+    def _ws(self, which: int):
+        return self._scratch(_lib.lib().dcn_workspace_bytes(ctypes.byref(self.p), which))
 
     def _check_offset(self, offset: torch.Tensor):
         want = (self.N, self.offset_channels) + tuple(self.out_size)
@@ -260,9 +268,8 @@ class Op:
 
     def _layer_ws(self, which: int):
         nbytes = _lib.lib().dcn_layer_workspace_bytes(ctypes.byref(self.p), which)
-        if nbytes == 0:
-            return None, 0
-        return torch.empty(nbytes, dtype=torch.uint8, device=self.device), nbytes
+        doff = self.N * self.offset_channels * int(torch.Size(self.out_size).numel()) * (8 if self.p.dtype else 4)
+        return self._scratch(nbytes, (doff + 255) // 256 * 256 if which == _lib.PASS_BACKWARD else 0)
 
     def layer_forward(self, x, offset_weight, offset_bias, weight, bias=None, keep_workspace: bool = False):
         """offset = conv(x, offset_weight) + offset_bias; y = deform_conv(x, offset, weight) + bias.

@@ -41,3 +41,52 @@ def test_exact_kernels_at_tile_and_segment_edges(case):
         if k == "doff":
             a, b = np.where(mask, 0, a), np.where(mask, 0, b)
         assert cases.rel_err(a, b) <= tol, (case.name, k)
+
+
+@pytest.mark.parametrize("kind", ["deform", "plain", "layer"])
+def test_a_call_without_room_for_its_workspace(kind):
+    """The exact precision needs no workspace: where the allocator has no room for one, a call runs on the kernels that do
+    without.  The room is limited through torch's allocator, to what the outputs take."""
+    import torch
+    import deform_conv3d_pytorch_op_b200 as dcn
+    g = torch.Generator(device="cuda").manual_seed(1)
+    n, c, s = 16, 96, 64                                              # every tensor of note over the 20 MB of a shared segment
+
+    def leaf(*shape, std=1.0):
+        return (torch.randn(shape, generator=g, device="cuda") * std).requires_grad_(True)
+
+    x, w = leaf(n, c, s, s), leaf(c, c, 3, 3, std=0.05)
+    dy = torch.randn((n, c, s, s), generator=g, device="cuda")
+    if kind == "deform":
+        args = [x, leaf(n, 72, s, s), w]
+        fn = lambda: dcn.ConvOffset2dFunction.apply(*args, None, 1, 1, 1, 24, 1)
+    elif kind == "plain":
+        args = [x, w]
+        fn = lambda: dcn.Conv2dFunction.apply(*args, None, 1, 1, 1)
+    else:
+        # offsets of 0.5 with a deviation of 0.06: rounding carries no point over the integer lattice, where values jump
+        args = [x, leaf(72, c, 3, 3, std=0.002), w]
+        half = torch.full((72,), 0.5, device="cuda")
+        fn = lambda: dcn.DeformLayerFunction.apply(x, args[1], half, w, None, 1, 1, 1, 24, 1)
+    y = fn()
+    want = (y.detach(),) + torch.autograd.grad(y, args, dy)
+    del y
+    mb = lambda *ts: sum((t.numel() * 4 + 2097151) // 2097152 * 2097152 for t in ts)
+    offsets = n * 72 * s * s * 4 if kind == "layer" else 0
+    total = torch.cuda.get_device_properties(0).total_memory
+
+    def limit(room):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + room) / total)
+
+    try:
+        limit(mb(x) + offsets + (4 << 20))
+        y = fn()
+        # the gradients, the offset gradient of a layer, and a segment of 20 MB for the small ones
+        limit(mb(*args) + offsets + (24 << 20))
+        got = (y.detach(),) + torch.autograd.grad(y, args, dy)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for a, b in zip(got, want):
+        assert cases.rel_err(a.cpu().numpy(), b.cpu().numpy()) <= 1e-4
