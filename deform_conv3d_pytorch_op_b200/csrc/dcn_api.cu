@@ -398,9 +398,9 @@ size_t dcn_layer_workspace_bytes(const dcn_problem* p, int pass) {
     make_geom(p, g);
     make_geom(&q, gq);
     if (p->precision == DCN_PREC_EXACT) {
-        // both convolutions' passes run one after the other in the same scratch
+        // both convolutions' passes run one after the other in the same scratch, which either of them may want
         size_t scratch = 0;
-        if (exact_worth(p, g)) {
+        if (!dcn::simt_small_layer_supported(g, gq, p->dtype, p->ndim)) {
             const dcn_problem* both[2] = {p, &q};
             for (const dcn_problem* r : both)
                 for (int k = 0; k < 4; ++k)

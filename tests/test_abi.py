@@ -142,3 +142,16 @@ def test_module_surface():
     layer = dcn.DeformLayer3d(8, 16, 3, padding=1, deformable_groups=2)
     assert tuple(layer.conv_offset.weight.shape) == (2 * 27 * 3, 8, 3, 3, 3)
     assert set(layer.state_dict().keys()) == {"conv.weight", "conv.bias", "conv_offset.weight", "conv_offset.bias"}
+
+
+def test_layer_workspace_covers_both_convolutions(L):
+    """EXACT: the offset-producing convolution gets its scratch also where the deformable one wants none (here: a small
+    problem, and a contraction of 18)."""
+    for p in (_lib.make_problem(2, torch.float32, 2, 32, 40, (13, 16), (3, 3), 1, 1, 1, 1, 16),
+              _lib.make_problem(2, torch.float32, 8, 16, 16, (64, 64), (3, 3), 1, 1, 1, 8, 16)):
+        q = _lib.dcn_problem()
+        assert L.dcn_offset_conv_problem(ctypes.byref(p), ctypes.byref(q)) == 0
+        assert L.dcn_workspace_bytes(ctypes.byref(p), _lib.PASS_FORWARD) == 0
+        for layer, passes in ((_lib.PASS_FORWARD, [0]), (_lib.PASS_BACKWARD, [1, 2])):
+            want = max(L.dcn_workspace_bytes(ctypes.byref(q), k) for k in passes)
+            assert 0 < want <= L.dcn_layer_workspace_bytes(ctypes.byref(p), layer)
