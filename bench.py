@@ -55,8 +55,7 @@ NCU_DRAM_BYTES = {
 
 def count_launches(step, declared):
     """Kernels of the library that one step really launches, counted by the profiler (outside every timed region); the
-    library's own figure where the profiler sees none.  It is smaller than that of the separate passes: a backward call
-    that is handed the forward workspace runs its layout passes as one kernel."""
+    library's own figure (dcn_launch_count) where the profiler sees none."""
     from torch.profiler import ProfilerActivity, profile
     try:
         with profile(activities=[ProfilerActivity.CUDA]) as p:

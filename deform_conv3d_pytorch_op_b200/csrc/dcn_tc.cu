@@ -336,20 +336,16 @@ size_t tc_workspace_bytes(const Geom& g, int ndim, int pass) {
     return bwd_weight_workspace(g).total;
 }
 
-// Kernels a pass enqueues when every gradient is wanted (memsets not counted).
+// Kernels a pass enqueues when every gradient of the tensors is wanted (see dcn_launch_count).
 int tc_launch_count(const Geom& g, int ndim, int deform, int pass) {
-    const bool b2 = use_bwd2d(g, ndim, deform);
-    Geom gt;
-    const bool gather = use_gather_dgrad(g, ndim, deform, gt);
     auto folds = [&](const Geom& f, int df) { return fwd_plan(f, fwd_workspace(f).split, ndim, df, nullptr, false).folds() ? 1 : 0; };
+    Geom gt;
     if (pass == 0) return 2 + folds(g, deform);            // prologue, implicit GEMM, (fold of the split tiles)
-    if (pass == 1 && gather) return 2 + folds(gt, 0);
-    if (pass == 1) return b2 || g.cl ? 2 : 3;              // prologue, GEMM + scatter, (dX transpose)
+    if (pass == 1 && use_bwd2d(g, ndim, deform)) return 2; // prologue, GEMM + scatter
+    if (pass == 1 && use_gather_dgrad(g, ndim, deform, gt)) return 2 + folds(gt, 0);
+    if (pass == 1) return g.cl ? 2 : 3;                    // prologue, GEMM + scatter, (dX transpose)
     if (pass == 2) return 3;                               // prologue, implicit GEMM, dW fold
-    // fused backward without the forward pass's workspace: the jobs of the prologue one by one, two GEMMs, epilogue
-    if (b2) return 8;                                      // points, slab tiles, zero fill, dy pack, input copy
-    // (gather: mirrored tiles, dy pack, dy copy, input copy)
-    return 7;                                              // weight tiles, zero fill, dy pack, input copy
+    return 4;                                              // all gradients: prologue, two GEMMs, epilogue
 }
 
 int tc_debug_points(const Geom& g, int ndim, int deform, const float* off, int n, float* coords, int32_t* valid,
@@ -454,8 +450,7 @@ int tc_backward(const Geom& g, int ndim, int deform, const float* x, const float
         p.copy_x(g, x, b.own_xcl());
         b.xcl = b.own_xcl();
     }
-    // (a call on its own launches its passes one by one, as dcn_launch_count states; autograd always hands the copy in)
-    r = p.launch(st, false, xcl_in == nullptr);
+    r = p.launch(st, false);
     if (r == 0) r = b.run(st);
     if (r != 0) return r;
     Passes q;

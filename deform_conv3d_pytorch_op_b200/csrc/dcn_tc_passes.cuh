@@ -641,20 +641,10 @@ public:
         need(32 * 33 * 4);
     }
 
-    // one launch; last: of the call; apart: one launch per job
-    int launch(cudaStream_t st, bool last, bool apart = false) {
+    // one launch; last: of the call
+    int launch(cudaStream_t st, bool last) {
         if (error != 0) return error;
         L.last = last ? 1 : 0;
-        if (apart) {
-            JobList one = L;
-            for (int i = 0; i < L.n; ++i) {
-                one.job[0] = L.job[i];
-                one.n = 1;
-                const int r = submit(one, st);
-                if (r != 0) return r;
-            }
-            return 0;
-        }
         return L.n == 0 ? 0 : submit(L, st);
     }
 

@@ -101,8 +101,9 @@ int dcn_precision_supported(const dcn_problem* p);
  * kernels, and wants none (0) where the problem is too small to gain from it. */
 size_t dcn_workspace_bytes(const dcn_problem* p, int pass);
 
-/* Number of kernel launches `pass` enqueues for this problem (memsets not counted); used by callers
- * that account for launches.  0 on an invalid problem. */
+/* Number of kernels `pass` launches for this problem (memsets not counted) when every gradient but the bias gradient is
+ * wanted and the workspace of dcn_workspace_bytes is there; used by callers that account for launches.  0 on an invalid
+ * problem. */
 int dcn_launch_count(const dcn_problem* p, int pass);
 
 /* y = conv(x sampled at offset, weight) + bias.  `offset` may be NULL when deformable == 0, `bias` may
@@ -186,7 +187,7 @@ int dcn_offset_conv_problem(const dcn_problem* p, dcn_problem* q);
 /* Scratch bytes of dcn_layer_forward (pass = DCN_PASS_FORWARD) / dcn_layer_backward (DCN_PASS_BACKWARD). */
 size_t dcn_layer_workspace_bytes(const dcn_problem* p, int pass);
 
-/* Kernel launches of dcn_layer_forward / dcn_layer_backward when every gradient is wanted (memsets not counted).
+/* Kernel launches of dcn_layer_forward / dcn_layer_backward, counted like those of dcn_launch_count.
  * A small fp32 problem under precision EXACT takes ONE forward launch: the offsets are formed inside the kernel,
  * from the plain patch of the CTA's positions, and stay in shared memory for the sampling that follows (they are
  * written out once, for the backward pass), and a zero-fill launch plus ONE backward launch in which the offset
