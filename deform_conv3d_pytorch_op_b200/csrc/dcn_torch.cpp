@@ -13,6 +13,8 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/DynamicTypes.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
@@ -68,6 +70,8 @@ enum Kind { kDeform, kPlain, kLayer };
 
 struct Spec {                            // what a call says beside its tensors
     Kind kind = kDeform;
+    bool std_rule = false;               // output size under the dilation-aware rule
+    int channels_last = -1;              // -1: as the input is stored
     int ndim = 0;
     int stride[3] = {1, 1, 1}, pad[3] = {0, 0, 0}, dil[3] = {1, 1, 1};
     int64_t cpg = 1, group = 1;
@@ -82,6 +86,8 @@ struct Problem {
     int64_t out[3] = {1, 1, 1};          // the last ndim hold the output size
 };
 
+std::string dtype_name(const Tensor& t) { return std::string("torch.") + torch::getTHPDtype(t.scalar_type())->name; }
+
 std::string lower(std::string s) {
     for (char& c : s) c = (char)tolower((unsigned char)c);
     return s;
@@ -93,7 +99,7 @@ void fill_problem(dcn_problem& p, const Spec& s, const Tensor& x, const Tensor& 
     p.dtype = x.scalar_type() == at::kDouble ? DCN_F64 : DCN_F32;
     p.precision = precision;
     p.deformable = s.kind != kPlain;
-    p.std_size_rule = s.kind == kPlain;
+    p.std_size_rule = s.std_rule ? 1 : 0;
     if (s.oob >= 0) {
         p.oob_offset_grad = s.oob;
     } else {
@@ -120,10 +126,10 @@ Problem make_problem(const Spec& s, const Tensor& x, const Tensor& w) {
     if (w.dim() != s.ndim + 2) fail("kernel dim");
     if (x.size(1) != w.size(1) * s.group) fail("input c != kernel c");
     if (x.scalar_type() != at::kFloat && x.scalar_type() != at::kDouble)
-        fail(std::string("tensors must be float32 or float64, got ") + c10::toString(x.scalar_type()));
+        fail("tensors must be float32 or float64, got " + dtype_name(x));
     Problem r;
     const at::MemoryFormat cl_format = s.ndim == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d;
-    const bool cl = !x.is_contiguous() && x.is_contiguous(cl_format);
+    const bool cl = s.channels_last < 0 ? !x.is_contiguous() && x.is_contiguous(cl_format) : s.channels_last != 0;
     std::string prec = s.precision;
     if (prec.empty()) {
         const char* e = getenv("DCN_PRECISION");
@@ -169,8 +175,7 @@ Tensor prep(const Tensor& t, const char* name, const Tensor& x, at::MemoryFormat
     if (t.device() != x.device())
         fail(std::string(name) + " is on " + t.device().str() + " but input is on " + x.device().str());
     if (t.scalar_type() != x.scalar_type())
-        fail(std::string(name) + " has dtype " + c10::toString(t.scalar_type()) + " but input has " +
-             c10::toString(x.scalar_type()));
+        fail(std::string(name) + " has dtype " + dtype_name(t) + " but input has " + dtype_name(x));
     return t.is_contiguous(format) ? t : t.contiguous(format);
 }
 
@@ -523,6 +528,7 @@ PyObject* conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return entry([&](Spec& s, CallTensors& t) {
         count_arg(n, 2, 8);
         s.kind = kPlain;
+        s.std_rule = true;
         s.ndim = ND;
         t.x = tensor_arg(a[0], "inputs");
         t.w = tensor_arg(a[1], "weight");
@@ -558,6 +564,36 @@ PyObject* deform_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
+// The dcn_problem of a call, as bytes: every check and rule on sizes, types, precision and storage that the Functions apply,
+// for ops.py.  (x, weight, stride, padding, dilation, channel_per_group, group, deformable, std_size_rule, oob_offset_grad,
+// precision, channels_last); the last three may be None
+PyObject* problem(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    try {
+        count_arg(n, 12, 12);
+        const Tensor x = tensor_arg(a[0], "x"), w = tensor_arg(a[1], "weight");
+        Spec s;
+        s.ndim = (int)x.dim() - 2;
+        if (s.ndim != 2 && s.ndim != 3) fail("input dim");
+        axes_arg(a[2], s.ndim, s.stride);
+        axes_arg(a[3], s.ndim, s.pad);
+        axes_arg(a[4], s.ndim, s.dil);
+        s.cpg = small_int(int_arg(a[5]));
+        s.group = small_int(int_arg(a[6]));
+        s.kind = PyObject_IsTrue(a[7]) ? kDeform : kPlain;
+        s.std_rule = PyObject_IsTrue(a[8]) != 0;
+        oob_arg(a[9], s);
+        precision_arg(a[10], s);
+        if (a[11] != Py_None) s.channels_last = PyObject_IsTrue(a[11]);
+        const Problem q = make_problem(s, x, w);
+        return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(&q.p), sizeof(q.p));
+    } catch (const DcnFailure& e) {
+        PyErr_SetString(g_error, e.text.c_str());
+        return nullptr;
+    }
+    END_HANDLE_TH_ERRORS
+}
+
 PyObject* set_error(PyObject*, PyObject* cls) {
     Py_INCREF(cls);
     Py_XDECREF(g_error);
@@ -572,6 +608,7 @@ PyMethodDef methods[] = {
     {"conv2d", DCN_FAST(conv<2>), nullptr},
     {"conv3d", DCN_FAST(conv<3>), nullptr},
     {"deform_layer", DCN_FAST(deform_layer), nullptr},
+    {"problem", DCN_FAST(problem), nullptr},
     {"set_error", set_error, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

@@ -16,9 +16,6 @@ import torch
 from . import _lib
 from ._lib import DcnError
 
-_PRECISIONS = {"exact": _lib.PREC_EXACT, "fp32": _lib.PREC_EXACT, "bf16": _lib.PREC_BF16}
-
-
 def default_precision() -> str:
     """``DCN_PRECISION`` = exact | bf16 | auto (default exact: compute in the tensor dtype)."""
     return os.environ.get("DCN_PRECISION", "exact").lower()
@@ -67,7 +64,8 @@ class _Range:
         return False
 
 
-def _prep(t: Optional[torch.Tensor], name: str, ref: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+def _prep(t: Optional[torch.Tensor], name: str, ref: Optional[torch.Tensor] = None,
+          memory_format: torch.memory_format = torch.contiguous_format) -> Optional[torch.Tensor]:
     if t is None:
         return None
     if not t.is_cuda:
@@ -77,7 +75,7 @@ def _prep(t: Optional[torch.Tensor], name: str, ref: Optional[torch.Tensor] = No
             raise DcnError("%s is on %s but input is on %s" % (name, t.device, ref.device))
         if t.dtype != ref.dtype:
             raise DcnError("%s has dtype %s but input has %s" % (name, t.dtype, ref.dtype))
-    return t.contiguous()
+    return t.contiguous(memory_format=memory_format)
 
 
 class Op:
@@ -87,49 +85,17 @@ class Op:
                  group: int, deformable: bool = True, std_size_rule: bool = False,
                  oob_offset_grad: Optional[bool] = None, precision: Optional[str] = None,
                  channels_last: Optional[bool] = None):
-        ndim = x.dim() - 2
-        if ndim not in (2, 3):
-            raise DcnError("input dim")                       # reference: check(input_dim == 5, "input dim")
-        if weight.dim() != ndim + 2:
-            raise DcnError("kernel dim")
-        if x.size(1) != weight.size(1) * group:
-            raise DcnError("input c != kernel c")
-        self.ndim = ndim
+        # Checks, the `auto` rule and the storage order are those of the autograd Functions (csrc/dcn_torch.cpp).
+        # (precision None: default_precision(); oob_offset_grad None: default_oob_offset_grad()).  Channels-last activations (torch.channels_last / channels_last_3d storage) are taken and produced as
+        # they are by the bf16 path: no layout pass around the kernels.  Default: follow the input's memory format.
+        p = _lib.dcn_problem.from_buffer_copy(_lib.native().problem(
+            x, weight, *[v if isinstance(v, int) else tuple(int(a) for a in v) for v in (stride, padding, dilation)],
+            int(channel_per_group), int(group), deformable, std_size_rule, oob_offset_grad, precision, channels_last))
+        ndim = self.ndim = p.ndim
         self.device = x.device
         self.dtype = x.dtype
-        prec = (precision or default_precision()).lower()
-        if oob_offset_grad is None:
-            oob_offset_grad = default_oob_offset_grad()
-        cpg = channel_per_group if deformable else x.size(1)
-        # Channels-last activations (torch.channels_last / channels_last_3d storage) are taken and produced as they
-        # are by the bf16 path: no layout pass around the kernels.  Default: follow the input's memory format.
+        cpg = p.cpg
         self.memory_format = torch.channels_last if ndim == 2 else torch.channels_last_3d
-        if channels_last is None:
-            channels_last = (not x.is_contiguous()) and x.is_contiguous(memory_format=self.memory_format)
-        mk = lambda pr: _lib.make_problem(ndim, x.dtype, x.size(0), x.size(1), weight.size(0), tuple(x.shape[2:]),
-                                          tuple(weight.shape[2:]), stride, padding, dilation, group, cpg,
-                                          deformable, std_size_rule, oob_offset_grad, pr,
-                                          channels_last and pr == _lib.PREC_BF16)
-        if prec == "auto":
-            # bf16 tensor-core path where the shape allows it and the problem is big enough to pay for its
-            # layout pre-passes (ten launches per step against three of the exact path)
-            kvol = int(torch.Size(weight.shape[2:]).numel())
-            out_guess = 1
-            for i, k_, s_, p_ in zip(x.shape[2:], weight.shape[2:], _lib._triple(stride, ndim, 1)[3 - ndim:],
-                                     _lib._triple(padding, ndim, 0)[3 - ndim:]):
-                out_guess *= max(1, (i + 2 * p_ - k_) // s_ + 1)
-            flops_per_pass = 2.0 * x.size(0) * weight.size(0) * weight.size(1) * kvol * out_guess
-            p = mk(_lib.PREC_BF16) if (x.dtype == torch.float32 and flops_per_pass >= 1e8) else None
-            if p is None or not _lib.lib().dcn_precision_supported(ctypes.byref(p)):
-                p = mk(_lib.PREC_EXACT)
-        elif prec in _PRECISIONS:
-            p = mk(_PRECISIONS[prec])
-        else:
-            raise DcnError("unknown precision %r (exact | bf16 | auto)" % prec)
-        _lib.check(_lib.lib().dcn_validate(ctypes.byref(p)), "shape check")
-        if not _lib.lib().dcn_precision_supported(ctypes.byref(p)):
-            raise DcnError("precision %r is not available for this problem (needs float32 tensors and channel "
-                           "counts per group that are multiples of 8); there is no silent fallback" % prec)
         self.p = p
         self.channels_last = bool(p.channels_last)
         self.deformable = deformable
@@ -141,14 +107,7 @@ class Op:
     # -- helpers ---------------------------------------------------------------------------------
     def _act(self, t: Optional[torch.Tensor], name: str, ref: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
         """An activation-like tensor (input, output gradient) in the storage order the problem was built for."""
-        t = _prep(t, name, ref) if not self.channels_last else t
-        if t is None or not self.channels_last:
-            return t
-        if not t.is_cuda:
-            raise DcnError("%s must be a CUDA tensor (there is no CPU implementation)" % name)
-        if ref is not None and (t.device != ref.device or t.dtype != ref.dtype):
-            raise DcnError("%s does not match the input's device / dtype" % name)
-        return t.contiguous(memory_format=self.memory_format)
+        return _prep(t, name, ref, self.memory_format if self.channels_last else torch.contiguous_format)
 
     def _new_act(self, shape, like: torch.Tensor, zero: bool = False) -> torch.Tensor:
         mf = self.memory_format if self.channels_last else torch.contiguous_format

@@ -156,3 +156,30 @@ def test_layer_workspace_covers_both_convolutions(L):
         for layer, passes in ((_lib.PASS_FORWARD, [0]), (_lib.PASS_BACKWARD, [1, 2])):
             want = max(L.dcn_workspace_bytes(ctypes.byref(q), k) for k in passes)
             assert 0 < want <= L.dcn_layer_workspace_bytes(ctypes.byref(p), layer)
+
+
+def test_both_host_paths_apply_the_same_checks(monkeypatch):
+    """Op and the autograd Functions refuse the same calls with the same words, and choose the same precision."""
+    import deform_conv3d_pytorch_op_b200 as dcn
+    x, w = torch.zeros(2, 8, 9, 9), torch.zeros(6, 4, 3, 3)
+    bad = [dict(x=torch.zeros(2, 8, 9)), dict(w=torch.zeros(6, 4, 3, 3, 3)), dict(w=torch.zeros(6, 3, 3, 3)),
+           dict(x=x.half(), w=w.half()), dict(stride=(1, 1, 1)), dict(group=4, w=torch.zeros(6, 2, 3, 3)), dict(cpg=3),
+           dict(stride=0), dict(pad=-1), dict(precision="fp8"), dict(precision="bf16")]
+    for change in bad:
+        a = dict(dict(x=x, w=w, stride=1, pad=1, dil=1, cpg=4, group=2, precision=None), **change)
+        texts = []
+        for call in (lambda: dcn.Op(a["x"], a["w"], a["stride"], a["pad"], a["dil"], a["cpg"], a["group"], precision=a["precision"]),
+                     lambda: dcn.ConvOffset2dFunction.apply(a["x"], torch.zeros(2, 36, 9, 9), a["w"], None, a["stride"],
+                                                            a["pad"], a["dil"], a["cpg"], a["group"], a["precision"])):
+            with pytest.raises(RuntimeError) as e:
+                call()
+            texts.append(str(e.value))
+        assert texts[0] == texts[1], change
+    big, wide = torch.zeros(4, 64, 32, 32), torch.zeros(64, 64, 3, 3)
+    for precision, want in (("auto", _lib.PREC_BF16), ("exact", _lib.PREC_EXACT), (None, _lib.PREC_EXACT)):
+        assert dcn.Op(big, wide, 1, 1, 1, 64, 1, precision=precision).p.precision == want
+    assert dcn.Op(x, w, 1, 1, 1, 4, 2, precision="auto").p.precision == _lib.PREC_EXACT
+    monkeypatch.setenv("DCN_PRECISION", "bf16")
+    assert dcn.Op(big, wide, 1, 1, 1, 64, 1).p.precision == _lib.PREC_BF16
+    assert dcn.Op(big.contiguous(memory_format=torch.channels_last), wide, 1, 1, 1, 64, 1).channels_last
+    assert not dcn.Op(big.contiguous(memory_format=torch.channels_last), wide, 1, 1, 1, 64, 1, channels_last=False).channels_last

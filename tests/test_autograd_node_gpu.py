@@ -98,3 +98,20 @@ def test_what_stays_allocated_until_the_backward_pass(kind, precision):
     tol = 1e-4 if precision == "exact" else 2e-2
     for a, b in zip(torch.autograd.grad(y.square().sum(), args), want):
         assert torch.allclose(a, b, rtol=tol, atol=tol * float(b.abs().max()))
+
+
+@pytest.mark.parametrize("precision", ["exact", "bf16"])
+def test_tensors_that_do_not_match_are_refused_alike(precision):
+    import deform_conv3d_pytorch_op_b200 as dcn
+    x, w, off = torch.zeros(2, 16, 9, 9).cuda(), torch.zeros(16, 16, 3, 3).cuda(), torch.zeros(2, 18, 9, 9).cuda()
+    for fmt in (torch.contiguous_format, torch.channels_last):
+        xf = x.contiguous(memory_format=fmt)
+        op = dcn.Op(xf, w, 1, 1, 1, 16, 1, precision=precision)
+        for o, u in ((off.double(), w), (off.cpu(), w), (off[:, :9], w), (off, w.double()), (off, w.cpu())):
+            texts = []
+            for call in (lambda: op.forward(xf, o, u),
+                         lambda: dcn.ConvOffset2dFunction.apply(xf, o, u, None, 1, 1, 1, 16, 1, precision)):
+                with pytest.raises(dcn.DcnError) as e:
+                    call()
+                texts.append(str(e.value))
+            assert texts[0] == texts[1]
