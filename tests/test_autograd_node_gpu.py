@@ -115,3 +115,91 @@ def test_tensors_that_do_not_match_are_refused_alike(precision):
                     call()
                 texts.append(str(e.value))
             assert texts[0] == texts[1]
+
+
+def test_a_second_backward_pass():
+    for kind in KINDS:
+        fn, args = _make(kind)
+        y = fn(*args)
+        dy = torch.randn_like(y)
+        first = torch.autograd.grad(y, args, dy, retain_graph=True)
+        for a, b in zip(torch.autograd.grad(y, args, dy), first):
+            assert _close(a, b)
+        with pytest.raises(RuntimeError, match="second time"):
+            torch.autograd.grad(y, args, dy)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_gradients_of_gradients_are_refused(kind):
+    fn, args = _make(kind)
+    y = fn(*args)
+    dy = torch.ones_like(y, requires_grad=True)
+    g = torch.autograd.grad(y, args, dy, create_graph=True)
+    assert all(v.requires_grad for v in g)
+    with pytest.raises(RuntimeError, match="once_differentiable"):
+        sum(v.sum() for v in g).backward()
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_change_in_place_before_the_backward_pass_is_refused(kind):
+    for i in range(len(_make(kind)[1]) - 1):                         # the last is the bias, which the gradients do not read
+        fn, args = _make(kind)
+        if kind == "layer" and i == 2:                               # (so is the offset-producing convolution's)
+            continue
+        y = fn(*args)
+        with torch.no_grad():
+            args[i].mul_(2)
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            y.sum().backward()
+
+
+@pytest.mark.parametrize("precision", ["exact", "bf16"])
+@pytest.mark.parametrize("kind", KINDS)
+def test_gradients_for_some_inputs_only(kind, precision):
+    fn, args = _make(kind, precision)
+    y = fn(*args)
+    dy = torch.randn_like(y)
+    want = torch.autograd.grad(y, args, dy)
+    tol = 1e-4 if precision == "exact" else 2e-2
+    for mask in range(1, 2 ** len(args)):
+        some = [a.detach().requires_grad_(bool(mask >> i & 1)) for i, a in enumerate(args)]
+        got = torch.autograd.grad(fn(*some), [a for a in some if a.requires_grad], dy)
+        for a, b in zip(got, [b for i, b in enumerate(want) if mask >> i & 1]):
+            assert torch.allclose(a, b, rtol=tol, atol=tol * float(b.abs().max())), mask
+    with torch.no_grad():
+        assert fn(*args).grad_fn is None
+
+
+@pytest.mark.parametrize("precision", ["exact", "bf16"])
+def test_threads_with_streams_of_their_own(precision):
+    """Four threads, each on its own stream, run steps of a layer and of the operator at the same time."""
+    import threading
+    made = [_make(kind, precision) for kind in ("deform", "layer", "plain", "deform")]
+    want = []
+    for fn, args in made:
+        y = fn(*args)
+        want.append((y.detach(),) + torch.autograd.grad(y, args, torch.ones_like(y)))
+    torch.cuda.synchronize()
+    got, errors = [None] * len(made), []
+
+    def work(i):
+        try:
+            fn, args = made[i]
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(20):
+                    y = fn(*args)
+                    g = torch.autograd.grad(y, args, torch.ones_like(y))
+                torch.cuda.current_stream().synchronize()
+                got[i] = (y.detach(),) + g
+        except Exception as e:                                       # handed to the test's own thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(made))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    tol = 1e-4 if precision == "exact" else 2e-2
+    for a, b in zip(sum(got, ()), sum(want, ())):
+        assert torch.allclose(a, b, rtol=tol, atol=tol * float(b.abs().max()))
