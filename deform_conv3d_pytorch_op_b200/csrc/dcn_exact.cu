@@ -1246,12 +1246,6 @@ exact_fold_kernel(const Geom g, const ExactGeom xg, const FoldArgs<T> a) {
 // ------------------------------------------------------------------------------------------------------------------
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
-int sm_count() {
-    int dev = 0, n = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 148;
-}
-
 // channels of a vector: 16 bytes' worth, except where a segment is so short that most of the vector would be padding
 int vec_width(const Geom& g, int dtype, int S) {
     (void)g;

@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "dcn_common.cuh"
 
 namespace dcn {
@@ -14,6 +16,21 @@ namespace dcn {
 inline bool pdl_enabled() {
     static const bool off = [] { const char* e = getenv("DCN_PDL"); return e != nullptr && e[0] == '0'; }();
     return !off;
+}
+
+// SMs of the current device, asked for once per device (148 where there is none to ask: sizes are also computed on hosts
+// without a GPU).
+inline int sm_count() {
+    constexpr int kMaxDevices = 64;
+    static std::atomic<int> count_of_device[kMaxDevices];
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
+    int n = count_of_device[dev];
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+        count_of_device[dev] = n;              // racing first calls find the same number
+    }
+    return n;
 }
 
 // Launch of a kernel that calls pdl_wait() before it reads or writes global memory (see dcn_common.cuh).

@@ -560,10 +560,7 @@ int launch_backward_data(const Geom& g, const void* x, const void* off, const vo
 inline void weight_grid(const Geom& g, dim3& grid, int& cps, int bm = 64) {
     const long long chunks = (g.P + 15) / 16;
     const long long tiles = (long long)((g.Kg + 63) / 64) * g.G * ((g.Og + bm - 1) / bm);
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms < 1) sms = 148;
-    long long splits = ((long long)sms * 8 + tiles - 1) / tiles;      // ~8 CTAs per SM overall, >= 8 chunks per split
+    long long splits = (sm_count() * 8ll + tiles - 1) / tiles;      // ~8 CTAs per SM overall, >= 8 chunks per split
     if (splits > chunks / 8) splits = chunks / 8;
     if (splits < 1) splits = 1;
     if (splits > 65535) splits = 65535;

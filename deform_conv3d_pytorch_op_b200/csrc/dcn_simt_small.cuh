@@ -514,7 +514,7 @@ inline bool small_supported(const Geom& g, int dtype, int ndim, int deform) {
     if (macs > (lg < 0 ? 33554432.0 : (double)(1ull << (lg > 40 ? 40 : lg)))) return false;
     const SmallDims d = small_dims(g, ndim);
     if (lg < 0) {
-        const long long ctas = (g.P + d.TP - 1) / d.TP * g.G, waves = (ctas + 147) / 148;
+        const long long ctas = (g.P + d.TP - 1) / d.TP * g.G, sms = sm_count(), waves = (ctas + sms - 1) / sms;
         if ((double)waves * (25e3 + macs / (double)ctas) > 110e3) return false;
     }
     return d.smem_bwd <= 96 * 1024 && d.smem_fwd <= 96 * 1024;

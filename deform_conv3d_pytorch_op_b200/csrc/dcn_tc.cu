@@ -92,19 +92,6 @@ __device__ __forceinline__ uint4 sample_chunk(const Geom& g, const __nv_bfloat16
                       pack_bf16x2(acc[6], acc[7]));
 }
 
-int sm_count() {
-    constexpr int kMaxDevices = 64;
-    static volatile int count_of_device[kMaxDevices] = {};
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
-    int n = count_of_device[dev];
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
-        count_of_device[dev] = n;              // racing first calls find the same number
-    }
-    return n;
-}
-
 #include "dcn_tc_passes.cuh"
 #include "dcn_tc_fwd_direct.cuh"
 #include "dcn_tc_sampler.cuh"
