@@ -197,7 +197,15 @@ size_t gather_dgrad_bytes(const Geom& g) {
 }
 
 // The shared-memory-accumulating backward-data kernel is taken whenever it fits (DCN_BWD2D=0 forces the
-// global-reduction kernels, for A/B measurements).
+// global-reduction kernels, for A/B measurements): its dX is a fixed-point sum that does not depend on the order of its
+// terms, the other's is added up by reductions in whichever order they arrive.  It is the faster one where its items (one
+// sample x eight channels, a whole plane on one SM) fill the SMs, and not where they are few or the planes tiny.  Backward
+// data of n x c -> c channels, 3x3, one deformable group, B200, kernel time plane / reductions in us:
+//   8 items    1 x 64:  14x14 11 / 18, 28x28 26 / 19, 56x56 84 / 20       32 items   2 x 128: 28x28 27 / 20, 56x56 88 / 35
+//   64 items   4 x 128, 56x56 87 / 63; 8 x 64, 56x56 84 / 65              128 items  4 x 256: 14x14 14 / 22, 28x28 31 / 40
+//   256 items  8 x 256, 28x28 56 / 54; 32 x 64, 56x56 165 / 209           512 items  16 x 256, 14x14 40 / 39
+//   1024 items 32 x 256: 14x14 66 / 52, 56x56 (four groups) 626 / 760
+// (about 5 us + 25 ns a position for each wave of items against 15 us + 3.4 ps a sample of C x taps x positions).
 bool use_bwd2d(const Geom& g, int ndim, int deform) {
     static const bool off = [] { const char* e = getenv("DCN_BWD2D"); return e != nullptr && e[0] == '0'; }();
     return !off && b2_supported(g, ndim, deform);
