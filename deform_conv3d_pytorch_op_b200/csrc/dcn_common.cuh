@@ -48,6 +48,68 @@ struct FastDiv {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Loads of such kernels.  What they read may still be in the making when they become resident: by the kernel before them in
+// the call or, in a call's first kernel, by the one before the call.  __ldg and loads through const __restrict__ pointers
+// (ld.global.nc) state that the data does not change while the kernel is resident, and may be moved above pdl_wait(); a
+// point entry read that early was a wild corner address.  These are ordinary loads that stay behind it.
+__device__ __forceinline__ float gload(const float* p) {
+    float r;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ double gload(const double* p) {
+    double r;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ uint32_t gload(const uint32_t* p) {
+    uint32_t r;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ uint2 gload(const uint2* p) {
+    uint2 r;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ uint4 gload(const uint4* p) {
+    uint4 r;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+// past L1: written by other CTAs of the same kernel
+__device__ __forceinline__ uint4 gload_cg(const uint4* p) {
+    uint4 r;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+    return r;
+}
+__device__ __forceinline__ float2 gload(const float2* p) {
+    float2 r;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float4 gload(const float4* p) {
+    float4 r;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ uint2 gload_if(bool ok, const uint2* p) {
+    uint2 r;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\t"
+                 "@q ld.global.v2.u32 {%0, %1}, [%2];\n\t}"
+                 : "=&r"(r.x), "=&r"(r.y) : "l"(p), "r"((uint32_t)ok));
+    return r;
+}
+// ... of 16 bytes where `ok`, else zeros (one predicated load, no branch)
+__device__ __forceinline__ uint4 gload_if(bool ok, const uint4* p) {
+    uint4 r;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+                 "mov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+                 "@q ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+                 : "=&r"(r.x), "=&r"(r.y), "=&r"(r.z), "=&r"(r.w) : "l"(p), "r"((uint32_t)ok));
+    return r;
+}
+
 // Problem geometry as the kernels see it.  Axis order is (l, h, w); 2-D problems keep a unit l axis.
 struct Geom {
     int N, C, O, G, cpg, dg;
@@ -158,7 +220,7 @@ __device__ __forceinline__ void locate(const Geom& g, const T* __restrict__ off_
     const T* ob = offset_ptr<T, D>(g, off_n, grp, tap, op);
     T offv[D];
 #pragma unroll
-    for (int a = 0; a < D; ++a) offv[a] = __ldg(ob + (size_t)a * g.ov);
+    for (int a = 0; a < D; ++a) offv[a] = gload(ob + (size_t)a * g.ov);
     locate_with<T, D>(g, offv, tap, op, s);
 }
 

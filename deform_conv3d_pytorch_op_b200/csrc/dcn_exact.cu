@@ -51,11 +51,11 @@ template <typename T, int V>
 __device__ __forceinline__ Vec<T, V> load_vec(const T* p) {
     Vec<T, V> r;
     if constexpr (V * sizeof(T) == 16) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+        const uint4 q = gload(reinterpret_cast<const uint4*>(p));
         memcpy(&r, &q, 16);
     } else {
 #pragma unroll
-        for (int i = 0; i < V; ++i) r.v[i] = __ldg(p + i);
+        for (int i = 0; i < V; ++i) r.v[i] = gload(p + i);
     }
     return r;
 }
@@ -115,7 +115,7 @@ __device__ __forceinline__ Entry<T> load_entry(const Entry<T>* p) {
     const uint4* q = reinterpret_cast<const uint4*>(p);
     uint4 t[sizeof(Entry<T>) / 16];
 #pragma unroll
-    for (int i = 0; i < (int)(sizeof(Entry<T>) / 16); ++i) t[i] = __ldg(q + i);
+    for (int i = 0; i < (int)(sizeof(Entry<T>) / 16); ++i) t[i] = gload(q + i);
     memcpy(&e, t, sizeof(e));
     return e;
 }
@@ -418,7 +418,7 @@ exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
         for (long long i = threadIdx.x; i < g.P; i += kXThreads) {
             uint32_t n, opos;
             g.d_ov.divmod((uint32_t)i, n, opos);
-            s += __ldg(a.dy + ((size_t)n * g.O + b) * g.ov + opos);
+            s += gload(a.dy + ((size_t)n * g.O + b) * g.ov + opos);
         }
         T* red = &tile[0][0];
         red[threadIdx.x] = s;
@@ -447,7 +447,7 @@ exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
 #pragma unroll
             for (int h = 0; h < TC / 32; ++h) {
                 const int p = p0 + h * 32 + tx;
-                v[i][h] = ok && p < g.iv ? __ldg(xc + p) : (T)0;
+                v[i][h] = ok && p < g.iv ? gload(xc + p) : (T)0;
             }
         }
 #pragma unroll
@@ -481,7 +481,7 @@ exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
             op[i] = decompose_pos(g, P < g.P ? P : 0);
             const T* ob = offset_ptr<T, D>(g, offset_block<T, D>(g, a.off, op[i].n), (int)grp, (int)tap, op[i]);
 #pragma unroll
-            for (int d = 0; d < D; ++d) offv[i][d] = __ldg(ob + (size_t)d * g.ov);
+            for (int d = 0; d < D; ++d) offv[i][d] = gload(ob + (size_t)d * g.ov);
         }
 #pragma unroll
         for (int i = 0; i < kPtsPerThread; ++i) {
@@ -510,7 +510,7 @@ exact_prep_kernel(const Geom g, const ExactGeom xg, const PrepArgs<T> a) {
                 uint32_t tap, c4, seg, r4;
                 xg.d_Cg4.divmod(kp, tap, c4);
                 xg.d_S4.divmod(c4, seg, r4);
-                if ((int)r4 < xg.S) v = __ldg(a.w + ((size_t)(j * g.Og + o) * g.Cg + seg * xg.S + r4) * g.kv + tap);
+                if ((int)r4 < xg.S) v = gload(a.w + ((size_t)(j * g.Og + o) * g.Cg + seg * xg.S + r4) * g.kv + tap);
             }
             a.wk[e] = v;
         }
@@ -606,7 +606,7 @@ __device__ __forceinline__ bool fold_parts(Acc<T, TM, TN>& acc, T* slices, unsig
     for (unsigned z = 0; z < gridDim.z; ++z, all += TM * TN * NT) {
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-            const uint4 q = __ldcg(reinterpret_cast<const uint4*>(all + e * (NT * W)));
+            const uint4 q = gload_cg(reinterpret_cast<const uint4*>(all + e * (NT * W)));
             T t[W];
             memcpy(t, &q, 16);
 #pragma unroll
@@ -779,7 +779,7 @@ exact_forward_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl
             const int ol = o0 + ty * TM + i;
             if (ol >= g.Og) break;
             const int o = j * g.Og + ol;
-            const T bv = bias != nullptr ? __ldg(bias + o) : (T)0;
+            const T bv = bias != nullptr ? gload(bias + o) : (T)0;
             if (vec) {
                 *reinterpret_cast<float4*>(y + ((size_t)n * g.O + o) * g.ov + opos) =
                     make_float4((float)(acc.at(i, 4 * h) + bv), (float)(acc.at(i, 4 * h + 1) + bv),
@@ -884,7 +884,7 @@ exact_weight_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl,
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
             const int o = o0 + tid / kBK + i * TY;
-            dv[i] = (P < g.P && o < g.Og) ? __ldg(src + (size_t)o * g.ov) : (T)0;
+            dv[i] = (P < g.P && o < g.Og) ? gload(src + (size_t)o * g.ov) : (T)0;
         }
     };
     auto store_dy = [&](int buf) {
@@ -1017,7 +1017,7 @@ exact_data_kernel(const Geom g, const ExactGeom xg, const T* __restrict__ xcl, c
 #pragma unroll
         for (int i = 0; i < DY; ++i) {
             const int o = ch * kBK + tid / BN + i * (kXThreads / BN);
-            dv[i] = (Pb < g.P && o < g.Og) ? __ldg(dyb + (size_t)o * g.ov) : (T)0;
+            dv[i] = (Pb < g.P && o < g.Og) ? gload(dyb + (size_t)o * g.ov) : (T)0;
         }
     };
     auto store = [&](int ch) {
@@ -1200,7 +1200,7 @@ exact_fold_kernel(const Geom g, const ExactGeom xg, const FoldArgs<T> a) {
 #pragma unroll
             for (int h = 0; h < TC / 32; ++h) {
                 const int c4 = c0 + h * 32 + tx;
-                v[i][h] = (p < g.iv && c4 < xg.C4) ? __ldg(in + (size_t)p * xg.C4 + c4) : (T)0;
+                v[i][h] = (p < g.iv && c4 < xg.C4) ? gload(in + (size_t)p * xg.C4 + c4) : (T)0;
             }
         }
 #pragma unroll
@@ -1236,7 +1236,7 @@ exact_fold_kernel(const Geom g, const ExactGeom xg, const FoldArgs<T> a) {
     const T* src = a.dwp + (size_t)o * xg.Kp64 + kp;
     T s = (T)0;
 #pragma unroll 4
-    for (int i = 0; i < a.slices; ++i) s += __ldg(src + i * step);
+    for (int i = 0; i < a.slices; ++i) s += gload(src + i * step);
     T* dst = a.dw + ((size_t)o * g.Cg + seg * xg.S + r4) * g.kv + tap;
     *dst = a.add ? *dst + s : s;
 }

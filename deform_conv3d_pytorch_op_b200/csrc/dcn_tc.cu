@@ -64,7 +64,7 @@ __device__ __forceinline__ uint4 sample_chunk(const Geom& g, const __nv_bfloat16
     if (!DEFORM) {
         int idx;
         if (!locate_plain<D>(g, tap, op, idx)) return make_uint4(0, 0, 0, 0);
-        return __ldg(static_cast<const uint4*>(ptr_mad_u32(xn, (uint32_t)idx, pix_bytes)));
+        return gload(static_cast<const uint4*>(ptr_mad_u32(xn, (uint32_t)idx, pix_bytes)));
     }
     Pt<float, D> s;
     locate<float, D>(g, offset_block<float, D>(g, off, op.n), grp, tap, op, s);
@@ -75,7 +75,7 @@ __device__ __forceinline__ uint4 sample_chunk(const Geom& g, const __nv_bfloat16
     corner_weights<float, D>(s, cw);
     uint4 q[1 << D];
 #pragma unroll
-    for (int e = 0; e < (1 << D); ++e) q[e] = __ldg(static_cast<const uint4*>(ptr_mad_u32(xn, (uint32_t)idx[e], pix_bytes)));
+    for (int e = 0; e < (1 << D); ++e) q[e] = gload(static_cast<const uint4*>(ptr_mad_u32(xn, (uint32_t)idx[e], pix_bytes)));
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.f;

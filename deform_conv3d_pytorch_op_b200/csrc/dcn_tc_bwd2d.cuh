@@ -304,7 +304,7 @@ tc_bwd2d_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const uint4
 
         // fixed-point scale: one term |w * col| <= 4 * Og * max|dy| * max|W| (corner weights reach 2 per axis in the
         // one-pixel border band, where the low weight is 1 - lw with lw in (-1, 0))
-        const float bound = (float)g.Og * __uint_as_float(scale_bits[0]) * __uint_as_float(scale_bits[1]) * 1.01f;
+        const float bound = (float)g.Og * __uint_as_float(gload(scale_bits)) * __uint_as_float(gload(scale_bits + 1)) * 1.01f;
         const int ex = (int)((__float_as_uint(bound) >> 23) & 0xffu) - 127;            // bound < 2^(ex + 1)
         float fx_scale, fx_inv;
         if (!(bound < 3.0e38f)) {                       // inf or NaN in dy / W: poison dX like fp32 arithmetic would
@@ -346,8 +346,7 @@ tc_bwd2d_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const uint4
 #pragma unroll
                 for (int u = 0; u < TG; ++u) {
                     const int tap = tg + WQ * u;
-                    ent[u] = (in && (FULL || tap < g.kv)) ? __ldg(pts_n + (uint32_t)tap * (uint32_t)g.ov + (uint32_t)(P - pbeg))
-                                                : make_uint4(0u, 0u, 0u, 0u);
+                    ent[u] = gload_if(in && (FULL || tap < g.kv), pts_n + (uint32_t)tap * (uint32_t)g.ov + (uint32_t)(P - pbeg));
                 }
             };
             fetch_points(Pfirst, (kq + (int)tl) % WQ);
@@ -362,11 +361,18 @@ tc_bwd2d_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const uint4
             }
             if (want_off) {
                 const __nv_bfloat16* xn = xcl + (size_t)wi.n * g.iv * g.C + wi.ch0;
-                for (int i = etid; i < g.iv; i += ET) {
-                    uint32_t r, c;
-                    d_iw.divmod((uint32_t)i, r, c);
-                    const uint4 v = __ldg(reinterpret_cast<const uint4*>(xn + (size_t)i * g.C));
-                    st_shared_v4(xs_s + (r * (uint32_t)Wp + c) * 16u, v.x, v.y, v.z, v.w);
+                for (int i0 = etid; i0 < g.iv; i0 += 4 * ET) {       // four loads of a thread in flight
+                    uint4 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        v[u] = gload_if(i0 + u * ET < g.iv, reinterpret_cast<const uint4*>(xn + (size_t)(i0 + u * ET) * g.C));
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (i0 + u * ET >= g.iv) break;
+                        uint32_t r, c;
+                        d_iw.divmod((uint32_t)(i0 + u * ET), r, c);
+                        st_shared_v4(xs_s + (r * (uint32_t)Wp + c) * 16u, v[u].x, v[u].y, v[u].z, v[u].w);
+                    }
                 }
             }
             b2_epi_barrier();

@@ -202,7 +202,7 @@ tc_dgrad_rowwise_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, con
                             for (int e = 0; e < (1 << D); ++e) {
                                 const size_t a = base + (size_t)idx[e] * g.C;
                                 if (doff != nullptr) {
-                                    const uint4 xv = __ldg(reinterpret_cast<const uint4*>(xcl + a));
+                                    const uint4 xv = gload(reinterpret_cast<const uint4*>(xcl + a));
                                     float d = T[e];
                                     d = fmaf(f[0], bf16_lo(xv.x), d); d = fmaf(f[1], bf16_hi(xv.x), d);
                                     d = fmaf(f[2], bf16_lo(xv.y), d); d = fmaf(f[3], bf16_hi(xv.y), d);

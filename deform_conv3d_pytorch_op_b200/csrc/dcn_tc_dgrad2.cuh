@@ -316,9 +316,8 @@ tc_dgrad_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const float
                     const __nv_bfloat16* xb = xcl + cbase;
 #pragma unroll
                     for (int e = 0; e < NE; ++e)
-                        rd.xv[e] = (want_x && rd.valid)
-                                       ? __ldg(reinterpret_cast<const uint2*>(xb + (uint64_t)(uint32_t)rd.idx[e] * (uint32_t)g.C))
-                                       : make_uint2(0, 0);
+                        rd.xv[e] = gload_if(want_x && rd.valid,
+                                            reinterpret_cast<const uint2*>(xb + (uint64_t)(uint32_t)rd.idx[e] * (uint32_t)g.C));
                 };
                 auto consume = [&](int rr, const RowData& rd) {
                     const int row = rr * 4 + r4;

@@ -281,7 +281,7 @@ tc_forward_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, const flo
                     const int ol = (mb * 2 + mt) * 128 + q * 32 + lane;      // output channel within the group
                     const bool o_ok = ol < g.Og;
                     const int o = j * g.Og + ol;
-                    const float bv = (bias != nullptr && o_ok) ? __ldg(bias + o) : 0.f;
+                    const float bv = (bias != nullptr && o_ok) ? gload(bias + o) : 0.f;
                     if constexpr (TURN) {
                         // Channel-first y whose rows are not 16-byte aligned: 32 x 32 pieces are turned in shared memory
                         // and leave as 128-byte runs along the positions.  (A lane storing its own row of an odd size

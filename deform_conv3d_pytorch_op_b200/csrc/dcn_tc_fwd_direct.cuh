@@ -178,7 +178,7 @@ tc_forward_direct_kernel(const Geom g, const __nv_bfloat16* __restrict__ xcl, co
                 const int ol = (mb * 2 + mt) * 128 + q * 32 + lane;      // output channel within the group
                 const bool o_ok = ol < g.Og;
                 const int o = j * g.Og + ol;
-                const float bv = (bias != nullptr && o_ok) ? __ldg(bias + o) : 0.f;
+                const float bv = (bias != nullptr && o_ok) ? gload(bias + o) : 0.f;
 #pragma unroll 1
                 for (int cc = 0; cc < kTileN / 32; ++cc) {
                     uint32_t v[32];

@@ -70,7 +70,7 @@ __device__ __forceinline__ void job_copy_x(const Geom& g, const Job& J, unsigned
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int p = p0 + h * 32 + tx;
-            v[h][i] = (c < C && p < iv) ? __ldg(xn + (size_t)c * iv + p) : 0.f;
+            v[h][i] = (c < C && p < iv) ? gload(xn + (size_t)c * iv + p) : 0.f;
         }
     }
 #pragma unroll
@@ -89,8 +89,8 @@ __device__ __forceinline__ void job_copy_x(const Geom& g, const Job& J, unsigned
 // fp32 -> bf16 of an input that already is channels-last.  z: groups of 8 elements
 __device__ __forceinline__ void job_cast_x(const Job& J, unsigned blk) {
     for (size_t i = (size_t)blk * kPassThreads + threadIdx.x; i < J.z; i += (size_t)J.blocks * kPassThreads) {
-        const float4 a = __ldg(static_cast<const float4*>(J.src) + 2 * i);
-        const float4 b = __ldg(static_cast<const float4*>(J.src) + 2 * i + 1);
+        const float4 a = gload(static_cast<const float4*>(J.src) + 2 * i);
+        const float4 b = gload(static_cast<const float4*>(J.src) + 2 * i + 1);
         static_cast<uint4*>(J.dst)[i] = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y),
                                                    pack_bf16x2(b.z, b.w));
     }
@@ -114,7 +114,7 @@ __device__ __forceinline__ void job_weight(const Geom& g, const Job& J, unsigned
         uint32_t r, i;
         J.div.divmod((uint32_t)e, r, i);
         float v = 0.f;
-        if (r0 + (int)r < g.Og && (int)i < nc * kv) v = __ldg(w + ((size_t)(j * g.Og + r0 + r) * g.Cg + c0) * kv + i);
+        if (r0 + (int)r < g.Og && (int)i < nc * kv) v = gload(w + ((size_t)(j * g.Og + r0 + r) * g.Cg + c0) * kv + i);
         sm[r * stride + i] = v;
         mx = fmaxf(mx, fabsf(v));
     }
@@ -213,11 +213,11 @@ __device__ __forceinline__ void job_pack_dy(const Geom& g, const Job& J, unsigne
             a[u] = b[u] = 0.f;
             if (ol < g.Og) {
                 if (pair) {
-                    const float2 t = __ldg(reinterpret_cast<const float2*>(src0 + (size_t)ol * g.ov));
+                    const float2 t = gload(reinterpret_cast<const float2*>(src0 + (size_t)ol * g.ov));
                     a[u] = t.x; b[u] = t.y;
                 } else {
-                    if (ok0) a[u] = __ldg(src0 + (size_t)ol * g.ov);
-                    if (ok1) b[u] = __ldg(src1 + (size_t)ol * g.ov);
+                    if (ok0) a[u] = gload(src0 + (size_t)ol * g.ov);
+                    if (ok1) b[u] = gload(src1 + (size_t)ol * g.ov);
                 }
             }
         }
@@ -262,7 +262,7 @@ __device__ __forceinline__ void job_pack_dy_cl(const Geom& g, const Job& J, unsi
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const long long P = pc * 64 + ck * 8 + e;
-            v[e] = (ol < g.Og && P < g.P) ? __ldg(dy + (size_t)P * g.O + j * g.Og + ol) : 0.f;
+            v[e] = (ol < g.Og && P < g.P) ? gload(dy + (size_t)P * g.O + j * g.Og + ol) : 0.f;
             sum += v[e];
         }
         *reinterpret_cast<uint4*>(dst + swz_offset(row, ck)) =
@@ -306,8 +306,8 @@ __device__ __forceinline__ void job_points(const Geom& g, const Job& J, unsigned
         grp = q2 - n * (uint32_t)g.dg;
         op[u] = decompose_pos(g, (long long)n * g.ov + pos);
         const float* ob = offset_ptr<float, 2>(g, offset_block<float, 2>(g, off, (int)n), (int)grp, (int)tap[u], op[u]);
-        offv[u][0] = __ldg(ob);
-        offv[u][1] = __ldg(ob + g.ov);
+        offv[u][0] = gload(ob);
+        offv[u][1] = gload(ob + g.ov);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -368,7 +368,7 @@ __device__ __forceinline__ void job_dx(const Geom& g, const Job& J, unsigned blk
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int c = c0 + h * 32 + tx;
-            v[h][i] = (p < iv && c < C) ? __ldg(in + (size_t)p * C + c) : 0.f;
+            v[h][i] = (p < iv && c < C) ? gload(in + (size_t)p * C + c) : 0.f;
         }
     }
 #pragma unroll
@@ -410,7 +410,7 @@ __device__ __forceinline__ void job_dw(const Geom& g, const Job& J, unsigned blk
         for (int s0 = 0; s0 < J.d; s0 += 4) {
             float4 q[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) q[u] = (s0 + u < J.d) ? __ldg(s + (size_t)(s0 + u) * (J.z / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int u = 0; u < 4; ++u) q[u] = (s0 + u < J.d) ? gload(s + (size_t)(s0 + u) * (J.z / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int u = 0; u < 4; ++u) { v.x += q[u].x; v.y += q[u].y; v.z += q[u].z; v.w += q[u].w; }
         }
@@ -434,7 +434,7 @@ __device__ __forceinline__ void job_bias(const Geom& g, const Job& J, unsigned b
     const int j = o / g.Og, ol = o - j * g.Og;
     const float* s = static_cast<const float*>(J.src) + ((size_t)j * J.a * 128 + ol) * J.z;
     float v = 0.f;
-    for (size_t i = lane; i < J.z; i += 32) v += __ldg(s + i);
+    for (size_t i = lane; i < J.z; i += 32) v += gload(s + i);
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
     if (lane == 0) static_cast<float*>(J.dst)[o] = v;
@@ -461,12 +461,12 @@ __device__ __forceinline__ void fold_y(const Geom& g, const FoldY& a, unsigned s
     const size_t step = (size_t)a.halves * kSliceHalf / 4;
     const float4* s = reinterpret_cast<const float4*>(a.slices) + (size_t)slot * a.parts * step +
                       (mt * kSliceHalf + q * (kSliceHalf / 4) + cg * 2 * kSliceGroup) / 4 + threadIdx.x;
-    const float bv = a.bias != nullptr && o0 + lane < g.Og ? __ldg(a.bias + j * g.Og + o0 + lane) : 0.f;
+    const float bv = a.bias != nullptr && o0 + lane < g.Og ? gload(a.bias + j * g.Og + o0 + lane) : 0.f;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int k0 = 0; k0 < a.parts; k0 += 4) {    // loads in batches of four (all in flight), additions in order
         float4 t[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) t[u] = k0 + u < a.parts ? __ldg(s + (k0 + u) * step) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int u = 0; u < 4; ++u) t[u] = k0 + u < a.parts ? gload(s + (k0 + u) * step) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int u = 0; u < 4; ++u) { v.x += t[u].x; v.y += t[u].y; v.z += t[u].z; v.w += t[u].w; }
     }

@@ -154,7 +154,7 @@ __device__ __forceinline__ void gather_issue_s(uint32_t entry_s, const __nv_bflo
     const bool valid = (int)idx[0] >= 0;
 #pragma unroll
     for (int i = 0; i < NQ; ++i)
-        q[i] = valid ? __ldg(static_cast<const uint4*>(ptr_mad_u32(xrow, idx[i], pix_bytes))) : make_uint4(0, 0, 0, 0);
+        q[i] = gload_if(valid, static_cast<const uint4*>(ptr_mad_u32(xrow, idx[i], pix_bytes)));
 }
 
 template <int D, bool DEFORM>

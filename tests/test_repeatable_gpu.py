@@ -83,3 +83,54 @@ def test_bf16_plain_input_gradient_is_repeatable():
     want = torch.nn.grad.conv2d_input(x.shape, w.double(), dy.double(), padding=1)
     assert cases.rel_err(first.cpu().numpy().astype(np.float64), want.cpu().numpy()) <= 2e-2
     assert all(torch.equal(dx(), first) for _ in range(20))
+
+
+CHAIN = [
+    (Case("exact_3d_many_points", 3, 44, 32, 64, (2, 12, 16), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), 2, 32, offset_std=1.0), "exact"),
+    (Case("exact_two_groups", 2, 5, 96, 96, (30, 33), (3, 3), (1, 1), (1, 1), (1, 1), 2, 24, offset_std=2.0, bias=True), "exact"),
+    (Case("exact_fp64", 2, 2, 39, 39, (16, 12), (3, 3), (2, 2), (1, 1), (1, 1), 1, 39, dtype="float64", offset_std=2.0), "exact"),
+    (Case("exact_narrow", 3, 3, 128, 64, (4, 21, 21), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), 1, 16, offset_std=1.0), "exact"),
+    (Case("bf16_plane", 2, 4, 64, 64, (40, 44), (3, 3), (1, 1), (1, 1), (1, 1), 1, 32, offset_std=2.0, bias=True), "bf16"),
+    (Case("bf16_split", 2, 1, 256, 256, (50, 41), (3, 3), (1, 1), (1, 1), (1, 1), 1, 64, offset_std=2.0), "bf16"),
+    (Case("bf16_3d", 3, 6, 32, 48, (4, 14, 14), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1), 1, 32, offset_std=1.0), "bf16"),
+]
+
+
+def test_calls_in_a_row_wait_for_their_own_prologue():
+    """The kernels of a call become resident while the one before them still runs, and must not read what it writes before
+    it has finished.  Calls of different problems in a row, over workspaces whose memory holds zeros instead of the last
+    call's values (a point read too early then is a wrong one, but an address within the input): the same bits as each call
+    alone."""
+    import ctypes
+    from deform_conv3d_pytorch_op_b200 import _lib
+    made = []
+    for case, precision in CHAIN:
+        tensors = [None if t is None else t.cuda() for t in cases.make_inputs(case)]
+        p = _lib.make_problem(case.ndim, tensors[0].dtype, case.N, case.C, case.O, case.in_size, case.kernel, case.stride,
+                              case.pad, case.dil, case.G, case.cpg, True, False, True,
+                              _lib.PREC_BF16 if precision == "bf16" else _lib.PREC_EXACT)
+        sizes = [_lib.lib().dcn_workspace_bytes(ctypes.byref(p), k) for k in (_lib.PASS_FORWARD, _lib.PASS_BACKWARD)]
+        made.append((case, precision, tensors, sizes))
+
+    def step(case, precision, tensors, sizes, alone):
+        x, w, off, dy, b = tensors
+        x, w = x.detach().requires_grad_(True), w.detach().requires_grad_(True)
+        for n in sizes[:1]:
+            torch.zeros(n, dtype=torch.uint8, device="cuda")          # freed at once: the memory of the next workspace
+        y = _forward(case, (x, w, off, dy, b), precision)
+        if alone:
+            torch.cuda.synchronize()
+        torch.zeros(sizes[1], dtype=torch.uint8, device="cuda")
+        dw, dx = torch.autograd.grad(y, (w, x), dy)
+        if alone:
+            torch.cuda.synchronize()
+        return y.detach(), dw, dx
+
+    want = [step(*m, True) for m in made]
+    for _ in range(15):
+        got = [step(*m, False) for m in made]
+        for (case, precision, _, _), a, b in zip(made, got, want):
+            assert torch.equal(a[0], b[0]), case.name
+            assert torch.equal(a[1], b[1]), case.name
+            scale = float(b[2].abs().max())
+            assert float((a[2] - b[2]).abs().max()) <= (2e-2 if precision == "bf16" else 1e-4) * scale, case.name
