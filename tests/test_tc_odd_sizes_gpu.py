@@ -1,5 +1,6 @@
-"""Tensor-core forward kernels on outputs whose rows are not 16-byte aligned (they leave through shared memory): ragged
-tails of positions and channels, K parts added up, the variant that locates points in its producers."""
+"""Tensor-core kernels on outputs whose rows are not 16-byte aligned (the forward kernel turns them in shared memory, its
+variant that locates points in its producers stores them from registers): ragged tails of positions and channels, K parts
+added up.  All gradients beside the output."""
 import numpy as np
 import pytest
 
@@ -21,5 +22,9 @@ def test_odd_output_sizes(case):
     tensors = cases.make_inputs(case)
     ours = helpers.run_ours(case, tensors, "bf16")
     ref = helpers.run_oracle(case, tensors, np.float64)
-    for k in ("y", "dx", "dw", "db"):
-        assert cases.rel_err(ours[k].astype(np.float64), ref[k]) <= 2e-2, (case.name, k)
+    mask = helpers.lattice_mask(case, tensors[2].numpy()) if case.deformable else None
+    for k in ref:
+        a, b = ours[k].astype(np.float64), ref[k]
+        if k == "doff":
+            a, b = np.where(mask, 0, a), np.where(mask, 0, b)
+        assert cases.rel_err(a, b) <= 2e-2, (case.name, k)
