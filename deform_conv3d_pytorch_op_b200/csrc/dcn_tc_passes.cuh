@@ -445,9 +445,8 @@ __device__ __forceinline__ void job_bias(const Geom& g, const Job& J, unsigned b
 // one 16-byte vector of every slice per thread, in the order in which the epilogue stored them; y leaves in 128-byte runs,
 // along the positions or the channels.
 // Bound by latency (launch, one read of L2, one turn).  Against the reductions, B200: one image 256 -> 256 channels 50x76,
-// 30 tiles in 4 parts: kernel 26.3 -> 20.0 us and 4.2 us of fold, call 28.5 -> 29.1; 8 x 128 -> 128, 28x28 as a layer, three
-// forward kernels in 3 parts: step 140 -> 152 us; config 2, 44 of 784 tiles in 3 parts: 1211 -> 1219; 2 x 128, 101x151, a tail
-// over two groups that could not be split before: 264 -> 256.  Folding in the CTA that finishes a tile last is slower: its
+// 30 tiles in 4 parts: kernel 26.3 -> 20.0 us and 4.2 us of fold, call 28.2 -> 28.5; 8 x 128 -> 128, 28x28 as a layer, three
+// forward kernels in 3 parts: step 142 -> 150 us; config 2, 44 of 784 tiles in 3 parts: 1210 -> 1214.  Folding in the CTA that finishes a tile last is slower: its
 // slices then pass through one SM (kernel 34.6 us for the first, step 170 us for the second).
 // piece: [half][lane quarter][32 positions]
 __device__ __forceinline__ void fold_y(const Geom& g, const FoldY& a, unsigned slot, unsigned piece, float* sm) {

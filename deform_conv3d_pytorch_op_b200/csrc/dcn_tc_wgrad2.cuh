@@ -4,8 +4,8 @@
 //
 // GEMM view: M = output channels (128-row tiles, up to two per CTA), N = a block of up to 256 k' columns,
 // K = output positions, 64 per pipeline stage.  One CTA owns one (group, o-block, k'-block) and a slice of
-// the position range; partial sums are added with 16-byte fp32 reductions to a packed, zero-filled scratch
-// dwpk[o][k'] (tiny and L2-resident) that the dW fold brings into dW's [O][Cg][kv] layout afterwards.
+// the position range; partial sums are stored in a slice of the packed scratch dwpk[split][k' / 4][rows][4] of its own,
+// and the dW fold adds the slices in slice order into dW's [O][Cg][kv] layout afterwards.
 //   A operand: dy, bf16, pre-packed into swizzled [128 o][64 P] tiles  -> K-major, bulk-copied
 //   B operand: sampled patch, [64 P rows][64 k' per 128-byte row] sub-tiles        -> MN-major, produced here
 // Warps: 0 MMA issue, 1 dy-tile loader, 2-5 coordinate warps (warp k fills the table of every 4th stage, as in
